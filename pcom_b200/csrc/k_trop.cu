@@ -672,33 +672,54 @@ int trop_res_max_blocks(int TX, int TY) {
 // Fast variant of the resident kernel: the same arithmetic with every division
 // by a static metric, bottom pressure or Coriolis denominator done with its
 // correctly rounded reciprocal (dvr), which removes the per-division
-// reciprocal-approximation instruction from the critical path.
-
+// reciprocal-approximation instruction from the critical path, and tiles
+// that meet only their neighbours.
+//
+// Exchange: a tile's border points (within 2 of its edge) are sent as
+// {value, sequence number} words (xch_put), ub and vb as soon as S6 has
+// them, ch from S8; the threads of the 2-cell ring poll for exactly the
+// words they need.  There is no grid barrier and no fence: the number
+// arrives with the value.  Two buffers by substep parity suffice: a tile
+// overwrites its words of substep n - 2 in substep n, after it has read its
+// neighbours' words of n - 1, which they sent after reading its n - 2 (being
+// in reach is symmetric).  `seq` + n numbers substep n; the caller advances
+// it by nstep per launch and no two launches share a number.
 //
 // GROUP = true: the same kernel over a work list of tiles of several domains
 // (ensemble members, basins), one tile per CTA; each CTA reads its domain's
-// Dev from `Ps`, and the grid barrier counts on `gcnt` (zeroed before the
-// launch) with timeouts flagged in `gerr`.
+// Dev from `Ps`, the sequence base from *gseq, and flags timeouts in `gerr`.
 //
 // CTX, CTY > 0: the same kernel compiled for one tile shape, so that the
 // region's row length and plane size are constants and every shared-memory
 // operand is a fixed offset from the thread's own point (fewer instructions
 // and registers per substep than the general form, CTX = CTY = 0).
+namespace {
+// region fields in shared memory; what a later stage needs at the thread's
+// own point only stays in registers
+enum {
+  X_CH, X_UB, X_VB,
+  X_S1, X_X2,  // supb1, supb2*rh3 (reused for the corrector's supb)
+  X_PRED,
+  X_A1U, X_A1V, X_GY, X_CN,
+  X_A2U, X_A2V, X_GX, X_CE,
+  X_COUNT
+};
+}  // namespace
+
 template <bool GROUP, int CTX = 0, int CTY = 0>
 __global__ void __launch_bounds__(kResThreads, 1)
     k_trop_fast(const __grid_constant__ Dev P0, const Dev *__restrict__ Ps, const TileRef *__restrict__ tiles,
-                int TX, int TY, int ntx, unsigned long long epoch, unsigned long long *gcnt, int *gerr) {
+                int TX, int TY, int ntx, unsigned long long seq0, const unsigned long long *gseq, int *gerr) {
   if (CTX > 0) { TX = CTX; TY = CTY; }
   extern __shared__ double sm[];
-  __shared__ int s_stop;
   const TileRef T = GROUP ? tiles[blockIdx.x] : TileRef{0, 0, 0, 0, 0};
   const Dev &P = GROUP ? Ps[T.m] : P0;
-  unsigned long long *const bar_cnt = GROUP ? gcnt : P.tile_flag;
-  int *const bar_err = GROUP ? gerr : P.err;
+  const unsigned long long seq = GROUP ? *gseq : seq0;
+  int *const err = GROUP ? gerr : P.err;
   const int ni = P.ni, nj = P.nj, njm = P.njm, G = P.glo_ni;
   const int W = TX + 4, H = TY + 4, RS = W * H;
-  double *vx = sm + R_COUNT * RS;  // dxx[1..4], 1/dxx[1..4] over lx: 8*W
-  double *vy = vx + 8 * W;         // kFastVy vectors over ly (see below)
+  double *vx = sm + X_COUNT * RS;  // dxx[1..4], 1/dxx[1..4] over lx: 8*W
+  double *vy = vx + 8 * W;         // 19 vectors over ly (see below)
   const double a = P.c.a, bt = (double)P.bt, gamma_b = P.c.gamma_b;
   const int nstep = P.nstep;
   const int tid = threadIdx.x;
@@ -759,6 +780,11 @@ __global__ void __launch_bounds__(kResThreads, 1)
   const bool inN = active && lx >= 1 && lx < tw + 3 && ly >= 1 && ly < th + 2;
   const bool inE = active && lx >= 1 && lx < tw + 2 && ly >= 1 && ly < th + 3;
   const bool inS8 = active && lx >= 2 && lx < tw + 2 && ly >= 2 && ly < th + 2;
+  // points some tile's ring covers (this tile's own, where the ring wraps)
+  const bool border = inS8 && (lx < 4 || lx >= tw || ly < 4 || ly >= th);
+  // points of this tile's ring (columns and rows past a partial tile's
+  // region are nobody's)
+  const bool ring = active && !inS8 && lx < tw + 4 && ly < th + 4;
   const int levu = active ? __ldg(P.lev_u + q) : 0, levt = active ? __ldg(P.lev_t + q) : 0;
   const double seau = (double)(levu >= 1), mskt1 = (double)(levt >= 1);
   const double prh_u = active ? ld(P.prh_u, q) : 1.0, prh_t = active ? ld(P.prh_t, q) : 1.0;
@@ -783,188 +809,179 @@ __global__ void __launch_bounds__(kResThreads, 1)
     acc_u = P.ubc[q]; acc_v = P.vbc[q];
   }
   const double land_ch0 = inS4 ? P.chc[q] : 0.0;
+  // ch, ub, vb at this thread's point, as staged for the current substep
+  double c0 = 0.0, u0 = 0.0, v0 = 0.0;
+  if (active && (inS8 || ring)) {
+    c0 = __ldcg(P.chp + q);
+    S(X_CH, p) = c0;
+    if (inS2) {
+      u0 = __ldcg(P.ubp + q); v0 = __ldcg(P.vbp + q);
+      S(X_UB, p) = u0; S(X_VB, p) = v0;
+    }
+  }
   __syncthreads();
 
-  // S2 at this thread's point: sch = sqrt(ter(ch)) on U and the fluxes
-  // supb.  Points with lx in 2..tw and ly in 2..th read only the tile's own
-  // state (ch at the point and its E, N, NE neighbours; ub, vb at the point)
-  auto s2 = [&]() {
-    double sch = 1.0;
-    if (levu > 0) {
-      const double w = nrow ? (S(R_CH, p) + S(R_CH, p + W) + S(R_CH, p + 1) + S(R_CH, p + W + 1)) * 0.25 : 0.0;
-      sch = sqrt(w);
-    }
-    const double ps = prh_u * sch;
-    S(R_S1, p) = ps * S(R_UB, p);
-    S(R_X2, p) = ps * S(R_VB, p) * RH(3, ly);
-  };
-  const bool s2own = inS2 && lx >= 2 && lx <= tw && ly >= 2 && ly <= th;
-
-  const unsigned long long base = epoch;  // arrivals counted before this launch
   for (int nt = 1; nt <= nstep; ++nt) {
-    const int d = (nt - 1) & 1;
-    const double *src_ch = (nt == 1) ? P.chp : P.tr_ch[1 - d];
-    const double *src_ub = (nt == 1) ? P.ubp : P.tr_ub[1 - d];
-    const double *src_vb = (nt == 1) ? P.vbp : P.tr_vb[1 - d];
-    // S1: previous state.  After the first substep the tile's own points
-    // already hold it (written in S8), so only the 2-cell ring comes from
-    // L2 (.cg loads: written by other SMs)
-    if (active && (nt == 1 || !inS8)) {
-      S(R_CH, p) = __ldcg(src_ch + q);
-      if (inS2) { S(R_UB, p) = __ldcg(src_ub + q); S(R_VB, p) = __ldcg(src_vb + q); }
+    ulonglong2 *const out = P.xch + (long long)(nt & 1) * 3 * P.n2 + q;  // this substep's words of this point
+    // S2: sch = sqrt(ter(ch)) on U, supb
+    double s1 = 0.0, x2 = 0.0;
+    if (inS2) {
+      double sch = 1.0;
+      if (levu > 0) {
+        const double w = nrow ? (c0 + S(X_CH, p + W) + S(X_CH, p + 1) + S(X_CH, p + W + 1)) * 0.25 : 0.0;
+        sch = sqrt(w);
+      }
+      const double ps = prh_u * sch;
+      s1 = ps * u0;
+      x2 = ps * v0 * RH(3, ly);
+      S(X_S1, p) = s1;
+      S(X_X2, p) = x2;
     }
-    __syncthreads();
-    // S2: sch = sqrt(ter(ch)) on U, supb (after the first substep the
-    // points whose inputs are all the tile's own were done while waiting at
-    // the grid barrier)
-    if (inS2 && (nt == 1 || !s2own)) s2();
     __syncthreads();
     // S4: predictor ch; the ter U->E (rows >= 2) and U->N means of supb are
     // formed here from the staged supb
+    double pred = 0.0;
     if (inS4) {
       // tE at (i, j) and (i-1, j): j >= 2 ? 0.5 (s1(j-1) + s1(j)) : 0
-      const double tEc = srow ? 0.5 * (S(R_S1, p - W) + S(R_S1, p)) : 0.0;
-      const double tEw = srow ? 0.5 * (S(R_S1, p - W - 1) + S(R_S1, p - 1)) : 0.0;
+      const double tEc = srow ? 0.5 * (S(X_S1, p - W) + s1) : 0.0;
+      const double tEw = srow ? 0.5 * (S(X_S1, p - W - 1) + S(X_S1, p - 1)) : 0.0;
       const double A = dvr(tEc - tEw, DXX(1, lx), RDXX(1, lx));
       double B = 0.0;
       if (srow) {
         // tN at (i, j) and (i, j-1): 0.5 (x2(i-1) + x2(i))
-        const double tNc = 0.5 * (S(R_X2, p - 1) + S(R_X2, p));
-        const double tNs = 0.5 * (S(R_X2, p - W - 1) + S(R_X2, p - W));
+        const double tNc = 0.5 * (S(X_X2, p - 1) + x2);
+        const double tNs = 0.5 * (S(X_X2, p - W - 1) + S(X_X2, p - W));
         B = dvr(tNc - tNs, DXY(1, ly), RDXY(1, ly));
       }
       const double div = dvr(A + B, vy[12 * H + ly], vy[13 * H + ly]);
-      double pred;
-      if (levt > 0) pred = S(R_CH, p) - dvr(div * bt * gamma_b, prh_t, rprh_t);
-      else pred = (nt == 1) ? land_ch0 : S(R_CH, p);
-      S(R_PRED, p) = pred;
+      if (levt > 0) pred = c0 - dvr(div * bt * gamma_b, prh_t, rprh_t);
+      else pred = (nt == 1) ? land_ch0 : c0;
+      S(X_PRED, p) = pred;
     }
     __syncthreads();
     // S5: sch on U; N- and E-grid intermediates
-    if (inS6) {
-      double sch = 1.0;
-      if (levu > 0) {
-        const double w = nrow ? (S(R_PRED, p) + S(R_PRED, p + W) + S(R_PRED, p + 1) + S(R_PRED, p + W + 1)) * 0.25 : 0.0;
-        sch = sqrt(w);
-      }
-      S(R_SCHE, p) = sch;
+    double sche = 1.0, a1u = 0.0, a1v = 0.0, gy = 0.0, cn = 0.0, a2u = 0.0, a2v = 0.0, gx = 0.0, ce = 0.0;
+    if (inS6 && levu > 0) {
+      const double w = nrow ? (pred + S(X_PRED, p + W) + S(X_PRED, p + 1) + S(X_PRED, p + W + 1)) * 0.25 : 0.0;
+      sche = sqrt(w);
     }
     if (inN) {
       const double dx4 = DXX(4, lx), rdx4 = RDXX(4, lx), rh4 = RH(4, ly), rrh4 = vy[16 * H + ly];
-      S(R_A1U, p) = dvr(dvr(S(R_UB, p) - S(R_UB, p - 1), dx4, rdx4), rh4, rrh4);
-      S(R_A1V, p) = dvr(dvr(S(R_VB, p) - S(R_VB, p - 1), dx4, rdx4), rh4, rrh4);
+      a1u = dvr(dvr(u0 - S(X_UB, p - 1), dx4, rdx4), rh4, rrh4);
+      a1v = dvr(dvr(v0 - S(X_VB, p - 1), dx4, rdx4), rh4, rrh4);
       if (nrow) {
-        S(R_GY, p) = dvr(dvr(S(R_PRED, p + W) - S(R_PRED, p), DXY(4, ly), RDXY(4, ly)), a, ra);
-        S(R_CN, p) = 0.5 * (S(R_PRED, p) + S(R_PRED, p + W));
-      } else {
-        S(R_GY, p) = 0.0;
-        S(R_CN, p) = 0.0;
+        gy = dvr(dvr(S(X_PRED, p + W) - pred, DXY(4, ly), RDXY(4, ly)), a, ra);
+        cn = 0.5 * (pred + S(X_PRED, p + W));
       }
+      S(X_A1U, p) = a1u;
+      S(X_A1V, p) = a1v;
+      S(X_GY, p) = gy;
+      S(X_CN, p) = cn;
     }
     if (inE) {
       const double rh2 = RH(2, ly);
       if (srow) {
         const double dy2 = DXY(2, ly), rdy2 = RDXY(2, ly);
-        S(R_A2U, p) = dvr(S(R_UB, p) - S(R_UB, p - W), dy2, rdy2) * rh2;
-        S(R_A2V, p) = dvr(S(R_VB, p) - S(R_VB, p - W), dy2, rdy2) * rh2;
-      } else {
-        S(R_A2U, p) = 0.0;
-        S(R_A2V, p) = 0.0;
+        a2u = dvr(u0 - S(X_UB, p - W), dy2, rdy2) * rh2;
+        a2v = dvr(v0 - S(X_VB, p - W), dy2, rdy2) * rh2;
       }
-      S(R_GX, p) = dvr(dvr(S(R_PRED, p + 1) - S(R_PRED, p), DXX(2, lx), RDXX(2, lx)), vy[14 * H + ly], vy[15 * H + ly]);
-      S(R_CE, p) = 0.5 * (S(R_PRED, p) + S(R_PRED, p + 1));
+      gx = dvr(dvr(S(X_PRED, p + 1) - pred, DXX(2, lx), RDXX(2, lx)), vy[14 * H + ly], vy[15 * H + ly]);
+      ce = 0.5 * (pred + S(X_PRED, p + 1));
+      S(X_A2U, p) = a2u;
+      S(X_A2V, p) = a2v;
+      S(X_GX, p) = gx;
+      S(X_CE, p) = ce;
     }
     __syncthreads();
     // S6: corrector velocity (viscosity, pressure gradient, Coriolis adjustment)
+    double ubc = 0.0, vbc = 0.0;
     if (inS6) {
       const double rh3 = RH(3, ly), dx3 = DXX(3, lx), rdx3 = RDXX(3, lx), dy3 = DXY(3, ly), rdy3 = RDXY(3, ly);
       const double aarh = vy[17 * H + ly], raarh = vy[18 * H + ly];
-      const double L1u = dvr(S(R_A1U, p + 1) - S(R_A1U, p), dx3, rdx3);
-      const double L1v = dvr(S(R_A1V, p + 1) - S(R_A1V, p), dx3, rdx3);
-      const double L2u = nrow ? dvr(S(R_A2U, p + W) - S(R_A2U, p), dy3, rdy3) : 0.0;
-      const double L2v = nrow ? dvr(S(R_A2V, p + W) - S(R_A2V, p), dy3, rdy3) : 0.0;
+      const double L1u = dvr(S(X_A1U, p + 1) - a1u, dx3, rdx3);
+      const double L1v = dvr(S(X_A1V, p + 1) - a1v, dx3, rdx3);
+      const double L2u = nrow ? dvr(S(X_A2U, p + W) - a2u, dy3, rdy3) : 0.0;
+      const double L2v = nrow ? dvr(S(X_A2V, p + W) - a2v, dy3, rdy3) : 0.0;
       const double vsu = sam1 * dvr(L1u + L2u, aarh, raarh);
       const double vsv = sam1 * dvr(L1v + L2v, aarh, raarh);
       if (nt == 1) { vs0u = vsu; vs0v = vsv; }
       const double dvu = vsu - vs0u, dvv = vsv - vs0v;
       double gi1 = 0.0, cg1 = 0.0;
       if (nrow) {
-        gi1 = 0.5 * (S(R_GX, p) * bxn + S(R_GX, p + W) * bxs);
-        cg1 = 0.5 * (S(R_CE, p) * gxn + S(R_CE, p + W) * gxs);
+        gi1 = 0.5 * (gx * bxn + S(X_GX, p + W) * bxs);
+        cg1 = 0.5 * (ce * gxn + S(X_CE, p + W) * gxs);
       }
-      const double gi2 = 0.5 * (S(R_GY, p) * bye + S(R_GY, p + 1) * byw);
-      const double cg2 = 0.5 * (S(R_CN, p) * gye + S(R_CN, p + 1) * gyw);
-      const double sch = S(R_SCHE, p);
-      const double pg1 = (gi1 + cg1 + ghx) * seau * sch;
-      const double pg2 = (gi2 + cg2 + ghy) * seau * sch;
-      const double ubp = S(R_UB, p), vbp = S(R_VB, p);
-      double p1 = seau * (dvu + ut - pg1 + 0.5 * cor * vbp);
-      double p2 = seau * (dvv + vt - pg2 - 0.5 * cor * ubp);
-      const double w1 = p1 * bt + ubp, w2 = p2 * bt + vbp;
+      const double gi2 = 0.5 * (gy * bye + S(X_GY, p + 1) * byw);
+      const double cg2 = 0.5 * (cn * gye + S(X_CN, p + 1) * gyw);
+      const double pg1 = (gi1 + cg1 + ghx) * seau * sche;
+      const double pg2 = (gi2 + cg2 + ghy) * seau * sche;
+      double p1 = seau * (dvu + ut - pg1 + 0.5 * cor * v0);
+      double p2 = seau * (dvv + vt - pg2 - 0.5 * cor * u0);
+      const double w1 = p1 * bt + u0, w2 = p2 * bt + v0;
       const double cb = 0.5 * cor * bt;
       const double den = 1 + cb * cb;
       double u1 = dvr(w1 + 0.5 * cor * bt * w2, den, rden);
       double v1 = dvr(w2 - 0.5 * cor * bt * w1, den, rden);
-      u1 = 0.5 * (u1 + ubp);
-      v1 = 0.5 * (v1 + vbp);
+      u1 = 0.5 * (u1 + u0);
+      v1 = 0.5 * (v1 + v0);
       p1 = seau * (dvu - pg1 + ut + cor * v1);
       p2 = seau * (dvv - pg2 + vt - cor * u1);
-      const double ubc = p1 * bt + ubp, vbc = p2 * bt + vbp;
-      S(R_UBC, p) = ubc;
-      S(R_VBC, p) = vbc;
-      const double ps = prh_u * sch;
-      S(R_S1, p) = ps * ubc;
-      S(R_X2, p) = ps * vbc * rh3;
+      ubc = p1 * bt + u0;
+      vbc = p2 * bt + v0;
+      if (border && nt < nstep) {
+        xch_put(out + P.n2, ubc, seq + nt);
+        xch_put(out + 2 * P.n2, vbc, seq + nt);
+      }
+      const double ps = prh_u * sche;
+      s1 = ps * ubc;
+      x2 = ps * vbc * rh3;
+      S(X_S1, p) = s1;
+      S(X_X2, p) = x2;
     }
     __syncthreads();
-    // S8: corrector ch (with the ter means of the corrector's supb), store, accumulate
+    // S8: corrector ch (with the ter means of the corrector's supb), send, accumulate
     if (inS8) {
-      const double tEc = srow ? 0.5 * (S(R_S1, p - W) + S(R_S1, p)) : 0.0;
-      const double tEw = srow ? 0.5 * (S(R_S1, p - W - 1) + S(R_S1, p - 1)) : 0.0;
+      const double tEc = srow ? 0.5 * (S(X_S1, p - W) + s1) : 0.0;
+      const double tEw = srow ? 0.5 * (S(X_S1, p - W - 1) + S(X_S1, p - 1)) : 0.0;
       const double A = dvr(tEc - tEw, DXX(1, lx), RDXX(1, lx));
       double B = 0.0;
       if (srow) {
-        const double tNc = 0.5 * (S(R_X2, p - 1) + S(R_X2, p));
-        const double tNs = 0.5 * (S(R_X2, p - W - 1) + S(R_X2, p - W));
+        const double tNc = 0.5 * (S(X_X2, p - 1) + x2);
+        const double tNs = 0.5 * (S(X_X2, p - W - 1) + S(X_X2, p - W));
         B = dvr(tNc - tNs, DXY(1, ly), RDXY(1, ly));
       }
       const double div = dvr(A + B, vy[12 * H + ly], vy[13 * H + ly]);
-      const double chn = S(R_CH, p) - dvr(mskt1 * div * bt, prh_t, rprh_t);
-      const double ubc = S(R_UBC, p), vbc = S(R_VBC, p);
-      const int d2 = d;
-      st2(P.tr_ch[d2], P, i, q, chn);
-      st2(P.tr_ub[d2], P, i, q, ubc);
-      st2(P.tr_vb[d2], P, i, q, vbc);
-      // the next substep's state at this point (during S8 only this thread
-      // reads these three entries)
-      S(R_CH, p) = chn;
-      S(R_UB, p) = ubc;
-      S(R_VB, p) = vbc;
+      const double chn = c0 - dvr(mskt1 * div * bt, prh_t, rprh_t);
+      if (border && nt < nstep) xch_put(out, chn, seq + nt);
+      // the next substep's state at this point (nobody reads these three
+      // entries in S8)
+      c0 = chn; u0 = ubc; v0 = vbc;
+      S(X_CH, p) = c0;
+      S(X_UB, p) = u0;
+      S(X_VB, p) = v0;
       if (nt <= nstep / 2) acc_m = acc_m + chn;
       acc_m2 = acc_m2 + chn;
       acc_u = acc_u + ubc;
       acc_v = acc_v + vbc;
     }
-    // grid barrier on a monotone arrival counter: after the CTA barrier,
-    // thread 0 adds 1 with release semantics (cumulative over the CTA's
-    // writes ordered before it by bar.sync), then waits (bounded, acquire)
-    // for all arrivals of this substep; the counter is never reset, targets
-    // grow per launch.  The outcome reaches the CTA through shared memory.
-    // Between the arrival and the wait the CTA does the next substep's S2 on
-    // the points that need no other tile's state (shared memory only: the
-    // S8 reads of supb are behind the CTA barrier).
-    __syncthreads();
-    if (tid == 0) {
-      cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> c(*bar_cnt);
-      c.fetch_add(1ULL, cuda::memory_order_release);
+    if (nt == nstep) break;
+    // the ring's state of this substep from the tiles around (after this
+    // warp's own words are out: a warp holds points of both kinds)
+    __syncwarp();
+    int fail = 0;
+    if (ring) {
+      const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : nullptr, inS2 ? out + 2 * P.n2 : nullptr};
+      double v[3] = {0.0, 0.0, 0.0};
+      fail = !xch_wait(in, seq + nt, v, err, P.wait_ns);
+      c0 = v[0];
+      S(X_CH, p) = c0;
+      if (inS2) {
+        u0 = v[1]; v0 = v[2];
+        S(X_UB, p) = u0;
+        S(X_VB, p) = v0;
+      }
     }
-    if (nt < nstep && s2own) s2();
-    if (tid == 0) {
-      const unsigned long long want = base + (unsigned long long)nt * gridDim.x;
-      s_stop = wait_count(bar_cnt, want, bar_err, P.wait_ns) ? 0 : 1;
-    }
-    __syncthreads();
-    if (s_stop) return;
+    if (__syncthreads_or(fail)) return;
   }
   if (inS8) {
     const double ub = acc_u / (nstep + 1), vb = acc_v / (nstep + 1);
@@ -983,17 +1000,13 @@ __global__ void __launch_bounds__(kResThreads, 1)
 
 
 // The resident kernel's synchronisation skeleton, its latency floor: the
-// same grid, block and shared memory (so the same residency, one CTA per SM),
-// and per substep the same ring reload of ch, ub, vb from L2, the same seven
-// CTA barriers, the same interior stores and the same grid barrier on the
-// monotone arrival counter, with none of the arithmetic.  It writes only the
-// subcycle's ping-pong buffers, which every barotropic launch starts afresh
-// from chp, ubp, vbp.  (The real kernel also does the next substep's S2 on
-// its own points while it waits at the grid barrier.)
+// same grid, block and shared memory (so the same residency), and per
+// substep the same five CTA barriers and the same messages to and from the
+// tiles around, with none of the arithmetic.  It writes only the message
+// buffer, with sequence numbers of its own.
 __global__ void __launch_bounds__(kResThreads, 1)
-    k_trop_floor(const __grid_constant__ Dev P, int TX, int TY, int ntx, unsigned long long epoch) {
+    k_trop_floor(const __grid_constant__ Dev P, int TX, int TY, int ntx, unsigned long long seq) {
   extern __shared__ double sm[];
-  __shared__ int s_stop;
   const int nj = P.nj, G = P.glo_ni;
   const int W = TX + 4, H = TY + 4, RS = W * H;
   const int tid = threadIdx.x;
@@ -1011,47 +1024,45 @@ __global__ void __launch_bounds__(kResThreads, 1)
   const long long q = active ? I2(P, i, j) : 0;
   const bool inS2 = active && lx < tw + 3 && ly < th + 3;
   const bool inS8 = active && lx >= 2 && lx < tw + 2 && ly >= 2 && ly < th + 2;
+  const bool border = inS8 && (lx < 4 || lx >= tw || ly < 4 || ly >= th);
+  const bool ring = active && !inS8 && lx < tw + 4 && ly < th + 4;
+  if (active) S(X_CH, p) = S(X_UB, p) = S(X_VB, p) = 0.0;
   __syncthreads();
-  for (int nt = 1; nt <= P.nstep; ++nt) {
-    const int d = (nt - 1) & 1;
-    const double *src_ch = (nt == 1) ? P.chp : P.tr_ch[1 - d];
-    const double *src_ub = (nt == 1) ? P.ubp : P.tr_ub[1 - d];
-    const double *src_vb = (nt == 1) ? P.vbp : P.tr_vb[1 - d];
-    if (active && (nt == 1 || !inS8)) {
-      S(R_CH, p) = __ldcg(src_ch + q);
-      if (inS2) { S(R_UB, p) = __ldcg(src_ub + q); S(R_VB, p) = __ldcg(src_vb + q); }
-    }
+  for (int nt = 1; nt < P.nstep; ++nt) {
+    ulonglong2 *const out = P.xch + (long long)(nt & 1) * 3 * P.n2 + q;
     #pragma unroll 1
-    for (int b = 0; b < 5; ++b) __syncthreads();  // after S1, S2, S4, S5, S6
-    if (inS8) {
-      st2(P.tr_ch[d], P, i, q, S(R_CH, p));
-      st2(P.tr_ub[d], P, i, q, S(R_UB, p));
-      st2(P.tr_vb[d], P, i, q, S(R_VB, p));
+    for (int b = 0; b < 3; ++b) __syncthreads();  // after S2, S4, S5
+    if (border) {
+      xch_put(out + P.n2, S(X_UB, p), seq + nt);
+      xch_put(out + 2 * P.n2, S(X_VB, p), seq + nt);
     }
-    __syncthreads();
-    if (tid == 0) {
-      cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> c(*P.tile_flag);
-      c.fetch_add(1ULL, cuda::memory_order_release);
-      const unsigned long long want = epoch + (unsigned long long)nt * gridDim.x;
-      s_stop = wait_count(P.tile_flag, want, P.err, P.wait_ns) ? 0 : 1;
+    __syncthreads();  // after S6
+    if (border) xch_put(out, S(X_CH, p), seq + nt);
+    __syncwarp();
+    int fail = 0;
+    if (ring) {
+      const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : nullptr, inS2 ? out + 2 * P.n2 : nullptr};
+      double v[3] = {0.0, 0.0, 0.0};
+      fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns);
+      S(X_CH, p) = v[0];
+      if (inS2) { S(X_UB, p) = v[1]; S(X_VB, p) = v[2]; }
     }
-    __syncthreads();
-    if (s_stop) return;
+    if (__syncthreads_or(fail)) return;
   }
 }
 
-cudaError_t launch_trop_floor(const Dev &P, int TX, int TY, unsigned long long epoch, cudaStream_t s) {
+cudaError_t launch_trop_floor(const Dev &P, int TX, int TY, unsigned long long seq, cudaStream_t s) {
   const int ntx = (P.glo_ni + TX - 1) / TX, nty = (P.nj + TY - 1) / TY;
   const size_t smem = trop_fast_smem_bytes(TX, TY);
   cudaError_t e = cudaFuncSetAttribute(k_trop_floor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int nthreads = ((TX + 4) * (TY + 4) + 31) / 32 * 32;
-  void *args[] = {(void *)&P, (void *)&TX, (void *)&TY, (void *)&ntx, (void *)&epoch};
+  void *args[] = {(void *)&P, (void *)&TX, (void *)&TY, (void *)&ntx, (void *)&seq};
   return cudaLaunchCooperativeKernel((const void *)k_trop_floor, dim3(ntx * nty), dim3(nthreads), args, smem, s);
 }
 
 size_t trop_fast_smem_bytes(int TX, int TY) {
-  return ((size_t)R_COUNT * (TX + 4) * (TY + 4) + 8 * (TX + 4) + 19 * (TY + 4)) * sizeof(double);
+  return ((size_t)X_COUNT * (TX + 4) * (TY + 4) + 8 * (TX + 4) + 19 * (TY + 4)) * sizeof(double);
 }
 
 namespace {
@@ -1075,7 +1086,7 @@ const void *group_kernel(int TX, int TY) {
 }
 }  // namespace
 
-cudaError_t launch_trop_fast(const Dev &P, int TX, int TY, unsigned long long epoch, cudaStream_t s) {
+cudaError_t launch_trop_fast(const Dev &P, int TX, int TY, unsigned long long seq, cudaStream_t s) {
   const int ntx = (P.glo_ni + TX - 1) / TX, nty = (P.nj + TY - 1) / TY;
   const size_t smem = trop_fast_smem_bytes(TX, TY);
   const void *fn = fast_kernel(TX, TY);
@@ -1084,9 +1095,9 @@ cudaError_t launch_trop_fast(const Dev &P, int TX, int TY, unsigned long long ep
   int nthreads = ((TX + 4) * (TY + 4) + 31) / 32 * 32;
   const Dev *nps = nullptr;
   const TileRef *nts = nullptr;
-  unsigned long long *ncnt = nullptr;
+  const unsigned long long *ncnt = nullptr;
   int *nerr = nullptr;
-  void *args[] = {(void *)&P, (void *)&nps, (void *)&nts, (void *)&TX, (void *)&TY, (void *)&ntx, (void *)&epoch,
+  void *args[] = {(void *)&P, (void *)&nps, (void *)&nts, (void *)&TX, (void *)&TY, (void *)&ntx, (void *)&seq,
                   (void *)&ncnt, (void *)&nerr};
   return cudaLaunchCooperativeKernel(fn, dim3(ntx * nty), dim3(nthreads), args, smem, s);
 }
@@ -1110,20 +1121,25 @@ int fast_max_blocks(int TX, int TY) {
 int trop_fast_max_blocks(int TX, int TY) { return fast_max_blocks<false>(TX, TY); }
 int trop_group_max_blocks(int TX, int TY) { return fast_max_blocks<true>(TX, TY); }
 
-cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY,
+namespace {
+__global__ void k_advance(unsigned long long *cnt, int n) { *cnt += (unsigned long long)n; }
+}  // namespace
+
+cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nstep,
                               unsigned long long *cnt, int *err, cudaStream_t s) {
   const size_t smem = trop_fast_smem_bytes(TX, TY);
   const void *fn = group_kernel(TX, TY);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  // the group's barrier counter starts from zero in every launch
-  e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s);
-  if (e != cudaSuccess) return e;
+  // sequence numbers no message of an earlier launch carries (the launch may
+  // be a node of a graph that is replayed, so they come from device memory)
+  k_advance<<<1, 1, 0, s>>>(cnt, nstep);
   const int nthreads = ((TX + 4) * (TY + 4) + 31) / 32 * 32;
   Dev none{};
   const int ntx = 0;
-  const unsigned long long epoch = 0;
-  void *args[] = {(void *)&none, (void *)&dPs, (void *)&dtiles, (void *)&TX, (void *)&TY, (void *)&ntx, (void *)&epoch,
-                  (void *)&cnt, (void *)&err};
+  const unsigned long long seq = 0;
+  const unsigned long long *ccnt = cnt;
+  void *args[] = {(void *)&none, (void *)&dPs, (void *)&dtiles, (void *)&TX, (void *)&TY, (void *)&ntx, (void *)&seq,
+                  (void *)&ccnt, (void *)&err};
   return cudaLaunchCooperativeKernel(fn, dim3(ntiles), dim3(nthreads), args, smem, s);
 }

@@ -72,7 +72,11 @@ struct DevCommon {
   double *tr_ch[2], *tr_ub[2], *tr_vb[2];
   double *tr_acc[6];  // mch, mch2, ub, vb accumulators; first-substep viscosity (u, v)
   unsigned *bar;   // [0] arrival count, [1] generation
-  unsigned long long *tile_flag;  // per-tile progress of the barotropic kernel (monotone across launches)
+  // messages between the tiles of the resident barotropic kernels: one
+  // 16-byte {value, sequence number} word per point and field (ch, ub, vb), two
+  // substeps deep: xch[(2-parity * 3 + field) * n2 + point]; null on domains
+  // too large to be resident
+  ulonglong2 *xch;
   int *err;        // [0] timeout flag, [1] watchdog flag
   // longest a device-side wait (the barotropic kernels' grid barriers) may
   // take before it gives up and sets err[0] (ns of global time)
@@ -161,6 +165,50 @@ PD bool wait_count(unsigned long long *cnt, unsigned long long want, int *err, u
     if (e.load(cuda::memory_order_relaxed) != 0) return false;
     if (global_ns() - t0 > limit_ns) break;
     if (it > 1024) __nanosleep(32);
+  }
+  e.store(1, cuda::memory_order_relaxed);
+  return false;
+}
+
+// A message of the resident barotropic kernels: a value and its sequence
+// number written as one 128-bit relaxed store, which is single-copy atomic,
+// so a reader that sees the expected number has the value that came with it.
+// The number replaces both the fence before a flag and the second round trip
+// after it: what a neighbour waits for is one store and one load through L2.
+PD void xch_put(ulonglong2 *a, double v, unsigned long long seq) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(a),
+               "l"(__double_as_longlong(v)), "l"(seq)
+               : "memory");
+}
+PD bool xch_get(const ulonglong2 *a, unsigned long long seq, double &v) {
+  long long x;
+  unsigned long long n;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(x), "=l"(n)
+               : "l"(a)
+               : "memory");
+  v = __longlong_as_double(x);
+  return n == seq;
+}
+// One thread's bounded wait for the N messages at a[0 .. N-1] (their loads in
+// flight together; a null address needs no message): false when another
+// thread has set *err or after limit_ns of global time (then *err is set;
+// an iteration cap bounds the loop as well).
+template <int N>
+PD bool xch_wait(const ulonglong2 *const (&a)[N], unsigned long long seq, double (&v)[N], int *err,
+                 unsigned long long limit_ns) {
+  cuda::atomic_ref<int, cuda::thread_scope_device> e(*err);
+  unsigned long long t0 = 0;
+  for (int it = 0; it < (1 << 26); ++it) {
+    bool ok = true;
+    #pragma unroll
+    for (int f = 0; f < N; ++f)
+      if (a[f] && !xch_get(a[f], seq, v[f])) ok = false;
+    if (ok) return true;
+    const unsigned long long t = global_ns();
+    if (it == 0) t0 = t;
+    else if (t - t0 > limit_ns) break;
+    if ((it & 15) == 15 && e.load(cuda::memory_order_relaxed) != 0) return false;
   }
   e.store(1, cuda::memory_order_relaxed);
   return false;

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -369,7 +370,7 @@ struct pcom_handle {
   int ntiles1 = 0;
   unsigned long long *d_cnt1 = nullptr;
   double *frc_months = nullptr;  // taux, tauy, t, s, pa: [5][12][nj][ni]
-  unsigned long long trop_epoch = 0;  // barrier arrivals of the barotropic kernel so far
+  unsigned long long trop_seq = 0;  // sequence base of the next resident barotropic launch (message_space)
   // second stream of the full step: phases that share no array with the
   // main stream's concurrent phases run on it, forked and joined by events
   bool overlap = true;
@@ -433,6 +434,15 @@ struct Prof {
   }
 };
 
+// First sequence number of a range of 2^40 that no other handle or batch of
+// this process uses: a handle's messages (DevCommon::xch) are written by its own
+// launches and by the launches of every batch it is a member of, and a number
+// must never repeat in them.
+unsigned long long message_space() {
+  static std::atomic<unsigned long long> n{0};
+  return ++n << 40;
+}
+
 int sync_check(pcom_handle *h) {
   CK(cudaStreamSynchronize(h->stream));
   if (h->side) CK(cudaStreamSynchronize(h->side));
@@ -444,9 +454,7 @@ int sync_check(pcom_handle *h) {
   if (err[0]) {
     cudaMemsetAsync(h->D.err, 0, sizeof err, h->stream);
     cudaMemsetAsync(h->D.bar, 0, 2 * sizeof(unsigned), h->stream);
-    cudaMemsetAsync(h->D.tile_flag, 0, sizeof(unsigned long long), h->stream);
     cudaStreamSynchronize(h->stream);
-    h->trop_epoch = 0;
     return fail(PCOM_ERR_TIMEOUT, "a device-side grid barrier gave up waiting (bounded spin)");
   }
   return PCOM_OK;
@@ -492,7 +500,7 @@ int pick_trop_config(pcom_handle *h) {
   // tiling with the fewest tiles (fewest CTAs at the grid barrier)
   h->trop_resident = false;
   h->trop_multi = false;
-  if (h->D.separable && (h->trop_force == 0 || h->trop_force == 1)) {
+  if (h->D.separable && h->D.xch && (h->trop_force == 0 || h->trop_force == 1)) {
     int best_n = 1 << 30, bx = 0, by = 0;
     const int mb = trop_fast_max_blocks(24, 18);
     for (int ty = 6; ty <= 40; ++ty)
@@ -631,12 +639,11 @@ int do_trop(pcom_handle *h) {
   Prof p(h, "int_trop");
   cudaError_t e;
   if (h->trop_resident) {
-    // the kernel's barrier counter is monotone: pass the arrivals so far
     if (h->mixed && trop_mixed_max_blocks(h->trop_tx, h->trop_ty) >= h->trop_blocks)
-      e = launch_trop_mixed(h->D, h->trop_tx, h->trop_ty, h->trop_epoch, h->stream);
+      e = launch_trop_mixed(h->D, h->trop_tx, h->trop_ty, h->trop_seq, h->stream);
     else
-      e = launch_trop_fast(h->D, h->trop_tx, h->trop_ty, h->trop_epoch, h->stream);
-    h->trop_epoch += (unsigned long long)h->D.nstep * (unsigned long long)h->trop_blocks;
+      e = launch_trop_fast(h->D, h->trop_tx, h->trop_ty, h->trop_seq, h->stream);
+    h->trop_seq += (unsigned long long)h->D.nstep;
   } else if (h->trop_multi && h->mixed) {
     e = launch_trop_multi_mixed(h->D, h->mm, h->d_tiles1, h->ntiles1, h->trop_tx, h->trop_ty, h->trop_blocks,
                                 h->d_cnt1, h->D.err, h->stream);
@@ -1082,9 +1089,13 @@ int pcom_gpu_create(const pcom_dims *dims, pcom_handle **out) {
   if (!rc) rc = h->alloc(&err, 4);
   if (!rc) rc = h->alloc(&h->d_count, 1);
   {
-    unsigned long long *tf = nullptr;
-    if (!rc) rc = h->alloc(&tf, 4096);
-    D.tile_flag = tf;
+    // a resident kernel has one thread per region point and at most
+    // kResThreads of them per SM; the padded plane is at most twice the
+    // interior
+    int nsm = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+    if (!rc && n2 <= 2LL * 640 * nsm) rc = h->alloc(&D.xch, 6 * n2);
+    h->trop_seq = message_space();
   }
   D.bar = bar; D.err = err;
   if (rc) { pcom_gpu_destroy(h); return rc; }
@@ -1704,8 +1715,8 @@ int pcom_gpu_trop_floor(pcom_handle *h, double *ms) {
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   CK(cudaEventRecord(e0, h->stream));
-  cudaError_t e = launch_trop_floor(h->D, h->trop_tx, h->trop_ty, h->trop_epoch, h->stream);
-  if (e == cudaSuccess) h->trop_epoch += (unsigned long long)h->D.nstep * (unsigned long long)h->trop_blocks;
+  cudaError_t e = launch_trop_floor(h->D, h->trop_tx, h->trop_ty, h->trop_seq, h->stream);
+  if (e == cudaSuccess) h->trop_seq += (unsigned long long)h->D.nstep;
   CK(cudaEventRecord(e1, h->stream));
   int rc = sync_check(h);
   float t = 0.f;
@@ -1789,6 +1800,8 @@ struct pcom_batch {
   int TX = 24, TY = 18;
   int max_resident = 0;  // > 0: cap on the tiles of one resident group
   int64_t launches = 0;  // kernels this batch launched
+  // [0] barrier arrivals of the multi-tile kernel, [1] sequence base of the
+  // resident groups' messages
   unsigned long long *cnt = nullptr;
   int *err = nullptr;
   // per-phase device copies of the members' Dev (phase = ring indices)
@@ -1838,7 +1851,7 @@ int batch_tiles(pcom_batch *b, int TX, int TY) {
   std::vector<TileRef> big;               // members that cannot be resident
   for (int m : order) {
     const int nt = (int)mt[m].size();
-    if (nt > cap) {
+    if (nt > cap || !b->hs[m]->D.xch) {
       big.insert(big.end(), mt[m].begin(), mt[m].end());
       continue;
     }
@@ -1882,7 +1895,7 @@ int batch_tiles(pcom_batch *b, int TX, int TY) {
 // the barotropic subcycles of all members
 cudaError_t batch_trop(pcom_batch *b, const Dev *dP) {
   for (const pcom_batch::TropGroup &g : b->groups) {
-    cudaError_t e = g.resident ? launch_trop_group(dP, g.d, g.ntiles, b->TX, b->TY, b->cnt, b->err, b->stream)
+    cudaError_t e = g.resident ? launch_trop_group(dP, g.d, g.ntiles, b->TX, b->TY, b->nstep, b->cnt + 1, b->err, b->stream)
                                : launch_trop_batch(dP, g.d, g.ntiles, b->TX, b->TY, g.nblocks, b->cnt, b->err, b->stream);
     if (e != cudaSuccess) return e;
   }
@@ -1992,9 +2005,11 @@ int pcom_gpu_batch_create(pcom_handle *const *hs, int32_t n, pcom_batch **out) {
       b->member_streams.push_back(h->stream);
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc(&b->cnt, sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&b->cnt, 2 * sizeof(unsigned long long));
   if (e == cudaSuccess) { b->allocs.push_back(b->cnt); e = cudaMalloc(&b->err, sizeof(int)); }
   if (e == cudaSuccess) { b->allocs.push_back(b->err); e = cudaMemsetAsync(b->err, 0, sizeof(int), b->stream); }
+  const unsigned long long cnt0[2] = {0, message_space()};
+  if (e == cudaSuccess) e = cudaMemcpy(b->cnt, cnt0, sizeof cnt0, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) { delete b; return fail(PCOM_ERR_CUDA, "batch scratch: %s", cudaGetErrorString(e)); }
   int rc = batch_tiles(b, 24, 18);
   if (rc) { delete b; return rc; }
@@ -2081,7 +2096,9 @@ int pcom_gpu_batch_step_async(pcom_batch *b, int64_t tctr_i) {
   if (rc) return rc;
   rc = batch_join_out(b);
   if (rc) return rc;
-  b->launches += 13 + (int64_t)b->groups.size();  // kernels of one batched step
+  // kernels of one batched step (a resident group: its sequence base, then its tiles)
+  b->launches += 13 + (int64_t)b->groups.size();
+  for (const pcom_batch::TropGroup &g : b->groups) b->launches += g.resident;
   for (pcom_handle *h : b->hs) {
     h->D.ab3_mode = 0;
     h->n_ch++; h->n_uv++; h->n_ssh++; h->n_w++; h->n_ts++;

@@ -44,12 +44,13 @@ cudaError_t launch_trop_res(const Dev &P, int TX, int TY, cudaStream_t s);
 int trop_res_max_blocks(int TX, int TY);
 // the same with reciprocal divisions (handle path)
 size_t trop_fast_smem_bytes(int TX, int TY);
-cudaError_t launch_trop_fast(const Dev &P, int TX, int TY, unsigned long long epoch, cudaStream_t s);
+// (seq + n numbers the messages of substep n: no two launches share a number)
+cudaError_t launch_trop_fast(const Dev &P, int TX, int TY, unsigned long long seq, cudaStream_t s);
 // the resident kernel's synchronisation skeleton (latency floor), same grid
-cudaError_t launch_trop_floor(const Dev &P, int TX, int TY, unsigned long long epoch, cudaStream_t s);
+cudaError_t launch_trop_floor(const Dev &P, int TX, int TY, unsigned long long seq, cudaStream_t s);
 int trop_fast_max_blocks(int TX, int TY);
 // mixed path: the resident kernel with FP32 arithmetic outside the bottom pressure
-cudaError_t launch_trop_mixed(const Dev &P, int TX, int TY, unsigned long long epoch, cudaStream_t s);
+cudaError_t launch_trop_mixed(const Dev &P, int TX, int TY, unsigned long long seq, cudaStream_t s);
 int trop_mixed_max_blocks(int TX, int TY);
 // batched barotropic subcycle: one persistent launch over the tiles of all members
 struct TileRef {
@@ -81,9 +82,10 @@ cudaError_t launch_trop_batch(const Dev *dPs, const TileRef *dtiles, int ntiles,
 cudaError_t launch_trop_multi(const Dev &P, const TileRef *dtiles, int ntiles, int TX, int TY, int nblocks,
                               unsigned long long *cnt, int *err, cudaStream_t s);
 // resident form: one tile per CTA, coefficients in registers (the fast
-// kernel over a tile list); all tiles of the group must be co-resident
+// kernel over a tile list); all tiles of the group must be co-resident.  *cnt
+// is the sequence base, advanced by nstep before the launch
 int trop_group_max_blocks(int TX, int TY);
-cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY,
+cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nstep,
                               unsigned long long *cnt, int *err, cudaStream_t s);
 
 // the model constants (literal precision per PCOM_LIT_R8)
