@@ -1067,9 +1067,12 @@ size_t trop_fast_smem_bytes(int TX, int TY) {
 
 namespace {
 // the single-domain kernel for a tile shape: the fixed-shape form where one
-// is compiled (the 24 x 18 tiles of the 1-degree 360 x 160 domain)
+// is compiled, the general one otherwise
 const void *fast_kernel(int TX, int TY) {
-  if (TX == 24 && TY == 18) return (const void *)k_trop_fast<false, 24, 18>;
+#define PCOM_FAST_SHAPE(x, y) \
+  if (TX == (x) && TY == (y)) return (const void *)k_trop_fast<false, (x), (y)>;
+  PCOM_TROP_SHAPES(PCOM_FAST_SHAPE)
+#undef PCOM_FAST_SHAPE
   return (const void *)k_trop_fast<false>;
 }
 // the group kernel for a tile shape: a fixed-shape form for each tile shape

@@ -308,9 +308,13 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 namespace {
-// the fixed-shape form for the 24 x 18 tiles of the 1-degree 360 x 160 domain
+// the fixed-shape form for a tile shape where one is compiled, the general
+// one otherwise
 const void *mixed_kernel(int TX, int TY) {
-  if (TX == 24 && TY == 18) return (const void *)k_trop_mixed<24, 18>;
+#define PCOM_MIXED_SHAPE(x, y) \
+  if (TX == (x) && TY == (y)) return (const void *)k_trop_mixed<(x), (y)>;
+  PCOM_TROP_SHAPES(PCOM_MIXED_SHAPE)
+#undef PCOM_MIXED_SHAPE
   return (const void *)k_trop_mixed<>;
 }
 }  // namespace

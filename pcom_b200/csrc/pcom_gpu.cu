@@ -496,27 +496,44 @@ int apply_staged_forcing(pcom_handle *h) {
 }
 
 int pick_trop_config(pcom_handle *h) {
-  // resident kernel: one tile per CTA, one region point per thread; pick the
-  // tiling with the fewest tiles (fewest CTAs at the grid barrier)
+  // resident kernel: one tile per CTA, one region point per thread
   h->trop_resident = false;
   h->trop_multi = false;
   if (h->D.separable && h->D.xch && (h->trop_force == 0 || h->trop_force == 1)) {
-    int best_n = 1 << 30, bx = 0, by = 0;
+    auto tiles = [&](int tx, int ty) { return ((h->dims.glo_ni + tx - 1) / tx) * ((h->nj + ty - 1) / ty); };
+    auto take = [&](int tx, int ty, int n) {
+      h->trop_resident = true;
+      h->trop_tx = tx;
+      h->trop_ty = ty;
+      h->trop_blocks = n;
+      return PCOM_OK;
+    };
+    // the compiled shape with the fewest warps per CTA whose tiles fit one
+    // per SM, then the fewest tiles: a substep's stages issue every warp's
+    // instructions on one SM, while its messages cost the same whatever the
+    // number of tiles
+    int nsm = 0, best_w = 1 << 30, best_n = 0, bx = 0, by = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+#define PCOM_TRY_SHAPE(x, y)                                                                   \
+  {                                                                                            \
+    const int n_ = tiles((x), (y)), w_ = (((x) + 4) * ((y) + 4) + 31) / 32;                    \
+    if (n_ <= nsm && (w_ < best_w || (w_ == best_w && n_ < best_n))) { best_w = w_; best_n = n_; bx = (x); by = (y); } \
+  }
+    PCOM_TROP_SHAPES(PCOM_TRY_SHAPE)
+#undef PCOM_TRY_SHAPE
+    if (bx > 0 && trop_fast_max_blocks(bx, by) >= best_n) return take(bx, by, best_n);
+    // a domain that only another shape covers: the fewest tiles
+    best_n = 1 << 30;
+    bx = by = 0;
     const int mb = trop_fast_max_blocks(24, 18);
     for (int ty = 6; ty <= 40; ++ty)
       for (int tx = 6; tx <= 60; ++tx) {
         if (!trop_res_fits(tx, ty)) continue;
-        const int nt = ((h->dims.glo_ni + tx - 1) / tx) * ((h->nj + ty - 1) / ty);
+        const int nt = tiles(tx, ty);
         if (nt > mb) continue;
         if (nt < best_n || (nt == best_n && (tx + 4) * (ty + 4) < (bx + 4) * (by + 4))) { best_n = nt; bx = tx; by = ty; }
       }
-    if (bx > 0 && trop_fast_max_blocks(bx, by) >= best_n) {
-      h->trop_resident = true;
-      h->trop_tx = bx;
-      h->trop_ty = by;
-      h->trop_blocks = best_n;
-      return PCOM_OK;
-    }
+    if (bx > 0 && trop_fast_max_blocks(bx, by) >= best_n) return take(bx, by, best_n);
   }
   // too large to be resident: the multi-tile kernel (several tiles per CTA,
   // coefficients from L2) over this domain's tiles

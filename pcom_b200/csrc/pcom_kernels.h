@@ -34,6 +34,13 @@ enum {
 };
 void launch_batch(int kernel, const Dev *dPs, const BatchShape &b, int arg, cudaStream_t s);
 
+// Tile shapes the single-domain resident kernels (FP64 and mixed) are
+// compiled for, by warps per CTA of their (TX+4) x (TY+4) region: 4, 5, 6, 8, 8,
+// 9, 10, 12, 14, 15, 18, 20, 20
+#define PCOM_TROP_SHAPES(S) \
+  S(8, 6) S(12, 6) S(12, 8) S(16, 8) S(12, 12) S(16, 10) S(16, 12) S(20, 12) S(24, 12) S(20, 16) S(24, 16) S(24, 18) \
+      S(28, 16)
+
 size_t trop_smem_bytes(int TX, int TY);
 cudaError_t launch_trop(const Dev &P, int TX, int TY, int nblocks, cudaStream_t s);
 int trop_max_blocks(int TX, int TY);
