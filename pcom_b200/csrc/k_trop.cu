@@ -700,10 +700,13 @@ enum {
   X_CH, X_UB, X_VB,
   X_S1, X_X2,  // supb1, supb2*rh3 (reused for the corrector's supb)
   X_PRED,
-  X_A1U, X_A1V, X_GY, X_CN,
-  X_A2U, X_A2V, X_GX, X_CE,
+  X_A1U, X_A1V, X_A2U, X_A2V,
   X_COUNT
 };
+// doubles before the first field and after the last: the stages evaluate
+// every thread's point without branches and may read (and discard) a
+// neighbour that is outside the region
+__host__ __device__ constexpr int x_pad(int W) { return W + 1; }
 }  // namespace
 
 template <bool GROUP, int CTX = 0, int CTY = 0>
@@ -718,8 +721,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
   int *const err = GROUP ? gerr : P.err;
   const int ni = P.ni, nj = P.nj, njm = P.njm, G = P.glo_ni;
   const int W = TX + 4, H = TY + 4, RS = W * H;
-  double *vx = sm + X_COUNT * RS;  // dxx[1..4], 1/dxx[1..4] over lx: 8*W
-  double *vy = vx + 8 * W;         // 19 vectors over ly (see below)
+  double *const fs = sm + x_pad(W);
+  double *vx = fs + X_COUNT * RS + x_pad(W) + 32;  // dxx[1..4], 1/dxx[1..4] over lx: 8*W
+  double *vy = vx + 8 * W;                         // 19 vectors over ly (see below)
   const double a = P.c.a, bt = (double)P.bt, gamma_b = P.c.gamma_b;
   const int nstep = P.nstep;
   const int tid = threadIdx.x;
@@ -734,20 +738,22 @@ __global__ void __launch_bounds__(kResThreads, 1)
   const int rr0 = R0 - 2, jj0 = J0 - 2;
   auto ring_i = [&](int r) { r %= G; if (r < 0) r += G; return r + 2; };
 
-  // 1-D metrics and the reciprocals of every divisor (dvr)
+  // 1-D metrics and the reciprocals of every divisor (dvr).  Twice dxx[1] and
+  // dxy[1] and half their reciprocals: their dividends are differences of
+  // means, and a scaling by 2 is exact, so the halves of the means, of
+  // sqrt(ter()) and of the pressure-gradient terms all move into constants.
   for (int l = tid; l < W; l += blockDim.x) {
     const int i = ring_i(rr0 + l);
     for (int g = 1; g <= 4; ++g) {
-      vx[(g - 1) * W + l] = ld(P.dxx1d[g], i - 1);
-      vx[(4 + g - 1) * W + l] = ld(P.rdxx1d[g], i - 1);
+      vx[(g - 1) * W + l] = (g == 1 ? 2.0 : 1.0) * ld(P.dxx1d[g], i - 1);
+      vx[(4 + g - 1) * W + l] = (g == 1 ? 0.5 : 1.0) * ld(P.rdxx1d[g], i - 1);
     }
   }
   for (int l = tid; l < H; l += blockDim.x) {
-    const int j = jj0 + l;
-    if (j < 1 || j > nj) continue;
+    const int j = min(max(jj0 + l, 1), nj);
     for (int g = 1; g <= 4; ++g) {
-      vy[(g - 1) * H + l] = ld(P.dxy1d[g], j - 1);
-      vy[(4 + g - 1) * H + l] = ld(P.rdxy1d[g], j - 1);
+      vy[(g - 1) * H + l] = (g == 1 ? 2.0 : 1.0) * ld(P.dxy1d[g], j - 1);
+      vy[(4 + g - 1) * H + l] = (g == 1 ? 0.5 : 1.0) * ld(P.rdxy1d[g], j - 1);
       vy[(8 + g - 1) * H + l] = ld(P.rh1d[g], j - 1);
     }
     vy[12 * H + l] = ld(P.arh1d[1], j - 1);
@@ -758,27 +764,20 @@ __global__ void __launch_bounds__(kResThreads, 1)
     vy[17 * H + l] = ld(P.aarh3, j - 1);
     vy[18 * H + l] = ld(P.raarh3, j - 1);
   }
-  auto DXX = [&](int g, int lx) { return vx[(g - 1) * W + lx]; };
-  auto RDXX = [&](int g, int lx) { return vx[(4 + g - 1) * W + lx]; };
-  auto DXY = [&](int g, int ly) { return vy[(g - 1) * H + ly]; };
-  auto RDXY = [&](int g, int ly) { return vy[(4 + g - 1) * H + ly]; };
-  auto RH = [&](int g, int ly) { return vy[(8 + g - 1) * H + ly]; };
   const double ra = P.ra;
-  auto S = [&](int f, int p) -> double & { return sm[f * RS + p]; };
 
   // this thread's region point
   const int p = tid;
-  const int lx = p % W, ly = p / W;
+  const int ly = min(p / W, H - 1), lx = p - ly * W < W ? p - ly * W : 0;
   const int j = jj0 + ly;
-  const bool active = p < RS && j >= 1 && j <= nj;
+  const bool inR = p < RS;
+  const bool active = inR && j >= 1 && j <= nj;
   const int i = active ? ring_i(rr0 + lx) : 2;
   const long long q = active ? I2(P, i, j) : 0;
   const bool nrow = j <= njm, srow = j >= 2;
   const bool inS2 = active && lx < tw + 3 && ly < th + 3;
   const bool inS4 = active && lx >= 1 && lx < tw + 3 && ly >= 1 && ly < th + 3;
   const bool inS6 = active && lx >= 1 && lx < tw + 2 && ly >= 1 && ly < th + 2;
-  const bool inN = active && lx >= 1 && lx < tw + 3 && ly >= 1 && ly < th + 2;
-  const bool inE = active && lx >= 1 && lx < tw + 2 && ly >= 1 && ly < th + 3;
   const bool inS8 = active && lx >= 2 && lx < tw + 2 && ly >= 2 && ly < th + 2;
   // points some tile's ring covers (this tile's own, where the ring wraps)
   const bool border = inS8 && (lx < 4 || lx >= tw || ly < 4 || ly >= th);
@@ -786,21 +785,27 @@ __global__ void __launch_bounds__(kResThreads, 1)
   // region are nobody's)
   const bool ring = active && !inS8 && lx < tw + 4 && ly < th + 4;
   const int levu = active ? __ldg(P.lev_u + q) : 0, levt = active ? __ldg(P.lev_t + q) : 0;
-  const double seau = (double)(levu >= 1), mskt1 = (double)(levt >= 1);
-  const double prh_u = active ? ld(P.prh_u, q) : 1.0, prh_t = active ? ld(P.prh_t, q) : 1.0;
+  const double seau = (double)(levu >= 1);
+  // dtbt on sea, 0 on land: mask * x * dtbt = x * (mask * dtbt), masks being 0 or 1
+  const double sbt = seau * bt, tbt = (double)(levt >= 1) * bt, seau4 = 0.25 * seau;
+  const double prh_uh = 0.5 * (active ? ld(P.prh_u, q) : 1.0), prh_t = active ? ld(P.prh_t, q) : 1.0;
   const double rprh_t = active ? ld(P.rprh_t, q) : 1.0;
   const double rden = active ? ld(P.rwt, q) : 1.0;  // 1 / (1 + (0.5 cor dtbt)^2)
+  // where sqrt(ter()) is 1 (land, and points that need none: 2 sqrt(ter())
+  // = sqrt(4)) or 0 (row nj, where ter leaves 0)
+  const bool s2sea = inS2 && levu > 0 && nrow, s2zero = levu > 0 && !nrow, s6sea = inS6 && levu > 0 && nrow;
   // S6 coefficients (shifted where the reference's formulas shift them)
   double sam1 = 0, bxn = 0, bxs = 0, bye = 0, byw = 0, gxn = 0, gxs = 0, gye = 0, gyw = 0;
   double ghx = 0, ghy = 0, cor = 0, ut = 0, vt = 0;
   if (inS6) {
     sam1 = seau * ld(P.am, q);
     bxn = ld(P.bphi[0], q); bye = ld(P.bphi[2], q); byw = ld(P.bphi[3], q + 1);
-    gxn = ld(P.bgra[0], q); gye = ld(P.bgra[2], q); gyw = ld(P.bgra[3], q + 1);
-    if (nrow) { bxs = ld(P.bphi[1], q + ni); gxs = ld(P.bgra[1], q + ni); }
-    ghx = ld(P.graphihx, q); ghy = ld(P.graphihy, q);
+    gxn = 0.5 * ld(P.bgra[0], q); gye = 0.5 * ld(P.bgra[2], q); gyw = 0.5 * ld(P.bgra[3], q + 1);
+    if (nrow) { bxs = ld(P.bphi[1], q + ni); gxs = 0.5 * ld(P.bgra[1], q + ni); }
+    ghx = 2.0 * ld(P.graphihx, q); ghy = 2.0 * ld(P.graphihy, q);
     cor = ld(P.cor, q); ut = ld(P.ut, q); vt = ld(P.vt, q);
   }
+  const double cb = 0.5 * cor * bt, den = 1 + cb * cb;
   double vs0u = 0.0, vs0v = 0.0;
   // accumulators (mod_int.f90:176-180)
   double acc_m = 0, acc_m2 = 0, acc_u = 0, acc_v = 0;
@@ -813,154 +818,123 @@ __global__ void __launch_bounds__(kResThreads, 1)
   double c0 = 0.0, u0 = 0.0, v0 = 0.0;
   if (active && (inS8 || ring)) {
     c0 = __ldcg(P.chp + q);
-    S(X_CH, p) = c0;
-    if (inS2) {
-      u0 = __ldcg(P.ubp + q); v0 = __ldcg(P.vbp + q);
-      S(X_UB, p) = u0; S(X_VB, p) = v0;
-    }
+    if (inS2) { u0 = __ldcg(P.ubp + q); v0 = __ldcg(P.vbp + q); }
   }
+  // this thread's point in each field, and its row's and column's metrics
+  double *const f = fs + p;
+#define S(F, o) f[(F) * RS + (o)]
+#define MVX(n) vx[(n) * W + lx]
+#define MVY(n) vy[(n) * H + ly]
+  if (inR) { S(X_CH, 0) = c0; S(X_UB, 0) = u0; S(X_VB, 0) = v0; }
   __syncthreads();
 
+  // The stages run straight through for every thread, whatever its point
+  // belongs to: values at points a stage does not cover are formed from
+  // whatever is there and are never read by a point it does cover.  With a
+  // branch per part the parts' latencies added up (a substep of 4 to 20 warps
+  // on an SM is bound by its dependency chains, not by issue).
   for (int nt = 1; nt <= nstep; ++nt) {
     ulonglong2 *const out = P.xch + (long long)(nt & 1) * 3 * P.n2 + q;  // this substep's words of this point
-    // S2: sch = sqrt(ter(ch)) on U, supb
-    double s1 = 0.0, x2 = 0.0;
-    if (inS2) {
-      double sch = 1.0;
-      if (levu > 0) {
-        const double w = nrow ? (c0 + S(X_CH, p + W) + S(X_CH, p + 1) + S(X_CH, p + W + 1)) * 0.25 : 0.0;
-        sch = sqrt(w);
-      }
-      const double ps = prh_u * sch;
+    // S2: sch = sqrt(ter(ch)) on U and the fluxes supb; the viscosity's
+    // differences p1(ub)/rh4 on N and p2(ub) rh2 on E
+    double s1, x2, a1u, a1v, a2u, a2v;
+    {
+      const double w = c0 + S(X_CH, W) + S(X_CH, 1) + S(X_CH, W + 1);
+      double sch = sqrt(s2sea ? w : 4.0);
+      if (s2zero) sch = 0.0;
+      const double ps = prh_uh * sch;
       s1 = ps * u0;
-      x2 = ps * v0 * RH(3, ly);
-      S(X_S1, p) = s1;
-      S(X_X2, p) = x2;
+      x2 = ps * v0 * MVY(10);
+      const double dx4 = MVX(3), rdx4 = MVX(7), rh4 = MVY(11), rrh4 = MVY(16);
+      a1u = dvr(dvr(u0 - S(X_UB, -1), dx4, rdx4), rh4, rrh4);
+      a1v = dvr(dvr(v0 - S(X_VB, -1), dx4, rdx4), rh4, rrh4);
+      const double dy2 = MVY(1), rdy2 = MVY(5), rh2 = MVY(9);
+      a2u = dvr(u0 - S(X_UB, -W), dy2, rdy2) * rh2;
+      a2v = dvr(v0 - S(X_VB, -W), dy2, rdy2) * rh2;
+      if (!srow) a2u = a2v = 0.0;
+      if (inR) {
+        S(X_S1, 0) = s1;
+        S(X_X2, 0) = x2;
+        S(X_A1U, 0) = a1u;
+        S(X_A1V, 0) = a1v;
+        S(X_A2U, 0) = a2u;
+        S(X_A2V, 0) = a2v;
+      }
     }
     __syncthreads();
-    // S4: predictor ch; the ter U->E (rows >= 2) and U->N means of supb are
-    // formed here from the staged supb
-    double pred = 0.0;
-    if (inS4) {
-      // tE at (i, j) and (i-1, j): j >= 2 ? 0.5 (s1(j-1) + s1(j)) : 0
-      const double tEc = srow ? 0.5 * (S(X_S1, p - W) + s1) : 0.0;
-      const double tEw = srow ? 0.5 * (S(X_S1, p - W - 1) + S(X_S1, p - 1)) : 0.0;
-      const double A = dvr(tEc - tEw, DXX(1, lx), RDXX(1, lx));
-      double B = 0.0;
-      if (srow) {
-        // tN at (i, j) and (i, j-1): 0.5 (x2(i-1) + x2(i))
-        const double tNc = 0.5 * (S(X_X2, p - 1) + x2);
-        const double tNs = 0.5 * (S(X_X2, p - W - 1) + S(X_X2, p - W));
-        B = dvr(tNc - tNs, DXY(1, ly), RDXY(1, ly));
-      }
-      const double div = dvr(A + B, vy[12 * H + ly], vy[13 * H + ly]);
-      if (levt > 0) pred = c0 - dvr(div * bt * gamma_b, prh_t, rprh_t);
-      else pred = (nt == 1) ? land_ch0 : c0;
-      S(X_PRED, p) = pred;
-    }
-    __syncthreads();
-    // S5: sch on U; N- and E-grid intermediates
-    double sche = 1.0, a1u = 0.0, a1v = 0.0, gy = 0.0, cn = 0.0, a2u = 0.0, a2v = 0.0, gx = 0.0, ce = 0.0;
-    if (inS6 && levu > 0) {
-      const double w = nrow ? (pred + S(X_PRED, p + W) + S(X_PRED, p + 1) + S(X_PRED, p + W + 1)) * 0.25 : 0.0;
-      sche = sqrt(w);
-    }
-    if (inN) {
-      const double dx4 = DXX(4, lx), rdx4 = RDXX(4, lx), rh4 = RH(4, ly), rrh4 = vy[16 * H + ly];
-      a1u = dvr(dvr(u0 - S(X_UB, p - 1), dx4, rdx4), rh4, rrh4);
-      a1v = dvr(dvr(v0 - S(X_VB, p - 1), dx4, rdx4), rh4, rrh4);
-      if (nrow) {
-        gy = dvr(dvr(S(X_PRED, p + W) - pred, DXY(4, ly), RDXY(4, ly)), a, ra);
-        cn = 0.5 * (pred + S(X_PRED, p + W));
-      }
-      S(X_A1U, p) = a1u;
-      S(X_A1V, p) = a1v;
-      S(X_GY, p) = gy;
-      S(X_CN, p) = cn;
-    }
-    if (inE) {
-      const double rh2 = RH(2, ly);
-      if (srow) {
-        const double dy2 = DXY(2, ly), rdy2 = RDXY(2, ly);
-        a2u = dvr(u0 - S(X_UB, p - W), dy2, rdy2) * rh2;
-        a2v = dvr(v0 - S(X_VB, p - W), dy2, rdy2) * rh2;
-      }
-      gx = dvr(dvr(S(X_PRED, p + 1) - pred, DXX(2, lx), RDXX(2, lx)), vy[14 * H + ly], vy[15 * H + ly]);
-      ce = 0.5 * (pred + S(X_PRED, p + 1));
-      S(X_A2U, p) = a2u;
-      S(X_A2V, p) = a2v;
-      S(X_GX, p) = gx;
-      S(X_CE, p) = ce;
-    }
-    __syncthreads();
-    // S6: corrector velocity (viscosity, pressure gradient, Coriolis adjustment)
-    double ubc = 0.0, vbc = 0.0;
-    if (inS6) {
-      const double rh3 = RH(3, ly), dx3 = DXX(3, lx), rdx3 = RDXX(3, lx), dy3 = DXY(3, ly), rdy3 = RDXY(3, ly);
-      const double aarh = vy[17 * H + ly], raarh = vy[18 * H + ly];
-      const double L1u = dvr(S(X_A1U, p + 1) - a1u, dx3, rdx3);
-      const double L1v = dvr(S(X_A1V, p + 1) - a1v, dx3, rdx3);
-      const double L2u = nrow ? dvr(S(X_A2U, p + W) - a2u, dy3, rdy3) : 0.0;
-      const double L2v = nrow ? dvr(S(X_A2V, p + W) - a2v, dy3, rdy3) : 0.0;
-      const double vsu = sam1 * dvr(L1u + L2u, aarh, raarh);
-      const double vsv = sam1 * dvr(L1v + L2v, aarh, raarh);
+    // S4: predictor ch (the ter U->E and U->N means of supb formed from the
+    // staged supb; rows >= 2); the viscosity
+    double pred, dvu, dvv;
+    {
+      double A = dvr((S(X_S1, -W) + s1) - (S(X_S1, -W - 1) + S(X_S1, -1)), MVX(0), MVX(4));
+      double B = dvr((S(X_X2, -1) + x2) - (S(X_X2, -W - 1) + S(X_X2, -W)), MVY(0), MVY(4));
+      if (!srow) A = B = 0.0;
+      const double div = dvr(A + B, MVY(12), MVY(13));
+      pred = c0 - dvr(div * bt * gamma_b, prh_t, rprh_t);
+      if (levt <= 0) pred = nt == 1 ? land_ch0 : c0;
+      const double dx3 = MVX(2), rdx3 = MVX(6), dy3 = MVY(2), rdy3 = MVY(6), aarh = MVY(17), raarh = MVY(18);
+      const double L1u = dvr(S(X_A1U, 1) - a1u, dx3, rdx3), L1v = dvr(S(X_A1V, 1) - a1v, dx3, rdx3);
+      double L2u = dvr(S(X_A2U, W) - a2u, dy3, rdy3), L2v = dvr(S(X_A2V, W) - a2v, dy3, rdy3);
+      if (!nrow) L2u = L2v = 0.0;
+      const double vsu = sam1 * dvr(L1u + L2u, aarh, raarh), vsv = sam1 * dvr(L1v + L2v, aarh, raarh);
       if (nt == 1) { vs0u = vsu; vs0v = vsv; }
-      const double dvu = vsu - vs0u, dvv = vsv - vs0v;
-      double gi1 = 0.0, cg1 = 0.0;
-      if (nrow) {
-        gi1 = 0.5 * (gx * bxn + S(X_GX, p + W) * bxs);
-        cg1 = 0.5 * (ce * gxn + S(X_CE, p + W) * gxs);
-      }
-      const double gi2 = 0.5 * (gy * bye + S(X_GY, p + 1) * byw);
-      const double cg2 = 0.5 * (cn * gye + S(X_CN, p + 1) * gyw);
-      const double pg1 = (gi1 + cg1 + ghx) * seau * sche;
-      const double pg2 = (gi2 + cg2 + ghy) * seau * sche;
-      double p1 = seau * (dvu + ut - pg1 + 0.5 * cor * v0);
-      double p2 = seau * (dvv + vt - pg2 - 0.5 * cor * u0);
-      const double w1 = p1 * bt + u0, w2 = p2 * bt + v0;
-      const double cb = 0.5 * cor * bt;
-      const double den = 1 + cb * cb;
-      double u1 = dvr(w1 + 0.5 * cor * bt * w2, den, rden);
-      double v1 = dvr(w2 - 0.5 * cor * bt * w1, den, rden);
-      u1 = 0.5 * (u1 + u0);
-      v1 = 0.5 * (v1 + v0);
-      p1 = seau * (dvu - pg1 + ut + cor * v1);
-      p2 = seau * (dvv - pg2 + vt - cor * u1);
-      ubc = p1 * bt + u0;
-      vbc = p2 * bt + v0;
+      dvu = vsu - vs0u;
+      dvv = vsv - vs0v;
+      if (inR) S(X_PRED, 0) = pred;
+    }
+    __syncthreads();
+    // S6: sqrt(ter(pred)), the gradients and means of pred on E (rows j and
+    // j + 1) and N (columns i and i + 1), all from the same four values, and
+    // the corrector velocity (pressure gradient, Coriolis adjustment)
+    double ubc, vbc;
+    {
+      const double pe = S(X_PRED, 1), pn = S(X_PRED, W), pne = S(X_PRED, W + 1);
+      const double w = pred + pn + pe + pne;
+      double sch = sqrt(s6sea ? w : 4.0);
+      if (s2zero) sch = 0.0;
+      const double dx2 = MVX(1), rdx2 = MVX(5), dy4 = MVY(3), rdy4 = MVY(7);
+      const double gx0 = dvr(dvr(pe - pred, dx2, rdx2), MVY(14), MVY(15));
+      const double gx1 = dvr(dvr(pne - pn, dx2, rdx2), vy[14 * H + ly + 1], vy[15 * H + ly + 1]);
+      const double gy0 = dvr(dvr(pn - pred, dy4, rdy4), a, ra), gy1 = dvr(dvr(pne - pe, dy4, rdy4), a, ra);
+      double t1 = (gx0 * bxn + gx1 * bxs) + ((pred + pe) * gxn + (pn + pne) * gxs);
+      double t2 = (gy0 * bye + gy1 * byw) + ((pred + pn) * gye + (pe + pne) * gyw);
+      if (!nrow) t1 = t2 = 0.0;
+      const double pg1 = (t1 + ghx) * seau4 * sch, pg2 = (t2 + ghy) * seau4 * sch;
+      const double w1 = (dvu + ut - pg1 + 0.5 * cor * v0) * sbt + u0;
+      const double w2 = (dvv + vt - pg2 - 0.5 * cor * u0) * sbt + v0;
+      const double u1 = 0.5 * (dvr(w1 + cb * w2, den, rden) + u0);
+      const double v1 = 0.5 * (dvr(w2 - cb * w1, den, rden) + v0);
+      ubc = (dvu - pg1 + ut + cor * v1) * sbt + u0;
+      vbc = (dvv - pg2 + vt - cor * u1) * sbt + v0;
       if (border && nt < nstep) {
         xch_put(out + P.n2, ubc, seq + nt);
         xch_put(out + 2 * P.n2, vbc, seq + nt);
       }
-      const double ps = prh_u * sche;
+      const double ps = prh_uh * sch;
       s1 = ps * ubc;
-      x2 = ps * vbc * rh3;
-      S(X_S1, p) = s1;
-      S(X_X2, p) = x2;
+      x2 = ps * vbc * MVY(10);
+      if (inR) {
+        S(X_S1, 0) = s1;
+        S(X_X2, 0) = x2;
+      }
     }
     __syncthreads();
     // S8: corrector ch (with the ter means of the corrector's supb), send, accumulate
     if (inS8) {
-      const double tEc = srow ? 0.5 * (S(X_S1, p - W) + s1) : 0.0;
-      const double tEw = srow ? 0.5 * (S(X_S1, p - W - 1) + S(X_S1, p - 1)) : 0.0;
-      const double A = dvr(tEc - tEw, DXX(1, lx), RDXX(1, lx));
-      double B = 0.0;
-      if (srow) {
-        const double tNc = 0.5 * (S(X_X2, p - 1) + x2);
-        const double tNs = 0.5 * (S(X_X2, p - W - 1) + S(X_X2, p - W));
-        B = dvr(tNc - tNs, DXY(1, ly), RDXY(1, ly));
-      }
-      const double div = dvr(A + B, vy[12 * H + ly], vy[13 * H + ly]);
-      const double chn = c0 - dvr(mskt1 * div * bt, prh_t, rprh_t);
-      if (border && nt < nstep) xch_put(out, chn, seq + nt);
+      double A = dvr((S(X_S1, -W) + s1) - (S(X_S1, -W - 1) + S(X_S1, -1)), MVX(0), MVX(4));
+      double B = dvr((S(X_X2, -1) + x2) - (S(X_X2, -W - 1) + S(X_X2, -W)), MVY(0), MVY(4));
+      if (!srow) A = B = 0.0;
+      const double div = dvr(A + B, MVY(12), MVY(13));
+      c0 = c0 - dvr(div * tbt, prh_t, rprh_t);
+      if (border && nt < nstep) xch_put(out, c0, seq + nt);
       // the next substep's state at this point (nobody reads these three
       // entries in S8)
-      c0 = chn; u0 = ubc; v0 = vbc;
-      S(X_CH, p) = c0;
-      S(X_UB, p) = u0;
-      S(X_VB, p) = v0;
-      if (nt <= nstep / 2) acc_m = acc_m + chn;
-      acc_m2 = acc_m2 + chn;
+      u0 = ubc; v0 = vbc;
+      S(X_CH, 0) = c0;
+      S(X_UB, 0) = u0;
+      S(X_VB, 0) = v0;
+      if (nt <= nstep / 2) acc_m = acc_m + c0;
+      acc_m2 = acc_m2 + c0;
       acc_u = acc_u + ubc;
       acc_v = acc_v + vbc;
     }
@@ -970,19 +944,21 @@ __global__ void __launch_bounds__(kResThreads, 1)
     __syncwarp();
     int fail = 0;
     if (ring) {
-      const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : nullptr, inS2 ? out + 2 * P.n2 : nullptr};
+      const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : out, inS2 ? out + 2 * P.n2 : out};
       double v[3] = {0.0, 0.0, 0.0};
       fail = !xch_wait(in, seq + nt, v, err, P.wait_ns);
       c0 = v[0];
-      S(X_CH, p) = c0;
-      if (inS2) {
-        u0 = v[1]; v0 = v[2];
-        S(X_UB, p) = u0;
-        S(X_VB, p) = v0;
-      }
+      u0 = v[1];
+      v0 = v[2];
+      S(X_CH, 0) = c0;
+      S(X_UB, 0) = u0;
+      S(X_VB, 0) = v0;
     }
     if (__syncthreads_or(fail)) return;
   }
+#undef S
+#undef MVX
+#undef MVY
   if (inS8) {
     const double ub = acc_u / (nstep + 1), vb = acc_v / (nstep + 1);
     const double mch = acc_m / (nstep / 2 + 1), mch2 = acc_m2 / (nstep + 1);
@@ -1001,7 +977,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
 
 // The resident kernel's synchronisation skeleton, its latency floor: the
 // same grid, block and shared memory (so the same residency), and per
-// substep the same five CTA barriers and the same messages to and from the
+// substep the same four CTA barriers and the same messages to and from the
 // tiles around, with none of the arithmetic.  It writes only the message
 // buffer, with sequence numbers of its own.
 __global__ void __launch_bounds__(kResThreads, 1)
@@ -1031,7 +1007,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
   for (int nt = 1; nt < P.nstep; ++nt) {
     ulonglong2 *const out = P.xch + (long long)(nt & 1) * 3 * P.n2 + q;
     #pragma unroll 1
-    for (int b = 0; b < 3; ++b) __syncthreads();  // after S2, S4, S5
+    for (int b = 0; b < 2; ++b) __syncthreads();  // after S2, S4
     if (border) {
       xch_put(out + P.n2, S(X_UB, p), seq + nt);
       xch_put(out + 2 * P.n2, S(X_VB, p), seq + nt);
@@ -1041,7 +1017,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     __syncwarp();
     int fail = 0;
     if (ring) {
-      const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : nullptr, inS2 ? out + 2 * P.n2 : nullptr};
+      const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : out, inS2 ? out + 2 * P.n2 : out};
       double v[3] = {0.0, 0.0, 0.0};
       fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns);
       S(X_CH, p) = v[0];
@@ -1062,7 +1038,8 @@ cudaError_t launch_trop_floor(const Dev &P, int TX, int TY, unsigned long long s
 }
 
 size_t trop_fast_smem_bytes(int TX, int TY) {
-  return ((size_t)X_COUNT * (TX + 4) * (TY + 4) + 8 * (TX + 4) + 19 * (TY + 4)) * sizeof(double);
+  const int W = TX + 4, H = TY + 4;
+  return ((size_t)X_COUNT * W * H + 2 * x_pad(W) + 32 + 8 * W + 19 * H + 1) * sizeof(double);  // (+ 1: row ly + 1 of the last vector)
 }
 
 namespace {

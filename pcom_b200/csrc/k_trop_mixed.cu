@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncwarp();
     int fail = 0;
     if (ring) {
-      const ulonglong2 *const in[2] = {out, inS2 ? out + P.n2 : nullptr};
+      const ulonglong2 *const in[2] = {out, inS2 ? out + P.n2 : out};
       double v[2] = {0.0, 0.0};
       fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns);
       c0 = v[0];

@@ -180,35 +180,37 @@ PD void xch_put(ulonglong2 *a, double v, unsigned long long seq) {
                "l"(__double_as_longlong(v)), "l"(seq)
                : "memory");
 }
-PD bool xch_get(const ulonglong2 *a, unsigned long long seq, double &v) {
+PD void xch_get(const ulonglong2 *a, double &v, unsigned long long &seq) {
   long long x;
-  unsigned long long n;
   asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-               : "=l"(x), "=l"(n)
+               : "=l"(x), "=l"(seq)
                : "l"(a)
                : "memory");
   v = __longlong_as_double(x);
-  return n == seq;
 }
-// One thread's bounded wait for the N messages at a[0 .. N-1] (their loads in
-// flight together; a null address needs no message): false when another
-// thread has set *err or after limit_ns of global time (then *err is set;
-// an iteration cap bounds the loop as well).
+// One thread's bounded wait for the N messages at a[0 .. N-1]: false when
+// another thread has set *err or after limit_ns of global time (then *err is
+// set; an iteration cap bounds the loop as well).  Every poll issues its N
+// loads back to back: with a branch around each (messages some threads do
+// not need) a poll took N round trips.
 template <int N>
 PD bool xch_wait(const ulonglong2 *const (&a)[N], unsigned long long seq, double (&v)[N], int *err,
                  unsigned long long limit_ns) {
   cuda::atomic_ref<int, cuda::thread_scope_device> e(*err);
   unsigned long long t0 = 0;
   for (int it = 0; it < (1 << 26); ++it) {
+    unsigned long long n[N];
+    #pragma unroll
+    for (int f = 0; f < N; ++f) xch_get(a[f], v[f], n[f]);
     bool ok = true;
     #pragma unroll
-    for (int f = 0; f < N; ++f)
-      if (a[f] && !xch_get(a[f], seq, v[f])) ok = false;
+    for (int f = 0; f < N; ++f) ok = ok && n[f] == seq;
     if (ok) return true;
-    const unsigned long long t = global_ns();
-    if (it == 0) t0 = t;
-    else if (t - t0 > limit_ns) break;
-    if ((it & 15) == 15 && e.load(cuda::memory_order_relaxed) != 0) return false;
+    if (it == 0) t0 = global_ns();
+    else if ((it & 7) == 1) {
+      if (global_ns() - t0 > limit_ns) break;
+      if (e.load(cuda::memory_order_relaxed) != 0) return false;
+    }
   }
   e.store(1, cuda::memory_order_relaxed);
   return false;
