@@ -709,8 +709,14 @@ enum {
 __host__ __device__ constexpr int x_pad(int W) { return W + 1; }
 }  // namespace
 
+// threads of a CTA: a fixed single-domain shape's own count, so that small
+// tiles get the registers that let a stage's chains overlap (a group packs
+// several small tiles on an SM)
+template <bool GROUP, int CTX, int CTY>
+constexpr int fast_threads() { return !GROUP && CTX > 0 && (CTX + 4) * (CTY + 4) <= 256 ? ((CTX + 4) * (CTY + 4) + 31) / 32 * 32 : kResThreads; }
+
 template <bool GROUP, int CTX = 0, int CTY = 0>
-__global__ void __launch_bounds__(kResThreads, 1)
+__global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
     k_trop_fast(const __grid_constant__ Dev P0, const Dev *__restrict__ Ps, const TileRef *__restrict__ tiles,
                 int TX, int TY, int ntx, unsigned long long seq0, const unsigned long long *gseq, int *gerr) {
   if (CTX > 0) { TX = CTX; TY = CTY; }

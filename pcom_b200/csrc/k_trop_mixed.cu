@@ -22,11 +22,11 @@ namespace {
 
 constexpr int kThreads = 640;
 
-enum { D_CH, D_PRED, D_CN, D_CE, D_COUNT };  // FP64 region fields
-enum {                                       // FP32 region fields
-  F_UB, F_VB, F_S1, F_X2, F_A1U, F_A1V, F_GY, F_A2U, F_A2V, F_GX,
-  F_COUNT
-};
+enum { D_CH, D_PRED, D_COUNT };                                         // FP64 region fields
+enum { F_UB, F_VB, F_S1, F_X2, F_A1U, F_A1V, F_A2U, F_A2V, F_COUNT };  // FP32 region fields
+// entries before the first and after the last region field (k_trop_fast: the
+// stages run without branches and may read past the region)
+__host__ __device__ constexpr int pad(int W) { return W + 1; }
 constexpr int kVx = 8, kVy = 19;  // FP32 metric vectors over lx and ly
 
 // (ub, vb) as the 64-bit value of one message
@@ -49,8 +49,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ double smd[];
   const int nj = P.nj, njm = P.njm, ni = P.ni, G = P.glo_ni;
   const int W = TX + 4, H = TY + 4, RS = W * H;
-  float *smf = reinterpret_cast<float *>(smd + D_COUNT * RS);
-  float *vx = smf + F_COUNT * RS;
+  double *const ds = smd + pad(W);
+  float *const fs = reinterpret_cast<float *>(ds + D_COUNT * RS + pad(W) + 32) + pad(W);
+  float *vx = fs + F_COUNT * RS + pad(W) + 32;
   float *vy = vx + kVx * W;
   const float ra = (float)P.ra, bt = (float)P.bt, gamma_b = (float)P.c.gamma_b;
   const int nstep = P.nstep;
@@ -60,8 +61,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tw = min(TX, G - R0), th = min(TY, nj - J0 + 1);
   const int rr0 = R0 - 2, jj0 = J0 - 2;
   auto ring_i = [&](int r) { r %= G; if (r < 0) r += G; return r + 2; };
-  auto SD = [&](int f, int p) -> double & { return smd[f * RS + p]; };
-  auto SF = [&](int f, int p) -> float & { return smf[f * RS + p]; };
 
   for (int l = tid; l < W; l += blockDim.x) {
     const int i = ring_i(rr0 + l);
@@ -71,8 +70,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   }
   for (int l = tid; l < H; l += blockDim.x) {
-    const int j = jj0 + l;
-    if (j < 1 || j > nj) continue;
+    const int j = min(max(jj0 + l, 1), nj);
     for (int g = 1; g <= 4; ++g) {
       vy[(g - 1) * H + l] = (float)ld(P.dxy1d[g], j - 1);
       vy[(4 + g - 1) * H + l] = (float)ld(P.rdxy1d[g], j - 1);
@@ -86,22 +84,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     vy[17 * H + l] = (float)ld(P.aarh3, j - 1);
     vy[18 * H + l] = (float)ld(P.raarh3, j - 1);
   }
-  auto RDXX = [&](int g, int lx) { return vx[(4 + g - 1) * W + lx]; };
-  auto RDXY = [&](int g, int ly) { return vy[(4 + g - 1) * H + ly]; };
-  auto RH = [&](int g, int ly) { return vy[(8 + g - 1) * H + ly]; };
 
   const int p = tid;
-  const int lx = p % W, ly = p / W;
+  const int ly = min(p / W, H - 1), lx = p - ly * W < W ? p - ly * W : 0;
   const int j = jj0 + ly;
-  const bool active = p < RS && j >= 1 && j <= nj;
+  const bool inR = p < RS;
+  const bool active = inR && j >= 1 && j <= nj;
   const int i = active ? ring_i(rr0 + lx) : 2;
   const long long q = active ? I2(P, i, j) : 0;
   const bool nrow = j <= njm, srow = j >= 2;
   const bool inS2 = active && lx < tw + 3 && ly < th + 3;
   const bool inS4 = active && lx >= 1 && lx < tw + 3 && ly >= 1 && ly < th + 3;
   const bool inS6 = active && lx >= 1 && lx < tw + 2 && ly >= 1 && ly < th + 2;
-  const bool inN = active && lx >= 1 && lx < tw + 3 && ly >= 1 && ly < th + 2;
-  const bool inE = active && lx >= 1 && lx < tw + 2 && ly >= 1 && ly < th + 3;
   const bool inS8 = active && lx >= 2 && lx < tw + 2 && ly >= 2 && ly < th + 2;
   const bool border = inS8 && (lx < 4 || lx >= tw || ly < 4 || ly >= th);  // as in k_trop_fast
   const bool ring = active && !inS8 && lx < tw + 4 && ly < th + 4;
@@ -110,6 +104,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   const float prh_u = active ? (float)ld(P.prh_u, q) : 1.f;
   const float rprh_t = active ? (float)ld(P.rprh_t, q) : 1.f;
   const float rden = active ? (float)ld(P.rwt, q) : 1.f;
+  // where sqrt(ter()) is 1 (land, points that need none) or 0 (row nj)
+  const bool s2sea = inS2 && levu > 0 && nrow, s2zero = levu > 0 && !nrow, s6sea = inS6 && levu > 0 && nrow;
   float sam1 = 0, bxn = 0, bxs = 0, bye = 0, byw = 0, cor = 0, ut = 0, vt = 0;
   double gxn = 0, gxs = 0, gye = 0, gyw = 0, ghx = 0, ghy = 0;
   if (inS6) {
@@ -132,145 +128,128 @@ __global__ void __launch_bounds__(kThreads, 1)
   float u0 = 0.f, v0 = 0.f;
   if (active && (inS8 || ring)) {
     c0 = __ldcg(P.chp + q);
-    SD(D_CH, p) = c0;
-    if (inS2) {
-      u0 = (float)__ldcg(P.ubp + q); v0 = (float)__ldcg(P.vbp + q);
-      SF(F_UB, p) = u0; SF(F_VB, p) = v0;
-    }
+    if (inS2) { u0 = (float)__ldcg(P.ubp + q); v0 = (float)__ldcg(P.vbp + q); }
   }
+  double *const fd = ds + p;
+  float *const ff = fs + p;
+#define SD(F, o) fd[(F) * RS + (o)]
+#define SF(F, o) ff[(F) * RS + (o)]
+#define RDXX(g) vx[(4 + (g) - 1) * W + lx]
+#define RDXY(g) vy[(4 + (g) - 1) * H + ly]
+#define RH(g) vy[(8 + (g) - 1) * H + ly]
+  if (inR) { SD(D_CH, 0) = c0; SF(F_UB, 0) = u0; SF(F_VB, 0) = v0; }
   __syncthreads();
 
+  // the stages of k_trop_fast, straight through for every thread.  Which
+  // products fuse with a sum is written out (_rn intrinsics) wherever two
+  // roundings are possible, so that the results do not depend on how the
+  // stages are arranged: sums of the neighbours' quantities, the divergence,
+  // the viscosity and its change are of rounded terms, the rest is fused
   for (int nt = 1; nt <= nstep; ++nt) {
     ulonglong2 *const out = P.xch + (long long)(nt & 1) * 3 * P.n2 + q;
-    // S2: fluxes prh_u sqrt(ter(ch)) (ub, vb rh3)
-    float s1 = 0.f, x2 = 0.f;
-    if (inS2) {
-      float sch = 1.f;
-      if (levu > 0) {
-        const double w = nrow ? (c0 + SD(D_CH, p + W) + SD(D_CH, p + 1) + SD(D_CH, p + W + 1)) * 0.25 : 0.0;
-        sch = sqrtf((float)w);
-      }
+    // S2: fluxes prh_u sqrt(ter(ch)) (ub, vb rh3); the viscosity's differences
+    float s1, x2, a1u, a1v, a2u, a2v;
+    {
+      const double w = (c0 + SD(D_CH, W) + SD(D_CH, 1) + SD(D_CH, W + 1)) * 0.25;
+      float sch = sqrtf(s2sea ? (float)w : 1.f);
+      if (s2zero) sch = 0.f;
       const float ps = prh_u * sch;
-      s1 = ps * u0;
-      x2 = ps * v0 * RH(3, ly);
-      SF(F_S1, p) = s1;
-      SF(F_X2, p) = x2;
+      s1 = __fmul_rn(ps, u0);
+      x2 = __fmul_rn(ps * v0, RH(3));
+      const float rdx4 = RDXX(4), rrh4 = vy[16 * H + ly];
+      a1u = __fmul_rn((u0 - SF(F_UB, -1)) * rdx4, rrh4);
+      a1v = __fmul_rn((v0 - SF(F_VB, -1)) * rdx4, rrh4);
+      const float rdy2 = RDXY(2), rh2 = RH(2);
+      a2u = __fmul_rn((u0 - SF(F_UB, -W)) * rdy2, rh2);
+      a2v = __fmul_rn((v0 - SF(F_VB, -W)) * rdy2, rh2);
+      if (!srow) a2u = a2v = 0.f;
+      if (inR) {
+        SF(F_S1, 0) = s1;
+        SF(F_X2, 0) = x2;
+        SF(F_A1U, 0) = a1u;
+        SF(F_A1V, 0) = a1v;
+        SF(F_A2U, 0) = a2u;
+        SF(F_A2V, 0) = a2v;
+      }
     }
     __syncthreads();
-    // S4: predictor ch
-    double pred = 0.0;
-    if (inS4) {
-      const float tEc = srow ? 0.5f * (SF(F_S1, p - W) + s1) : 0.f;
-      const float tEw = srow ? 0.5f * (SF(F_S1, p - W - 1) + SF(F_S1, p - 1)) : 0.f;
-      const float A = (tEc - tEw) * RDXX(1, lx);
-      float B = 0.f;
-      if (srow) {
-        const float tNc = 0.5f * (SF(F_X2, p - 1) + x2);
-        const float tNs = 0.5f * (SF(F_X2, p - W - 1) + SF(F_X2, p - W));
-        B = (tNc - tNs) * RDXY(1, ly);
-      }
-      const float div = (A + B) * vy[13 * H + ly];
-      if (levt > 0) pred = c0 - (double)(div * bt * gamma_b * rprh_t);
-      else pred = (nt == 1) ? land_ch0 : c0;
-      SD(D_PRED, p) = pred;
-    }
-    __syncthreads();
-    // S5: sqrt(ter(pred)) on U; N- and E-grid intermediates
-    float sche = 1.f, a1u = 0.f, a1v = 0.f, gy = 0.f, a2u = 0.f, a2v = 0.f, gx = 0.f;
-    double cn = 0.0, ce = 0.0;
-    if (inS6 && levu > 0) {
-      const double w = nrow ? (pred + SD(D_PRED, p + W) + SD(D_PRED, p + 1) + SD(D_PRED, p + W + 1)) * 0.25 : 0.0;
-      sche = sqrtf((float)w);
-    }
-    if (inN) {
-      const float rdx4 = RDXX(4, lx), rrh4 = vy[16 * H + ly];
-      a1u = (u0 - SF(F_UB, p - 1)) * rdx4 * rrh4;
-      a1v = (v0 - SF(F_VB, p - 1)) * rdx4 * rrh4;
-      if (nrow) {
-        gy = (float)(SD(D_PRED, p + W) - pred) * RDXY(4, ly) * ra;
-        cn = 0.5 * (pred + SD(D_PRED, p + W));
-      }
-      SF(F_A1U, p) = a1u;
-      SF(F_A1V, p) = a1v;
-      SF(F_GY, p) = gy;
-      SD(D_CN, p) = cn;
-    }
-    if (inE) {
-      const float rh2 = RH(2, ly);
-      if (srow) {
-        const float rdy2 = RDXY(2, ly);
-        a2u = (u0 - SF(F_UB, p - W)) * rdy2 * rh2;
-        a2v = (v0 - SF(F_VB, p - W)) * rdy2 * rh2;
-      }
-      gx = (float)(SD(D_PRED, p + 1) - pred) * RDXX(2, lx) * vy[15 * H + ly];
-      ce = 0.5 * (pred + SD(D_PRED, p + 1));
-      SF(F_A2U, p) = a2u;
-      SF(F_A2V, p) = a2v;
-      SF(F_GX, p) = gx;
-      SD(D_CE, p) = ce;
-    }
-    __syncthreads();
-    // S6: corrector velocity
-    float ubc = 0.f, vbc = 0.f;
-    if (inS6) {
-      const float rh3 = RH(3, ly), rdx3 = RDXX(3, lx), rdy3 = RDXY(3, ly), raarh = vy[18 * H + ly];
-      const float L1u = (SF(F_A1U, p + 1) - a1u) * rdx3;
-      const float L1v = (SF(F_A1V, p + 1) - a1v) * rdx3;
-      const float L2u = nrow ? (SF(F_A2U, p + W) - a2u) * rdy3 : 0.f;
-      const float L2v = nrow ? (SF(F_A2V, p + W) - a2v) * rdy3 : 0.f;
-      const float vsu = sam1 * ((L1u + L2u) * raarh);
-      const float vsv = sam1 * ((L1v + L2v) * raarh);
+    // S4: predictor ch; the viscosity
+    double pred;
+    float dvu, dvv;
+    {
+      float tEc = 0.5f * (SF(F_S1, -W) + s1), tEw = 0.5f * (SF(F_S1, -W - 1) + SF(F_S1, -1));
+      const float tNc = 0.5f * (SF(F_X2, -1) + x2), tNs = 0.5f * (SF(F_X2, -W - 1) + SF(F_X2, -W));
+      if (!srow) tEc = tEw = 0.f;
+      const float A = __fmul_rn(tEc - tEw, RDXX(1));
+      float B = __fmul_rn(tNc - tNs, RDXY(1));
+      if (!srow) B = 0.f;
+      const float div = __fadd_rn(A, B) * vy[13 * H + ly];
+      pred = c0 - (double)(div * bt * gamma_b * rprh_t);
+      if (levt <= 0) pred = nt == 1 ? land_ch0 : c0;
+      const float rdx3 = RDXX(3), rdy3 = RDXY(3), raarh = vy[18 * H + ly];
+      const float L1u = __fmul_rn(SF(F_A1U, 1) - a1u, rdx3), L1v = __fmul_rn(SF(F_A1V, 1) - a1v, rdx3);
+      float L2u = __fmul_rn(SF(F_A2U, W) - a2u, rdy3), L2v = __fmul_rn(SF(F_A2V, W) - a2v, rdy3);
+      if (!nrow) L2u = L2v = 0.f;
+      const float vsu = __fmul_rn(sam1, __fadd_rn(L1u, L2u) * raarh);
+      const float vsv = __fmul_rn(sam1, __fadd_rn(L1v, L2v) * raarh);
       if (nt == 1) { vs0u = vsu; vs0v = vsv; }
-      const float dvu = vsu - vs0u, dvv = vsv - vs0v;
-      float gi1 = 0.f;
-      double cg1 = 0.0;
-      if (nrow) {
-        gi1 = 0.5f * (gx * bxn + SF(F_GX, p + W) * bxs);
-        cg1 = 0.5 * (ce * gxn + SD(D_CE, p + W) * gxs);
-      }
-      const float gi2 = 0.5f * (gy * bye + SF(F_GY, p + 1) * byw);
-      const double cg2 = 0.5 * (cn * gye + SD(D_CN, p + 1) * gyw);
-      const float pg1 = (float)((double)gi1 + cg1 + ghx) * seau * sche;
-      const float pg2 = (float)((double)gi2 + cg2 + ghy) * seau * sche;
-      float p1 = seau * (dvu + ut - pg1 + 0.5f * cor * v0);
-      float p2 = seau * (dvv + vt - pg2 - 0.5f * cor * u0);
-      const float w1 = p1 * bt + u0, w2 = p2 * bt + v0;
-      float u1 = (w1 + 0.5f * cor * bt * w2) * rden;
-      float v1 = (w2 - 0.5f * cor * bt * w1) * rden;
-      u1 = 0.5f * (u1 + u0);
-      v1 = 0.5f * (v1 + v0);
-      p1 = seau * (dvu - pg1 + ut + cor * v1);
-      p2 = seau * (dvv - pg2 + vt - cor * u1);
-      ubc = p1 * bt + u0;
-      vbc = p2 * bt + v0;
+      dvu = __fsub_rn(vsu, vs0u);
+      dvv = __fsub_rn(vsv, vs0v);
+      if (inR) SD(D_PRED, 0) = pred;
+    }
+    __syncthreads();
+    // S6: sqrt(ter(pred)), pred's gradients and means, corrector velocity
+    float ubc, vbc;
+    {
+      const double pe = SD(D_PRED, 1), pn = SD(D_PRED, W), pne = SD(D_PRED, W + 1);
+      const double w = (pred + pn + pe + pne) * 0.25;
+      float sch = sqrtf(s6sea ? (float)w : 1.f);
+      if (s2zero) sch = 0.f;
+      const float rdx2 = RDXX(2), rdy4 = RDXY(4);
+      const float gx0 = (float)(pe - pred) * rdx2 * vy[15 * H + ly], gx1 = (float)(pne - pn) * rdx2 * vy[15 * H + ly + 1];
+      const float gy0 = (float)(pn - pred) * rdy4 * ra, gy1 = (float)(pne - pe) * rdy4 * ra;
+      const double ce0 = 0.5 * (pred + pe), ce1 = 0.5 * (pn + pne), cn0 = 0.5 * (pred + pn), cn1 = 0.5 * (pe + pne);
+      float gi1 = 0.5f * __fmaf_rn(gx0, bxn, __fmul_rn(gx1, bxs)), gi2 = 0.5f * __fmaf_rn(gy0, bye, __fmul_rn(gy1, byw));
+      double cg1 = 0.5 * __fma_rn(ce0, gxn, __dmul_rn(ce1, gxs)), cg2 = 0.5 * __fma_rn(cn0, gye, __dmul_rn(cn1, gyw));
+      if (!nrow) { gi1 = gi2 = 0.f; cg1 = cg2 = 0.0; }
+      const float f1 = (float)((double)gi1 + cg1 + ghx) * seau, f2 = (float)((double)gi2 + cg2 + ghy) * seau;  // pg / sch
+      const float hc = 0.5f * cor, cb = hc * bt;
+      float p1 = seau * __fmaf_rn(hc, v0, __fmaf_rn(-f1, sch, dvu + ut));
+      float p2 = seau * __fmaf_rn(-hc, u0, __fmaf_rn(-f2, sch, dvv + vt));
+      const float w1 = __fmaf_rn(p1, bt, u0), w2 = __fmaf_rn(p2, bt, v0);
+      const float u1 = 0.5f * __fmaf_rn(__fmaf_rn(cb, w2, w1), rden, u0);
+      const float v1 = 0.5f * __fmaf_rn(__fmaf_rn(-cb, w1, w2), rden, v0);
+      p1 = seau * __fmaf_rn(cor, v1, __fmaf_rn(-f1, sch, dvu) + ut);
+      p2 = seau * __fmaf_rn(-cor, u1, __fmaf_rn(-f2, sch, dvv) + vt);
+      ubc = __fmaf_rn(p1, bt, u0);
+      vbc = __fmaf_rn(p2, bt, v0);
       if (border && nt < nstep) xch_put(out + P.n2, pack_uv(ubc, vbc), seq + nt);
-      const float ps = prh_u * sche;
-      s1 = ps * ubc;
-      x2 = ps * vbc * rh3;
-      SF(F_S1, p) = s1;
-      SF(F_X2, p) = x2;
+      const float ps = prh_u * sch;
+      s1 = __fmul_rn(ps, ubc);
+      x2 = __fmul_rn(ps * vbc, RH(3));
+      if (inR) {
+        SF(F_S1, 0) = s1;
+        SF(F_X2, 0) = x2;
+      }
     }
     __syncthreads();
     // S8: corrector ch, send, accumulate
     if (inS8) {
-      const float tEc = srow ? 0.5f * (SF(F_S1, p - W) + s1) : 0.f;
-      const float tEw = srow ? 0.5f * (SF(F_S1, p - W - 1) + SF(F_S1, p - 1)) : 0.f;
-      const float A = (tEc - tEw) * RDXX(1, lx);
-      float B = 0.f;
-      if (srow) {
-        const float tNc = 0.5f * (SF(F_X2, p - 1) + x2);
-        const float tNs = 0.5f * (SF(F_X2, p - W - 1) + SF(F_X2, p - W));
-        B = (tNc - tNs) * RDXY(1, ly);
-      }
-      const float div = (A + B) * vy[13 * H + ly];
-      const double chn = c0 - (double)(mskt1 * div * bt * rprh_t);
-      if (border && nt < nstep) xch_put(out, chn, seq + nt);
-      c0 = chn; u0 = ubc; v0 = vbc;
-      SD(D_CH, p) = c0;
-      SF(F_UB, p) = u0;
-      SF(F_VB, p) = v0;
-      if (nt <= nstep / 2) acc_m = acc_m + chn;
-      acc_m2 = acc_m2 + chn;
+      float tEc = 0.5f * (SF(F_S1, -W) + s1), tEw = 0.5f * (SF(F_S1, -W - 1) + SF(F_S1, -1));
+      const float tNc = 0.5f * (SF(F_X2, -1) + x2), tNs = 0.5f * (SF(F_X2, -W - 1) + SF(F_X2, -W));
+      if (!srow) tEc = tEw = 0.f;
+      const float A = __fmul_rn(tEc - tEw, RDXX(1));
+      float B = __fmul_rn(tNc - tNs, RDXY(1));
+      if (!srow) B = 0.f;
+      const float div = __fadd_rn(A, B) * vy[13 * H + ly];
+      c0 = c0 - (double)(mskt1 * div * bt * rprh_t);
+      if (border && nt < nstep) xch_put(out, c0, seq + nt);
+      u0 = ubc; v0 = vbc;
+      SD(D_CH, 0) = c0;
+      SF(F_UB, 0) = u0;
+      SF(F_VB, 0) = v0;
+      if (nt <= nstep / 2) acc_m = acc_m + c0;
+      acc_m2 = acc_m2 + c0;
       acc_u = acc_u + (double)ubc;
       acc_v = acc_v + (double)vbc;
     }
@@ -283,15 +262,18 @@ __global__ void __launch_bounds__(kThreads, 1)
       double v[2] = {0.0, 0.0};
       fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns);
       c0 = v[0];
-      SD(D_CH, p) = c0;
-      if (inS2) {
-        unpack_uv(v[1], u0, v0);
-        SF(F_UB, p) = u0;
-        SF(F_VB, p) = v0;
-      }
+      unpack_uv(v[1], u0, v0);
+      SD(D_CH, 0) = c0;
+      SF(F_UB, 0) = u0;
+      SF(F_VB, 0) = v0;
     }
     if (__syncthreads_or(fail)) return;
   }
+#undef SD
+#undef SF
+#undef RDXX
+#undef RDXY
+#undef RH
   if (inS8) {
     const double ub = acc_u / (nstep + 1), vb = acc_v / (nstep + 1);
     const double mch = acc_m / (nstep / 2 + 1), mch2 = acc_m2 / (nstep + 1);
@@ -320,8 +302,9 @@ const void *mixed_kernel(int TX, int TY) {
 }  // namespace
 
 size_t trop_mixed_smem_bytes(int TX, int TY) {
-  const size_t rs = (size_t)(TX + 4) * (TY + 4);
-  return D_COUNT * rs * sizeof(double) + (F_COUNT * rs + kVx * (TX + 4) + kVy * (TY + 4)) * sizeof(float);
+  const int W = TX + 4, H = TY + 4;
+  const size_t rs = (size_t)W * H, margin = 2 * (size_t)pad(W) + 32;
+  return (D_COUNT * rs + margin) * sizeof(double) + (F_COUNT * rs + margin + kVx * W + kVy * H + 1) * sizeof(float);
 }
 
 int trop_mixed_max_blocks(int TX, int TY) {
