@@ -60,41 +60,49 @@ __global__ void k_flip_t(const float *w, __nv_bfloat16 *wd, int N, int K) {
     wd[i] = __float2bfloat16(w[((long long)(8 - t) * N + n) * K + k]);
   }
 }
-// bias gradient: db[n] += sum_p g[p][n]
-__global__ void k_colsum(const __nv_bfloat16 *g, int N, long long npix, float *db) {
-  const long long gid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nthr = (long long)gridDim.x * blockDim.x;
-  const int n = (int)(gid % N);
-  float s = 0.f;
-  for (long long p = gid / N; p < npix; p += nthr / N) s += __bfloat162float(g[p * N + n]);
-  atomicAdd(db + n, s);
+// sum over the block's threads, added to *dst by one thread: an atomic per
+// warp on one FP64 address was 85 us of k_loss's 177
+__device__ void block_add(double s, double *dst) {
+  __shared__ double part[32];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x / 32] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)blockDim.x / 32; ++w) s += part[w];
+    atomicAdd(dst, s);
+  }
 }
 __global__ void k_mask_count(const float *mask, long long n, double *cnt) {
   double s = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     s += mask[i];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(cnt, s);
+  block_add(s, cnt);
 }
-// loss = sum mask (y - t)^2 / count; g = d loss / d y (BF16, 16 channels)
+// loss = sum mask (y - t)^2 / count; g = d loss / d y (BF16, 16 channels).
+// VEC: t and mask are 16-byte aligned (y and g are this library's own)
+template <bool VEC>
 __global__ void k_loss(const float *y, const float *t, const float *mask, long long npix, const double *cnt,
                        double *loss, __nv_bfloat16 *g) {
   const double c = *cnt;
   const float sc = c > 0 ? (float)(2.0 / c) : 0.f;
   double s = 0.0;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
-    #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float m = mask[p * 4 + q];
-      const float d = (y[p * 4 + q] - t[p * 4 + q]) * m;
-      s += (double)d * d;
-      g[p * 16 + q] = __float2bfloat16(sc * d);
-    }
-    #pragma unroll
-    for (int q = 4; q < 16; ++q) g[p * 16 + q] = __float2bfloat16(0.f);
+    const float4 yv = reinterpret_cast<const float4 *>(y)[p];
+    const float4 tv = VEC ? reinterpret_cast<const float4 *>(t)[p]
+                          : make_float4(t[p * 4], t[p * 4 + 1], t[p * 4 + 2], t[p * 4 + 3]);
+    const float4 mv = VEC ? reinterpret_cast<const float4 *>(mask)[p]
+                          : make_float4(mask[p * 4], mask[p * 4 + 1], mask[p * 4 + 2], mask[p * 4 + 3]);
+    const float d0 = (yv.x - tv.x) * mv.x, d1 = (yv.y - tv.y) * mv.y, d2 = (yv.z - tv.z) * mv.z, d3 = (yv.w - tv.w) * mv.w;
+    s += (double)d0 * d0;
+    s += (double)d1 * d1;
+    s += (double)d2 * d2;
+    s += (double)d3 * d3;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(sc * d0, sc * d1), hi = __floats2bfloat162_rn(sc * d2, sc * d3);
+    uint4 *o = reinterpret_cast<uint4 *>(g + p * 16);
+    o[0] = make_uint4(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi), 0u, 0u);
+    o[1] = make_uint4(0u, 0u, 0u, 0u);
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0 && c > 0) atomicAdd(loss, s / c);
+  block_add(c > 0 ? s / c : 0.0, loss);
 }
 // Adam (Kingma & Ba 2015) on the FP32 master parameters
 __global__ void k_adam(float *w, const float *g, float *m, float *v, long long n, float lr, float b1, float b2,
@@ -206,16 +214,16 @@ int backward(pcom_cnn *c, const __nv_bfloat16 *x, const float *target, const flo
   CC(cudaMemsetAsync(c->grad, 0, c->nparam * sizeof(float), c->stream));
   CC(cudaMemsetAsync(c->scal, 0, 2 * sizeof(double), c->stream));
   k_mask_count<<<592, 256, 0, c->stream>>>(mask, npix * 4, c->scal);
-  k_loss<<<592, 256, 0, c->stream>>>(c->y, target, mask, npix, c->scal, c->scal + 1, c->gout);
+  const bool vec = (((uintptr_t)target | (uintptr_t)mask) & 15u) == 0;
+  (vec ? k_loss<true> : k_loss<false>)<<<592, 256, 0, c->stream>>>(c->y, target, mask, npix, c->scal, c->scal + 1, c->gout);
   CC(cudaGetLastError());
   // layer inputs: x for layer 1, act[l] for layer l+1 (l = 1..4)
   auto layer_in = [&](int l) -> const __nv_bfloat16 * { return l == 0 ? x : c->act[l]; };
   const __nv_bfloat16 *g = c->gout;  // d loss / d (pre-activation of layer l)
   for (int l = kLayers - 1; l >= 0; --l) {
-    cudaError_t e = cnn_wgrad(kK[l], kN[l], layer_in(l), g, c->grad + c->woff[l], npix, c->H, c->W, c->periodic_x,
-                              c->err, c->stream);
+    cudaError_t e = cnn_wgrad(kK[l], kN[l], layer_in(l), g, c->grad + c->woff[l], c->grad + c->boff[l], npix, c->H, c->W,
+                              c->periodic_x, c->err, c->stream);
     if (e != cudaSuccess) return cfail(PCOM_CNN_ERR_CUDA, "wgrad layer %d: %s", l + 1, cudaGetErrorString(e));
-    k_colsum<<<592, 256, 0, c->stream>>>(g, kN[l], npix, c->grad + c->boff[l]);
     if (l == 0) break;
     // d loss / d (pre-activation of layer l-1) = conv^T(g) * (act[l] > 0)
     __nv_bfloat16 *gn = c->gbuf[l & 1];
@@ -389,8 +397,8 @@ int pcom_cnn_wgrad_layer(int32_t cin, int32_t nout, const void *in, const void *
   cudaStream_t s = (cudaStream_t)stream;
   CC(cudaMalloc(&err, sizeof(int)));
   CC(cudaMemsetAsync(err, 0, sizeof(int), s));
-  cudaError_t e = cnn_wgrad(cin, nout, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)g, dw, npix, H, W, periodic_x,
-                            err, s);
+  cudaError_t e = cnn_wgrad(cin, nout, (const __nv_bfloat16 *)in, (const __nv_bfloat16 *)g, dw, nullptr, npix, H, W,
+                            periodic_x, err, s);
   int h = 0;
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaMemcpy(&h, err, sizeof h, cudaMemcpyDeviceToHost);

@@ -30,6 +30,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include <cudaTypedefs.h>
 
@@ -850,7 +851,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_conv_rows(const __nv_bfloat
 #pragma nv_diag_default 128
 
 // ----------------------------------------------------------------------------
-// Weight gradient: dw[t][n][c] += sum_p in[src(p, t)][c] g[p][n]
+// Weight gradient of a pixel count that is not whole images: dw[t][n][c] +=
+// sum_p in[src(p, t)][c] g[p][n]
 // Tile rows r = (t - t0) * CIN + c for TPT = 128 / CIN taps starting at
 // t0 = blockIdx.y * TPT; K = pixels, 64 per stage; CTA x covers ppc pixels.
 template <int CIN, int NOUT>
@@ -955,6 +957,394 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_tc(const __nv_bfloat16 *__re
   if (warp == 0) tmem_dealloc(tmem, NCOLS);
 }
 
+// ----------------------------------------------------------------------------
+// Weight gradient of whole images: dw[t][n][c] += sum_p in[src(p, t)][c] g[p][n],
+// and the bias gradient db[n] += sum_p g[p][n].
+//
+// One pass over both activations.  The contraction runs over pixels, so both
+// operands are MN-major and a tensor-loaded row of pixels (channels
+// contiguous) is an operand as it lies in shared memory.  A CTA owns a run of
+// g rows of one tile column (128 pixels of an image row, RowRun above) and
+// streams the input rows around it: input row i meets g rows i - 1, i, i + 1
+// (row taps dy = +1, 0, -1) as one B operand of N = 3 NOUT, the three rows
+// lying in adjacent slots of the g ring (two MMAs where the ring wraps), and
+// the column taps are row blocks of A: the same pixels one pixel further on,
+// i.e. a leading byte offset of one pixel.  All 9 taps accumulate in tensor
+// memory for the whole run (64 channels: D1 = taps dx -1, 0 on 128 lanes, D2
+// tensor memory (64 channels: D1 = taps dx -1, 0 on 128 lanes, D2 = tap dx +1
+// on 64).  D2's other 64 lanes take a constant block of ones as A, so that its
+// middle column block is the bias gradient.
+//
+// Sums: tensor memory adds truncate (a chain of n adds of 16-pixel products
+// comes out n x 1.7e-8 short, measured), so after every `flush` input rows 12
+// epilogue warps add the accumulators to sums of their own (D1 in registers,
+// D2 in shared memory) and clear them, and each CTA adds its sums to dw once,
+// with FP32 atomics.  A flush takes well under a row's time; flushing to dw
+// itself took 8 us (148 CTAs' atomics on the same 147 KB) and rounded more.
+//
+// Bound: 2 MMAs of M = 128, N = 192 (96 cycles each) per 16 pixels and row
+// tap triple, 9/12 of their work useful: 71 us for a 64 -> 64 layer of 30
+// images of 360 x 160 at 1.9 GHz, beside 68 us for reading both activations
+// (442 MB) once.  Measured (with the flush rule): see the launcher.
+constexpr int kWgIn = 4, kWgG = 6;  // ring slots: input rows, g rows
+constexpr int kWgThreads = 16 * 32;  // loads, halo, MMA, (idle), 12 epilogue warps
+
+template <int C>
+__host__ __device__ constexpr int wg_in_slot() { return C == 64 ? kSlotSW : 18 * 256; }  // 136 and 144 pixels
+template <int N>
+__host__ __device__ constexpr int wg_g_slot() { return kM * N * 2; }
+template <int CIN, int NOUT>
+__host__ __device__ constexpr uint32_t wg_cols() {
+  // D1 and D2 (16 inputs: D2 is the bias gradient's NOUT columns), a power of two
+  return CIN == 16 ? 256u : (NOUT == 64 ? 512u : 128u);
+}
+template <int CIN, int NOUT>
+__host__ __device__ constexpr int wg_smem() {
+  return 1024 + kWgIn * wg_in_slot<CIN>() + kWgG * wg_g_slot<NOUT>() + 2048 +
+         (CIN == 64 ? 3 * NOUT * 64 : 0) * (int)sizeof(float);  // 64 -> 64: 215 KB
+}
+
+// MN-major operand of rows of C channels (64: 128-byte swizzle, 16: 32-byte
+// swizzle): stride byte offset = 8 rows (pixels), leading byte offset = the
+// next block of C rows of the matrix
+template <int C>
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t lbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)((8 * C * 2) >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)(C == 64 ? 2 : 6) << 61;
+  return d;
+}
+
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(
+          taddr),
+      "r"(0u)
+      : "memory");
+}
+
+template <int CIN, int NOUT>
+__global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_rows(const __nv_bfloat16 *__restrict__ in, float *dw, float *db,
+                                                              int nimg, int H, int W, int periodic_x, int flush, int *err,
+                                                              const __grid_constant__ CUtensorMap tmap_in,
+                                                              const __grid_constant__ CUtensorMap tmap_g) {
+  constexpr int ISLOT = wg_in_slot<CIN>(), GSLOT = wg_g_slot<NOUT>();
+  constexpr uint32_t NCOLS = wg_cols<CIN, NOUT>();
+  constexpr uint32_t D2 = 3 * NOUT;  // first column of D2
+  constexpr int PX = CIN * 2;        // bytes of an input pixel
+  constexpr int JA = 16 * CIN * 2 / 16, JB = 16 * NOUT * 2 / 16;  // one K step (16 pixels), 16-byte units
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t itma[kWgIn], ifull[kWgIn], iempty[kWgIn], gfull[kWgG], gempty[kWgG], dfull, dempty;
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int s_stop;
+  __shared__ float s_db[NOUT];
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t *const sbase = smem_raw + (base - smem_u32(smem_raw));
+  // (g slots first: 1024-byte aligned in both widths; then input slots, then
+  // the ones, which must lie above the input slots; then D2's sums)
+  const uint32_t Gr = base, In = base + kWgG * GSLOT, Ones = In + kWgIn * ISLOT;
+  float *const s_d2 = reinterpret_cast<float *>(sbase + (Ones - base) + 2048);  // [3 NOUT][64]
+  const int ntx = (W + kM - 1) / kM;
+  const int NR = nimg * H;
+  const long long ntiles = (long long)NR * ntx;
+  const long long chunk = (ntiles + gridDim.x - 1) / gridDim.x;
+  const long long t0 = (long long)blockIdx.x * chunk;
+  const long long t1 = t0 + chunk < ntiles ? t0 + chunk : ntiles;
+
+  if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), NCOLS);
+  if (tid == 0) {
+    for (int q = 0; q < kWgIn; ++q) {
+      mbar_init(smem_u32(&itma[q]), 1);
+      mbar_init(smem_u32(&ifull[q]), 1);
+      mbar_init(smem_u32(&iempty[q]), 1);
+    }
+    for (int q = 0; q < kWgG; ++q) {
+      mbar_init(smem_u32(&gfull[q]), 1);
+      mbar_init(smem_u32(&gempty[q]), 1);
+    }
+    mbar_init(smem_u32(&dfull), 1);
+    mbar_init(smem_u32(&dempty), 12);  // the epilogue warps
+    s_stop = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // 2048 bytes of BF16 ones (0x3F80)
+  if (tid < 128)
+    reinterpret_cast<uint4 *>(sbase + (Ones - base))[tid] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+  for (int q = tid; q < (CIN == 64 ? 3 * NOUT * 64 : 0); q += kWgThreads) s_d2[q] = 0.f;
+  for (int q = tid; q < NOUT; q += kWgThreads) s_db[q] = 0.f;
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  if (warp < 4)
+    for (uint32_t c = 0; c < NCOLS; c += 16) tmem_zero16(lane_addr + c);
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  auto stop = [&]() {
+    s_stop = 1;
+    atomicExch(err, 1);
+  };
+  RowRun run;
+
+  if (warp == 0) {
+    // ------------------------------------------------------- tensor loads
+    if (lane == 0) {
+      int ki = 0, kg = 0;
+      long long t = t0;
+      bool ok = true;
+      while (ok && !s_stop && next_run(t, t1, NR, H, run)) {
+        int y = run.rb;  // next g row to load
+        for (int i = run.ilo; ok && i <= run.ihi && !s_stop; ++i, ++ki) {
+          for (; ok && y <= run.re && y <= i + 1; ++y, ++kg) {
+            const int s = kg % kWgG, n = kg / kWgG;
+            if (n > 0 && !mbar_wait(smem_u32(&gempty[s]), (uint32_t)((n - 1) & 1))) ok = false;
+            if (!ok) break;
+            mbar_expect_tx(smem_u32(&gfull[s]), (uint32_t)GSLOT);
+            tma_load3(Gr + (uint32_t)(s * GSLOT), &tmap_g, 0, run.tx * kM, y, smem_u32(&gfull[s]));
+          }
+          const int s = ki % kWgIn, n = ki / kWgIn;
+          if (ok && n > 0 && !mbar_wait(smem_u32(&iempty[s]), (uint32_t)((n - 1) & 1))) ok = false;
+          if (!ok) break;
+          mbar_expect_tx(smem_u32(&itma[s]), (uint32_t)(kRowPix * PX));
+          tma_load3(In + (uint32_t)(s * ISLOT), &tmap_in, 0, run.tx * kM - 1, i, smem_u32(&itma[s]));
+        }
+      }
+      if (!ok) stop();
+      // no tensor load may still be writing when the CTA exits
+      for (int s = 0; s < kWgIn && s < ki; ++s) mbar_wait(smem_u32(&itma[s]), (uint32_t)(((ki - 1 - s) / kWgIn) & 1));
+      for (int s = 0; s < kWgG && s < kg; ++s) mbar_wait(smem_u32(&gfull[s]), (uint32_t)(((kg - 1 - s) / kWgG) & 1));
+    }
+  } else if (warp == 1) {
+    // --------------------------------------- periodic halo, slot release
+    int k = 0;
+    long long t = t0;
+    bool go = true;
+    while (go && !s_stop && next_run(t, t1, NR, H, run)) {
+      const int x0 = run.tx * kM;
+      const bool wl = periodic_x && run.tx == 0, wr = periodic_x && x0 + kM >= W;
+      for (int i = run.ilo; i <= run.ihi && !s_stop; ++i, ++k) {
+        const int s = k % kWgIn, n = k / kWgIn;
+        const int ok = __shfl_sync(0xffffffffu, lane == 0 ? (int)mbar_wait(smem_u32(&itma[s]), (uint32_t)(n & 1)) : 0, 0);
+        if (!ok) {
+          if (lane == 0) stop();
+          go = false;
+          break;
+        }
+        // the pixel left of x = 0 is x = W - 1; right of x = W - 1 is x = 0
+        constexpr int CH = CIN / 8;  // 16-byte chunks of a pixel
+        const int c = lane % CH;
+        const bool left = lane < CH && wl, right = lane >= CH && lane < 2 * CH && wr;
+        if (left || right) {
+          const int u = left ? 0 : W - x0 + 1, xs = left ? W - 1 : 0;
+          const int ph = CIN == 64 ? (u & 7) : ((u >> 2) & 1);  // the swizzle's row phase
+          const uint4 v = __ldg(reinterpret_cast<const uint4 *>(in + ((long long)i * W + xs) * CIN) + c);
+          *reinterpret_cast<uint4 *>(sbase + (In - base) + s * ISLOT + u * PX + ((c ^ ph) << 4)) = v;
+          fence_async_smem();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ifull[s]));
+      }
+    }
+  } else if (warp == 2) {
+    // ----------------------------------------------------------------- MMA
+    if (lane == 0) {
+      const uint64_t a1d = umma_desc_mn<CIN>(In, PX), bd = umma_desc_mn<NOUT>(Gr, GSLOT);
+      // A of D2.  64 channels: pixels two further on, then the ones: the
+      // leading byte offset shrinks as the start address grows
+      const uint64_t a2d = CIN == 64 ? umma_desc_mn<CIN>(In + 2 * PX, Ones - In - 2 * PX) : umma_desc_mn<CIN>(Ones, PX);
+      const uint32_t a1_hi = (uint32_t)(a1d >> 32), a2_hi = (uint32_t)(a2d >> 32), b_hi = (uint32_t)(bd >> 32);
+      const uint32_t a1_lo0 = (uint32_t)a1d, a2_lo0 = (uint32_t)a2d, b_lo0 = (uint32_t)bd;
+      constexpr uint32_t STEP2 = 1u - 65536u;  // start + 1, leading offset - 1 (16-byte units)
+      // K steps 0 .. KS - 1 of one run of n adjacent g rows: straight-line
+      // issue with compile-time offsets (as in k_conv_rows, branches and
+      // address arithmetic per MMA make the issuing thread the bound)
+      auto mmas = [&](auto ks_c, uint32_t d, uint32_t a1, uint32_t a2, uint32_t b, uint32_t id) {
+        constexpr int KS = decltype(ks_c)::value;
+        #pragma unroll
+        for (int j = 0; j < KS; ++j) {
+          umma_bf16_w(d, a1 + (uint32_t)(j * JA), a1_hi, b + (uint32_t)(j * JB), b_hi, id, 1u);
+          if (CIN == 64)
+            umma_bf16_w(d + D2, a2 + (uint32_t)(j * JA) * STEP2, a2_hi, b + (uint32_t)(j * JB), b_hi, id, 1u);
+        }
+      };
+      auto ones = [&](auto ks_c, uint32_t a2, uint32_t b) {  // 16 inputs: the bias gradient
+        constexpr int KS = decltype(ks_c)::value;
+        #pragma unroll
+        for (int j = 0; j < KS; ++j)
+          umma_bf16_w(tmem + D2, a2, a2_hi, b + (uint32_t)(j * JB), b_hi, umma_idesc(kM, NOUT, 1, 1), 1u);
+      };
+      int s = 0, gs0 = 0;          // slots of the input row and of the first g row it may meet (i - 1)
+      uint32_t ph = 0;             // parity of slot s's current fill
+      int ws = 0;                  // slot and parity of the next g row to wait for
+      uint32_t wp = 0;
+      uint32_t pre = 0;            // bit 0: the next input row is there, bit 1: the next g row is
+      int left = flush;            // rows until the next flush
+      uint32_t fl = 0;             // flushes so far
+      bool go = true;
+      long long t = t0;
+      while (go && !s_stop && next_run(t, t1, NR, H, run)) {
+        const int px = W - run.tx * kM;
+        // K steps that hold pixels of the image, rounded up to 1, 2, 4 or 8
+        // (the pixels past its edge are zero in g)
+        const int ks = px > 64 ? 8 : (px > 32 ? 4 : (px > 16 ? 2 : 1));
+        int yw = run.rb;  // next g row to wait for
+        int iy = run.ilo % H;
+        // slot of g row i - 1 (the first input row may be row rb - 1 or rb)
+        gs0 += run.ilo - 1 - run.rb;
+        if (gs0 < 0) gs0 += kWgG;
+        for (int i = run.ilo; i <= run.ihi; ++i) {
+          const bool vm = iy > 0 && i - 1 >= run.rb, v0 = i >= run.rb && i <= run.re, vp = iy < H - 1 && i + 1 <= run.re;
+          const int ya = vm ? 0 : (v0 ? 1 : 2), yb = vp ? 2 : (v0 ? 1 : 0);  // g rows i - 1 + (ya .. yb)
+          bool ok = true;
+          for (; ok && yw <= i - 1 + yb; ++yw, pre &= ~2u) {
+            if (!(pre & 2u)) ok = mbar_spin(smem_u32(&gfull[ws]), wp);
+            if (++ws == kWgG) { ws = 0; wp ^= 1u; }
+          }
+          if (ok && !(pre & 1u)) ok = mbar_spin(smem_u32(&ifull[s]), ph);
+          if (!ok || ((i & 7) == 0 && s_stop)) {
+            if (!ok) stop();
+            go = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sx = (uint32_t)(s * (ISLOT / 16));
+          const uint32_t a1 = a1_lo0 + sx, a2 = CIN == 64 ? a2_lo0 + sx * STEP2 : a2_lo0;
+          auto slot = [&](int y) { const int q = gs0 + y; return q >= kWgG ? q - kWgG : q; };
+          // one run of adjacent slots, or two where the ring wraps
+          int y = ya;
+          while (y <= yb) {
+            const int gs = slot(y);
+            const int n = min(yb - y + 1, kWgG - gs);
+            const uint32_t d = tmem + (uint32_t)(y * NOUT), b = b_lo0 + (uint32_t)(gs * (GSLOT / 16));
+            const uint32_t id = umma_idesc(kM, NOUT, 1, 1) + ((uint32_t)((n - 1) * (NOUT >> 3)) << 17);
+            if (ks == 8) mmas(std::integral_constant<int, 8>(), d, a1, a2, b, id);
+            else if (ks == 4) mmas(std::integral_constant<int, 4>(), d, a1, a2, b, id);
+            else if (ks == 2) mmas(std::integral_constant<int, 2>(), d, a1, a2, b, id);
+            else mmas(std::integral_constant<int, 1>(), d, a1, a2, b, id);
+            y += n;
+          }
+          if (CIN == 16 && v0) {
+            const uint32_t b = b_lo0 + (uint32_t)(slot(1) * (GSLOT / 16));
+            if (ks == 8) ones(std::integral_constant<int, 8>(), a2, b);
+            else if (ks == 4) ones(std::integral_constant<int, 4>(), a2, b);
+            else if (ks == 2) ones(std::integral_constant<int, 2>(), a2, b);
+            else ones(std::integral_constant<int, 1>(), a2, b);
+          }
+          // the next row's two barriers, tested together while this row's MMAs
+          // run (each test takes 300-500 cycles then)
+          pre = mbar_test2(smem_u32(&ifull[s + 1 == kWgIn ? 0 : s + 1]), s + 1 == kWgIn ? ph ^ 1u : ph,
+                           smem_u32(&gfull[ws]), wp);
+          umma_commit(smem_u32(&iempty[s]));
+          // g rows no later input row meets
+          if (vm) umma_commit(smem_u32(&gempty[slot(0)]));
+          if (iy == H - 1 && v0) umma_commit(smem_u32(&gempty[slot(1)]));
+          if (++iy == H) iy = 0;
+          if (++s == kWgIn) { s = 0; ph ^= 1u; }
+          if (++gs0 == kWgG) gs0 = 0;
+          if (--left == 0 && !(t >= t1 && i == run.ihi)) {
+            // the accumulators go to dw and start from zero again
+            umma_commit(smem_u32(&dfull));
+            if (!mbar_wait(smem_u32(&dempty), fl & 1u)) {
+              stop();
+              go = false;
+              break;
+            }
+            ++fl;
+            left = flush;
+            tc_fence_after();
+          }
+        }
+        // the next run's first g row follows this run's last: slot of row
+        // ihi + 1 - 1 = ihi, back to that of re + 1
+        gs0 += run.re + 1 - run.ihi;
+        if (gs0 >= kWgG) gs0 -= kWgG;
+      }
+      // the last flush (also on giving up: every MMA issued has completed
+      // before tensor memory is freed)
+      if (t0 < t1) {
+        umma_commit(smem_u32(&dfull));
+        if (!mbar_wait(smem_u32(&dfull), fl & 1u)) stop();
+      }
+    }
+  } else if (warp >= 4 && t0 < t1) {
+    // ----------------------------------------------------------- epilogue
+    long long rows = 0;
+    for (long long t = t0; next_run(t, t1, NR, H, run);) rows += run.ihi - run.ilo + 1;
+    const uint32_t nfl = (uint32_t)((rows + flush - 1) / flush);
+    const int quarter = warp & 3, sub = (warp - 4) / 4;
+    const int r = quarter * 32 + lane;
+    const int dxi = CIN == 64 ? r / 64 : r / 16, c = CIN == 64 ? r % 64 : r % 16;
+    // this warp's columns: NOUT from sub NOUT on, i.e. one row tap dy = 1 - sub
+    float acc[NOUT];
+    #pragma unroll
+    for (int q = 0; q < NOUT; ++q) acc[q] = 0.f;
+    bool ok = true;
+    for (uint32_t f = 0; f < nfl; ++f) {
+      ok = mbar_wait(smem_u32(&dfull), f & 1u);
+      if (!ok) stop();
+      ok = !__any_sync(0xffffffffu, !ok || s_stop);
+      if (!ok) break;
+      tc_fence_after();
+      #pragma unroll
+      for (int q = 0; q < NOUT; q += 16) {
+        float v[16];
+        tmem_ld16(lane_addr + sub * NOUT + q, v);
+        tmem_zero16(lane_addr + sub * NOUT + q);
+        #pragma unroll
+        for (int u = 0; u < 16; ++u) acc[q + u] += v[u];
+      }
+      if (CIN == 64 ? (quarter < 2 || (quarter == 2 && sub == 1)) : (quarter == 0 && sub == 0)) {
+        #pragma unroll 1
+        for (int q = 0; q < NOUT; q += 16) {
+          const uint32_t col = D2 + (CIN == 64 ? sub * NOUT : 0) + q;
+          float v[16];
+          tmem_ld16(lane_addr + col, v);
+          tmem_zero16(lane_addr + col);
+          if (CIN == 64 && quarter < 2) {
+            for (int u = 0; u < 16; ++u) s_d2[(sub * NOUT + q + u) * 64 + r] += v[u];
+          } else if (lane == 0) {  // a row of ones: the bias gradient
+            for (int u = 0; u < 16; ++u) s_db[q + u] += v[u];
+          }
+        }
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&dempty));
+    }
+    if (ok) {
+      // (16 channels: row blocks 3..7 are no taps)
+      const int tap0 = (2 - sub) * 3;
+      if (dxi < 3) {
+        float *const o = dw + ((long long)(tap0 + dxi) * NOUT) * CIN + c;
+        #pragma unroll
+        for (int q = 0; q < NOUT; ++q) atomicAdd(o + q * CIN, acc[q]);
+      }
+      if (CIN == 64 && quarter < 2) {
+        float *const o = dw + ((long long)(tap0 + 2) * NOUT) * CIN + c;
+        for (int q = 0; q < NOUT; ++q) {
+          const int n = (q + 7 * (int)blockIdx.x) % NOUT;
+          atomicAdd(o + n * CIN, s_d2[(sub * NOUT + n) * 64 + r]);
+        }
+      }
+      if (db && lane == 0 && (CIN == 64 ? quarter == 2 && sub == 1 : quarter == 0 && sub == 0))
+        for (int q = 0; q < NOUT; ++q) atomicAdd(db + q, s_db[q]);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, NCOLS);
+}
+
 // dynamic shared memory per CTA; with 64 accumulator columns at least 29 KB,
 // so that at most 7 CTAs share an SM's 512 tensor-memory columns
 template <int NOUT>
@@ -985,7 +1375,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // [image rows][W][C] BF16 activations as a 3-D tensor map with a box of
-// box_w pixels x C channels, 128-byte swizzle
+// box_w pixels x C channels, swizzled over a pixel's bytes (128, or 32 for 16 channels)
 bool act_tensor_map(CUtensorMap *tm, const void *p, int C, int W, int NR, int box_w) {
   auto enc = tensor_map_encoder();
   if (!enc || ((uintptr_t)p & 15u)) return false;
@@ -994,7 +1384,7 @@ bool act_tensor_map(CUtensorMap *tm, const void *p, int C, int W, int NR, int bo
   const cuuint32_t box[3] = {(cuuint32_t)C, (cuuint32_t)box_w, 1u};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(p), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, C == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1059,8 +1449,45 @@ cudaError_t conv_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const f
 }
 
 template <int CIN, int NOUT>
-cudaError_t wgrad_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *dw, long long npix, int H, int W,
-                         int periodic_x, int *err, cudaStream_t s) {
+cudaError_t wgrad_rows_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *dw, float *db, long long npix,
+                              int H, int W, int periodic_x, int *err, cudaStream_t s) {
+  constexpr int sm = wg_smem<CIN, NOUT>();
+  cudaError_t e = cudaFuncSetAttribute(k_wgrad_rows<CIN, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (e != cudaSuccess) return e;
+  const long long nimg = npix / ((long long)H * W);
+  if (nimg * H > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const int NR = (int)nimg * H;
+  CUtensorMap tin, tg;
+  if (!act_tensor_map(&tin, in, CIN, W, NR, kRowPix) || !act_tensor_map(&tg, g, NOUT, W, NR, kM)) return cudaErrorInvalidValue;
+  int dev = 0, nsm = 148, per = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_wgrad_rows<CIN, NOUT>, kWgThreads, sm);
+  const int tmem_cap = 512 / (int)wg_cols<CIN, NOUT>();
+  per = per < 1 ? 1 : (per > tmem_cap ? tmem_cap : per);
+  const long long ntiles = (long long)NR * ((W + kM - 1) / kM);
+  const long long grid = ntiles < (long long)nsm * per ? ntiles : (long long)nsm * per;
+  if (grid < 1) return cudaSuccess;
+  // a flush every 16 rows (chains of 128 adds, 2e-6 short) on long runs, every 3
+  // where a CTA has only a few.  30 images of 360 x 160: 165 us for a 64 -> 64
+  // layer (ncu) against 1,136 us of the per-tap form below (which reads both
+  // activations 5 times) and 118 us of the bias gradient's own pass; relative
+  // error against 64 bits 2e-6 (8e-6); 12 images of 131 x 67: 3.6e-7 (5.0e-7)
+  const int flush = ntiles >= 32 * grid ? 16 : 3;
+  k_wgrad_rows<CIN, NOUT><<<(unsigned)grid, kWgThreads, sm, s>>>(in, dw, db, (int)nimg, H, W, periodic_x, flush, err, tin,
+                                                                 tg);
+  return cudaGetLastError();
+}
+
+// whole images of 16-byte aligned activations (tensor loads): the row form;
+// otherwise one CTA per tap pair and pixel chunk, which gathers both
+// operands and has no bias gradient
+template <int CIN, int NOUT>
+cudaError_t wgrad_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *dw, float *db, long long npix, int H,
+                         int W, int periodic_x, int *err, cudaStream_t s) {
+  if (npix % ((long long)H * W) == 0 && (((uintptr_t)in | (uintptr_t)g) & 15u) == 0)
+    return wgrad_rows_launch<CIN, NOUT>(in, g, dw, db, npix, H, W, periodic_x, err, s);
+  if (db) return cudaErrorInvalidValue;
   const size_t sm = wgrad_smem<CIN, NOUT>();
   cudaError_t e = cudaFuncSetAttribute(k_wgrad_tc<CIN, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
@@ -1092,10 +1519,10 @@ cudaError_t cnn_conv(int cin, int nout, const __nv_bfloat16 *in, const __nv_bflo
   return cudaErrorInvalidValue;
 }
 
-cudaError_t cnn_wgrad(int cin, int nout, const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *dw, long long npix,
-                      int H, int W, int periodic_x, int *err, cudaStream_t s) {
-  if (cin == 16 && nout == 64) return wgrad_launch<16, 64>(in, g, dw, npix, H, W, periodic_x, err, s);
-  if (cin == 64 && nout == 64) return wgrad_launch<64, 64>(in, g, dw, npix, H, W, periodic_x, err, s);
-  if (cin == 64 && nout == 16) return wgrad_launch<64, 16>(in, g, dw, npix, H, W, periodic_x, err, s);
+cudaError_t cnn_wgrad(int cin, int nout, const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *dw, float *db,
+                      long long npix, int H, int W, int periodic_x, int *err, cudaStream_t s) {
+  if (cin == 16 && nout == 64) return wgrad_launch<16, 64>(in, g, dw, db, npix, H, W, periodic_x, err, s);
+  if (cin == 64 && nout == 64) return wgrad_launch<64, 64>(in, g, dw, db, npix, H, W, periodic_x, err, s);
+  if (cin == 64 && nout == 16) return wgrad_launch<64, 16>(in, g, dw, db, npix, H, W, periodic_x, err, s);
   return cudaErrorInvalidValue;
 }

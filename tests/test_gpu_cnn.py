@@ -143,6 +143,32 @@ def test_wgrad(cin, nout, px):
     assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
+# The weight gradient's row form where its bookkeeping turns: one- and
+# two-row images (a g row meets one or two input rows), widths of exactly one
+# and two tiles, one pixel over, ragged second columns of 1, 2, 4 and 8 K
+# steps, one CTA with several tile columns, and runs long enough to clear the
+# accumulators several times.  FP32 sums of up to 10^5 products of unit
+# normals: the bound of the other weight-gradient tests.
+@pytest.mark.parametrize("h,w,nimg", [(1, 130, 4), (2, 128, 3), (5, 256, 2), (7, 129, 2), (3, 150, 2), (4, 180, 1),
+                                      (3, 224, 2), (1, 3, 1), (40, 131, 12)])
+@pytest.mark.parametrize("px", [0, 1])
+@pytest.mark.parametrize("cin,nout", [(16, 64), (64, 64), (64, 16)])
+def test_wgrad_edge_shapes(cin, nout, px, h, w, nimg):
+    import torch
+
+    rng = np.random.default_rng(h * 1000 + w + 7 * cin + nout + px)
+    npix = h * w * nimg
+    xd, x = bf16(rng.standard_normal((npix, cin)))
+    gd, g = bf16(rng.standard_normal((npix, nout)))
+    dw = torch.ones(9 * nout * cin, dtype=torch.float32, device="cuda")  # the call adds to what is there
+    rc = L.load().pcom_cnn_wgrad_layer(cin, nout, xd.data_ptr(), gd.data_ptr(), dw.data_ptr(), npix, h, w, px,
+                                       C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    cnn_check(rc, "wgrad")
+    ref = pycnn.wgrad(cin, nout, x, g, h, w, px) + 1.0
+    got = dw.cpu().numpy().reshape(9, nout, cin)
+    assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
 # the 1-degree closure's images: one 160 x 360 level image per model level,
 # periodic in x (the production row walk of the persistent kernel)
 HF, WF, NF = 160, 360, 2
@@ -240,6 +266,40 @@ def test_network_gradient_matches_oracle():
     rel = np.linalg.norm(g - gref) / np.linalg.norm(gref)
     assert rel <= 2e-2, f"gradient relative error {rel:.3e}"
     lib.pcom_cnn_destroy(h)
+
+
+@pytest.mark.parametrize("h,w,nimg,off", [(7, 129, 2, 0), (1, 17, 3, 0), (9, 20, 2, 1)])
+def test_bias_gradient_and_loss(h, w, nimg, off):
+    """Each layer's bias gradient (the ones rows of the weight gradient's
+    second accumulator; an accumulator of its own for the first layer) and
+    the loss, with target and mask at 16-byte aligned and unaligned (off)
+    addresses, within the BF16 bounds of the whole-gradient test."""
+    import torch
+
+    lib = L.load()
+    par, x, t, m = _problem(h + w, nimg, h, w)
+    hn = _net(lib, nimg, h, w)
+    cnn_check(lib.pcom_cnn_set_params(hn, par.ctypes.data, par.size), "set_params")
+    xd, x16 = bf16(x)
+
+    def shifted(a):
+        d = torch.empty(a.size + off, dtype=torch.float32, device="cuda")
+        d[off:] = torch.from_numpy(a.reshape(-1)).cuda()
+        return d
+
+    td, md = shifted(t), shifted(m)
+    g = np.zeros(par.size, np.float32)
+    loss = C.c_double()
+    cnn_check(lib.pcom_cnn_gradient(hn, xd.data_ptr(), td.data_ptr() + 4 * off, md.data_ptr() + 4 * off, nimg,
+                                    g.ctypes.data, C.byref(loss)), "gradient")
+    lref, gref = pycnn.loss_grad(par, x16, t, m, h, w, 1, 1)
+    assert abs(loss.value - lref) <= 1e-3 * abs(lref)
+    o = 0
+    for k, n in ((16, 64), (64, 64), (64, 64), (64, 64), (64, 16)):
+        b = slice(o + 9 * n * k, o + 9 * n * k + n)
+        assert np.linalg.norm(g[b] - gref[b]) <= 2e-2 * np.linalg.norm(gref[b]), f"bias of the {k} -> {n} layer"
+        o += 9 * n * k + n
+    lib.pcom_cnn_destroy(hn)
 
 
 def test_training_reduces_loss():
