@@ -19,6 +19,7 @@
 #include <cuda/atomic>
 #include "pcom_dev.cuh"
 #include "pcom_kernels.h"
+#include "trop_stages.cuh"
 
 namespace {
 
@@ -693,22 +694,6 @@ int trop_res_max_blocks(int TX, int TY) {
 // region's row length and plane size are constants and every shared-memory
 // operand is a fixed offset from the thread's own point (fewer instructions
 // and registers per substep than the general form, CTX = CTY = 0).
-namespace {
-// region fields in shared memory; what a later stage needs at the thread's
-// own point only stays in registers
-enum {
-  X_CH, X_UB, X_VB,
-  X_S1, X_X2,  // supb1, supb2*rh3 (reused for the corrector's supb)
-  X_PRED,
-  X_A1U, X_A1V, X_A2U, X_A2V,
-  X_COUNT
-};
-// doubles before the first field and after the last: the stages evaluate
-// every thread's point without branches and may read (and discard) a
-// neighbour that is outside the region
-__host__ __device__ constexpr int x_pad(int W) { return W + 1; }
-}  // namespace
-
 // threads of a CTA: a fixed single-domain shape's own count, so that small
 // tiles get the registers that let a stage's chains overlap (a group packs
 // several small tiles on an SM)
@@ -721,8 +706,8 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
                 int TX, int TY, int ntx, unsigned long long seq0, const unsigned long long *gseq, int *gerr) {
   if (CTX > 0) { TX = CTX; TY = CTY; }
   extern __shared__ double sm[];
-  const TileRef T = GROUP ? tiles[blockIdx.x] : TileRef{0, 0, 0, 0, 0};
-  const Dev &P = GROUP ? Ps[T.m] : P0;
+  const TileRef tile = GROUP ? tiles[blockIdx.x] : TileRef{0, 0, 0, 0, 0};
+  const Dev &P = GROUP ? Ps[tile.m] : P0;
   const unsigned long long seq = GROUP ? *gseq : seq0;
   int *const err = GROUP ? gerr : P.err;
   const int ni = P.ni, nj = P.nj, njm = P.njm, G = P.glo_ni;
@@ -735,7 +720,7 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
   const int tid = threadIdx.x;
   int R0, J0, tw, th;
   if (GROUP) {
-    R0 = T.r0; J0 = T.j0; tw = T.tw; th = T.th;
+    R0 = tile.r0; J0 = tile.j0; tw = tile.tw; th = tile.th;
   } else {
     const int tx = blockIdx.x % ntx, ty = blockIdx.x / ntx;
     R0 = tx * TX; J0 = ty * TY + 1;
@@ -744,34 +729,10 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
   const int rr0 = R0 - 2, jj0 = J0 - 2;
   auto ring_i = [&](int r) { r %= G; if (r < 0) r += G; return r + 2; };
 
-  // 1-D metrics and the reciprocals of every divisor (dvr).  Twice dxx[1] and
-  // dxy[1] and half their reciprocals: their dividends are differences of
-  // means, and a scaling by 2 is exact, so the halves of the means, of
-  // sqrt(ter()) and of the pressure-gradient terms all move into constants.
-  for (int l = tid; l < W; l += blockDim.x) {
-    const int i = ring_i(rr0 + l);
-    for (int g = 1; g <= 4; ++g) {
-      vx[(g - 1) * W + l] = (g == 1 ? 2.0 : 1.0) * ld(P.dxx1d[g], i - 1);
-      vx[(4 + g - 1) * W + l] = (g == 1 ? 0.5 : 1.0) * ld(P.rdxx1d[g], i - 1);
-    }
-  }
-  for (int l = tid; l < H; l += blockDim.x) {
-    const int j = min(max(jj0 + l, 1), nj);
-    for (int g = 1; g <= 4; ++g) {
-      vy[(g - 1) * H + l] = (g == 1 ? 2.0 : 1.0) * ld(P.dxy1d[g], j - 1);
-      vy[(4 + g - 1) * H + l] = (g == 1 ? 0.5 : 1.0) * ld(P.rdxy1d[g], j - 1);
-      vy[(8 + g - 1) * H + l] = ld(P.rh1d[g], j - 1);
-    }
-    vy[12 * H + l] = ld(P.arh1d[1], j - 1);
-    vy[13 * H + l] = ld(P.rarh1d[1], j - 1);
-    vy[14 * H + l] = ld(P.arh1d[2], j - 1);
-    vy[15 * H + l] = ld(P.rarh1d[2], j - 1);
-    vy[16 * H + l] = ld(P.rrh1d[4], j - 1);
-    vy[17 * H + l] = ld(P.aarh3, j - 1);
-    vy[18 * H + l] = ld(P.raarh3, j - 1);
-  }
-  const double ra = P.ra;
+  for (int l = tid; l < kXVecs * W; l += blockDim.x) vx[l] = trop_xvec(P, l / W, ring_i(rr0 + l % W));
+  for (int l = tid; l < kYVecs * H; l += blockDim.x) vy[l] = trop_yvec(P, l / H, min(max(jj0 + l % H, 1), nj));
 
+  const double ra = P.ra;
   // this thread's region point
   const int p = tid;
   const int ly = min(p / W, H - 1), lx = p - ly * W < W ? p - ly * W : 0;
@@ -791,27 +752,25 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
   // region are nobody's)
   const bool ring = active && !inS8 && lx < tw + 4 && ly < th + 4;
   const int levu = active ? __ldg(P.lev_u + q) : 0, levt = active ? __ldg(P.lev_t + q) : 0;
-  const double seau = (double)(levu >= 1);
-  // dtbt on sea, 0 on land: mask * x * dtbt = x * (mask * dtbt), masks being 0 or 1
-  const double sbt = seau * bt, tbt = (double)(levt >= 1) * bt, seau4 = 0.25 * seau;
-  const double prh_uh = 0.5 * (active ? ld(P.prh_u, q) : 1.0), prh_t = active ? ld(P.prh_t, q) : 1.0;
-  const double rprh_t = active ? ld(P.rprh_t, q) : 1.0;
-  const double rden = active ? ld(P.rwt, q) : 1.0;  // 1 / (1 + (0.5 cor dtbt)^2)
-  // where sqrt(ter()) is 1 (land, and points that need none: 2 sqrt(ter())
-  // = sqrt(4)) or 0 (row nj, where ter leaves 0)
-  const bool s2sea = inS2 && levu > 0 && nrow, s2zero = levu > 0 && !nrow, s6sea = inS6 && levu > 0 && nrow;
-  // S6 coefficients (shifted where the reference's formulas shift them)
-  double sam1 = 0, bxn = 0, bxs = 0, bye = 0, byw = 0, gxn = 0, gxs = 0, gye = 0, gyw = 0;
-  double ghx = 0, ghy = 0, cor = 0, ut = 0, vt = 0;
+  TropCoef K{};
+  K.sea_u = levu >= 1;
+  K.sea_t = levt >= 1;
+  K.prh_uh = 0.5 * (active ? ld(P.prh_u, q) : 1.0);
+  K.prh_t = active ? ld(P.prh_t, q) : 1.0;
+  K.rprh_t = active ? ld(P.rprh_t, q) : 1.0;
+  K.rden = active ? ld(P.rwt, q) : 1.0;
   if (inS6) {
-    sam1 = seau * ld(P.am, q);
-    bxn = ld(P.bphi[0], q); bye = ld(P.bphi[2], q); byw = ld(P.bphi[3], q + 1);
-    gxn = 0.5 * ld(P.bgra[0], q); gye = 0.5 * ld(P.bgra[2], q); gyw = 0.5 * ld(P.bgra[3], q + 1);
-    if (nrow) { bxs = ld(P.bphi[1], q + ni); gxs = 0.5 * ld(P.bgra[1], q + ni); }
-    ghx = 2.0 * ld(P.graphihx, q); ghy = 2.0 * ld(P.graphihy, q);
-    cor = ld(P.cor, q); ut = ld(P.ut, q); vt = ld(P.vt, q);
+    K.sam1 = (double)(levu >= 1) * ld(P.am, q);
+    K.bxn = ld(P.bphi[0], q); K.bye = ld(P.bphi[2], q); K.byw = ld(P.bphi[3], q + 1);
+    K.gxn = 0.5 * ld(P.bgra[0], q); K.gye = 0.5 * ld(P.bgra[2], q); K.gyw = 0.5 * ld(P.bgra[3], q + 1);
+    if (nrow) { K.bxs = ld(P.bphi[1], q + ni); K.gxs = 0.5 * ld(P.bgra[1], q + ni); }
+    K.ghx = 2.0 * ld(P.graphihx, q); K.ghy = 2.0 * ld(P.graphihy, q);
+    K.cor = ld(P.cor, q); K.ut = ld(P.ut, q); K.vt = ld(P.vt, q);
   }
-  const double cb = 0.5 * cor * bt, den = 1 + cb * cb;
+  // (where sqrt(ter()) is not formed it is 1, 2 sqrt(ter()) = sqrt(4): land,
+  // and points that need none)
+  const TropPoint T{fs + p, vx, vy, W, H, RS, lx, ly, inR, nrow, srow, inS2 && levu > 0 && nrow, inS6 && levu > 0 && nrow,
+                    levu > 0 && !nrow};
   double vs0u = 0.0, vs0v = 0.0;
   // accumulators (mod_int.f90:176-180)
   double acc_m = 0, acc_m2 = 0, acc_u = 0, acc_v = 0;
@@ -820,129 +779,41 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
     acc_u = P.ubc[q]; acc_v = P.vbc[q];
   }
   const double land_ch0 = inS4 ? P.chc[q] : 0.0;
-  // ch, ub, vb at this thread's point, as staged for the current substep
-  double c0 = 0.0, u0 = 0.0, v0 = 0.0;
+  TropState s{};
   if (active && (inS8 || ring)) {
-    c0 = __ldcg(P.chp + q);
-    if (inS2) { u0 = __ldcg(P.ubp + q); v0 = __ldcg(P.vbp + q); }
+    s.c0 = __ldcg(P.chp + q);
+    if (inS2) { s.u0 = __ldcg(P.ubp + q); s.v0 = __ldcg(P.vbp + q); }
   }
-  // this thread's point in each field, and its row's and column's metrics
-  double *const f = fs + p;
-#define S(F, o) f[(F) * RS + (o)]
-#define MVX(n) vx[(n) * W + lx]
-#define MVY(n) vy[(n) * H + ly]
-  if (inR) { S(X_CH, 0) = c0; S(X_UB, 0) = u0; S(X_VB, 0) = v0; }
+  if (inR) { T.S(X_CH, 0) = s.c0; T.S(X_UB, 0) = s.u0; T.S(X_VB, 0) = s.v0; }
   __syncthreads();
 
-  // The stages run straight through for every thread, whatever its point
-  // belongs to: values at points a stage does not cover are formed from
-  // whatever is there and are never read by a point it does cover.  With a
-  // branch per part the parts' latencies added up (a substep of 4 to 20 warps
-  // on an SM is bound by its dependency chains, not by issue).
   for (int nt = 1; nt <= nstep; ++nt) {
     ulonglong2 *const out = P.xch + (long long)(nt & 1) * 3 * P.n2 + q;  // this substep's words of this point
-    // S2: sch = sqrt(ter(ch)) on U and the fluxes supb; the viscosity's
-    // differences p1(ub)/rh4 on N and p2(ub) rh2 on E
-    double s1, x2, a1u, a1v, a2u, a2v;
-    {
-      const double w = c0 + S(X_CH, W) + S(X_CH, 1) + S(X_CH, W + 1);
-      double sch = sqrt(s2sea ? w : 4.0);
-      if (s2zero) sch = 0.0;
-      const double ps = prh_uh * sch;
-      s1 = ps * u0;
-      x2 = ps * v0 * MVY(10);
-      const double dx4 = MVX(3), rdx4 = MVX(7), rh4 = MVY(11), rrh4 = MVY(16);
-      a1u = dvr(dvr(u0 - S(X_UB, -1), dx4, rdx4), rh4, rrh4);
-      a1v = dvr(dvr(v0 - S(X_VB, -1), dx4, rdx4), rh4, rrh4);
-      const double dy2 = MVY(1), rdy2 = MVY(5), rh2 = MVY(9);
-      a2u = dvr(u0 - S(X_UB, -W), dy2, rdy2) * rh2;
-      a2v = dvr(v0 - S(X_VB, -W), dy2, rdy2) * rh2;
-      if (!srow) a2u = a2v = 0.0;
-      if (inR) {
-        S(X_S1, 0) = s1;
-        S(X_X2, 0) = x2;
-        S(X_A1U, 0) = a1u;
-        S(X_A1V, 0) = a1v;
-        S(X_A2U, 0) = a2u;
-        S(X_A2V, 0) = a2v;
-      }
+    trop_s2(T, K, s);
+    __syncthreads();
+    trop_s4(T, K, s, bt, gamma_b, nt == 1 ? land_ch0 : s.c0, nt == 1, vs0u, vs0v);
+    __syncthreads();
+    trop_s6(T, K, s, bt, a, ra);
+    if (border && nt < nstep) {
+      xch_put(out + P.n2, s.ubc, seq + nt);
+      xch_put(out + 2 * P.n2, s.vbc, seq + nt);
     }
     __syncthreads();
-    // S4: predictor ch (the ter U->E and U->N means of supb formed from the
-    // staged supb; rows >= 2); the viscosity
-    double pred, dvu, dvv;
-    {
-      double A = dvr((S(X_S1, -W) + s1) - (S(X_S1, -W - 1) + S(X_S1, -1)), MVX(0), MVX(4));
-      double B = dvr((S(X_X2, -1) + x2) - (S(X_X2, -W - 1) + S(X_X2, -W)), MVY(0), MVY(4));
-      if (!srow) A = B = 0.0;
-      const double div = dvr(A + B, MVY(12), MVY(13));
-      pred = c0 - dvr(div * bt * gamma_b, prh_t, rprh_t);
-      if (levt <= 0) pred = nt == 1 ? land_ch0 : c0;
-      const double dx3 = MVX(2), rdx3 = MVX(6), dy3 = MVY(2), rdy3 = MVY(6), aarh = MVY(17), raarh = MVY(18);
-      const double L1u = dvr(S(X_A1U, 1) - a1u, dx3, rdx3), L1v = dvr(S(X_A1V, 1) - a1v, dx3, rdx3);
-      double L2u = dvr(S(X_A2U, W) - a2u, dy3, rdy3), L2v = dvr(S(X_A2V, W) - a2v, dy3, rdy3);
-      if (!nrow) L2u = L2v = 0.0;
-      const double vsu = sam1 * dvr(L1u + L2u, aarh, raarh), vsv = sam1 * dvr(L1v + L2v, aarh, raarh);
-      if (nt == 1) { vs0u = vsu; vs0v = vsv; }
-      dvu = vsu - vs0u;
-      dvv = vsv - vs0v;
-      if (inR) S(X_PRED, 0) = pred;
-    }
-    __syncthreads();
-    // S6: sqrt(ter(pred)), the gradients and means of pred on E (rows j and
-    // j + 1) and N (columns i and i + 1), all from the same four values, and
-    // the corrector velocity (pressure gradient, Coriolis adjustment)
-    double ubc, vbc;
-    {
-      const double pe = S(X_PRED, 1), pn = S(X_PRED, W), pne = S(X_PRED, W + 1);
-      const double w = pred + pn + pe + pne;
-      double sch = sqrt(s6sea ? w : 4.0);
-      if (s2zero) sch = 0.0;
-      const double dx2 = MVX(1), rdx2 = MVX(5), dy4 = MVY(3), rdy4 = MVY(7);
-      const double gx0 = dvr(dvr(pe - pred, dx2, rdx2), MVY(14), MVY(15));
-      const double gx1 = dvr(dvr(pne - pn, dx2, rdx2), vy[14 * H + ly + 1], vy[15 * H + ly + 1]);
-      const double gy0 = dvr(dvr(pn - pred, dy4, rdy4), a, ra), gy1 = dvr(dvr(pne - pe, dy4, rdy4), a, ra);
-      double t1 = (gx0 * bxn + gx1 * bxs) + ((pred + pe) * gxn + (pn + pne) * gxs);
-      double t2 = (gy0 * bye + gy1 * byw) + ((pred + pn) * gye + (pe + pne) * gyw);
-      if (!nrow) t1 = t2 = 0.0;
-      const double pg1 = (t1 + ghx) * seau4 * sch, pg2 = (t2 + ghy) * seau4 * sch;
-      const double w1 = (dvu + ut - pg1 + 0.5 * cor * v0) * sbt + u0;
-      const double w2 = (dvv + vt - pg2 - 0.5 * cor * u0) * sbt + v0;
-      const double u1 = 0.5 * (dvr(w1 + cb * w2, den, rden) + u0);
-      const double v1 = 0.5 * (dvr(w2 - cb * w1, den, rden) + v0);
-      ubc = (dvu - pg1 + ut + cor * v1) * sbt + u0;
-      vbc = (dvv - pg2 + vt - cor * u1) * sbt + v0;
-      if (border && nt < nstep) {
-        xch_put(out + P.n2, ubc, seq + nt);
-        xch_put(out + 2 * P.n2, vbc, seq + nt);
-      }
-      const double ps = prh_uh * sch;
-      s1 = ps * ubc;
-      x2 = ps * vbc * MVY(10);
-      if (inR) {
-        S(X_S1, 0) = s1;
-        S(X_X2, 0) = x2;
-      }
-    }
-    __syncthreads();
-    // S8: corrector ch (with the ter means of the corrector's supb), send, accumulate
+    // S8: corrector ch, send, accumulate
     if (inS8) {
-      double A = dvr((S(X_S1, -W) + s1) - (S(X_S1, -W - 1) + S(X_S1, -1)), MVX(0), MVX(4));
-      double B = dvr((S(X_X2, -1) + x2) - (S(X_X2, -W - 1) + S(X_X2, -W)), MVY(0), MVY(4));
-      if (!srow) A = B = 0.0;
-      const double div = dvr(A + B, MVY(12), MVY(13));
-      c0 = c0 - dvr(div * tbt, prh_t, rprh_t);
-      if (border && nt < nstep) xch_put(out, c0, seq + nt);
+      s.c0 = trop_s8(T, K, s, bt);
+      if (border && nt < nstep) xch_put(out, s.c0, seq + nt);
       // the next substep's state at this point (nobody reads these three
       // entries in S8)
-      u0 = ubc; v0 = vbc;
-      S(X_CH, 0) = c0;
-      S(X_UB, 0) = u0;
-      S(X_VB, 0) = v0;
-      if (nt <= nstep / 2) acc_m = acc_m + c0;
-      acc_m2 = acc_m2 + c0;
-      acc_u = acc_u + ubc;
-      acc_v = acc_v + vbc;
+      s.u0 = s.ubc; s.v0 = s.vbc;
+      T.S(X_CH, 0) = s.c0;
+      T.S(X_UB, 0) = s.u0;
+      T.S(X_VB, 0) = s.v0;
+      // (mch and mch2 have the same terms up to half the substeps)
+      acc_m2 = acc_m2 + s.c0;
+      if (nt == nstep / 2) acc_m = acc_m2;
+      acc_u = acc_u + s.u0;
+      acc_v = acc_v + s.v0;
     }
     if (nt == nstep) break;
     // the ring's state of this substep from the tiles around (after this
@@ -953,18 +824,15 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
       const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : out, inS2 ? out + 2 * P.n2 : out};
       double v[3] = {0.0, 0.0, 0.0};
       fail = !xch_wait(in, seq + nt, v, err, P.wait_ns);
-      c0 = v[0];
-      u0 = v[1];
-      v0 = v[2];
-      S(X_CH, 0) = c0;
-      S(X_UB, 0) = u0;
-      S(X_VB, 0) = v0;
+      s.c0 = v[0];
+      s.u0 = v[1];
+      s.v0 = v[2];
+      T.S(X_CH, 0) = s.c0;
+      T.S(X_UB, 0) = s.u0;
+      T.S(X_VB, 0) = s.v0;
     }
     if (__syncthreads_or(fail)) return;
   }
-#undef S
-#undef MVX
-#undef MVY
   if (inS8) {
     const double ub = acc_u / (nstep + 1), vb = acc_v / (nstep + 1);
     const double mch = acc_m / (nstep / 2 + 1), mch2 = acc_m2 / (nstep + 1);

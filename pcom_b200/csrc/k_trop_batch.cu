@@ -43,33 +43,23 @@ __device__ bool batch_barrier(unsigned long long *cnt, unsigned long long want, 
 
 }  // namespace
 
-// SINGLE: every tile belongs to one domain, passed by value (P0, read through
-// the constant cache); otherwise each tile's domain is Ps[tile.m].
-// CTX, CTY > 0: compiled for one tile shape, so the region strides and the
-// stage loops' point -> (lx, ly) divisions are constants; each stage walks
-// the rectangle a full tile would cover and skips points outside its part
-// of a partial tile.
-// Threads per CTA: 512 for one domain (about 40 registers: a region point
-// per thread for 32 x 10 tiles), 256 for a batch (more registers per thread).
-template <bool SINGLE>
-constexpr int batch_threads() { return SINGLE ? 512 : 256; }
+// Threads per CTA
+constexpr int kBatchThreads = 256;
 
-template <bool SINGLE, int CTX = 0, int CTY = 0>
-__global__ void __launch_bounds__(batch_threads<SINGLE>()) k_trop_batch(const __grid_constant__ Dev P0, const Dev *__restrict__ Ps,
-                                                    const TileRef *__restrict__ tiles, int ntiles, int TX, int TY,
-                                                    unsigned long long *cnt, int *err) {
-  if (CTX > 0) { TX = CTX; TY = CTY; }
+__global__ void __launch_bounds__(kBatchThreads) k_trop_batch(const Dev *__restrict__ Ps, const TileRef *__restrict__ tiles,
+                                                              int ntiles, int TX, int TY, unsigned long long *cnt,
+                                                              int *err) {
   extern __shared__ double sm[];
   const int W = TX + 4, RS = W * (TY + 4);
   const int tid = threadIdx.x, nth = blockDim.x;
-  const int nstep = SINGLE ? P0.nstep : Ps[0].nstep;
-  const unsigned long long wait_ns = SINGLE ? P0.wait_ns : Ps[0].wait_ns;
+  const int nstep = Ps[0].nstep;
+  const unsigned long long wait_ns = Ps[0].wait_ns;
   auto S = [&](int f, int p) -> double & { return sm[f * RS + p]; };
 
   // accumulators of owned points (mod_int.f90:176-180)
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const TileRef T = tiles[t];
-    const Dev &P = SINGLE ? P0 : Ps[T.m];
+    const Dev &P = Ps[T.m];
     for (int p = tid; p < T.tw * T.th; p += nth) {
       const int i = T.r0 + p % T.tw + 2, j = T.j0 + p / T.tw;
       const long long q = I2(P, i, j);
@@ -84,7 +74,7 @@ __global__ void __launch_bounds__(batch_threads<SINGLE>()) k_trop_batch(const __
     const int d = (nt - 1) & 1;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       const TileRef T = tiles[t];
-      const Dev &P = SINGLE ? P0 : Ps[T.m];
+      const Dev &P = Ps[T.m];
       const int G = P.glo_ni, nj = P.nj, njm = P.njm, ni = P.ni;
       const int tw = T.tw, th = T.th, rr0 = T.r0 - 2, jj0 = T.j0 - 2;
       const double a = P.c.a, ra = P.ra, bt = (double)P.bt, gamma_b = P.c.gamma_b;
@@ -288,7 +278,7 @@ __global__ void __launch_bounds__(batch_threads<SINGLE>()) k_trop_batch(const __
   // averages (mod_int.f90:276-288)
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const TileRef T = tiles[t];
-    const Dev &P = SINGLE ? P0 : Ps[T.m];
+    const Dev &P = Ps[T.m];
     for (int p = tid; p < T.tw * T.th; p += nth) {
       const int i = T.r0 + p % T.tw + 2, j = T.j0 + p / T.tw;
       const long long q = I2(P, i, j);
@@ -307,62 +297,27 @@ __global__ void __launch_bounds__(batch_threads<SINGLE>()) k_trop_batch(const __
   }
 }
 
-namespace {
-// the form for a tile shape: the fixed-shape one for the 32 x 10 tiles the
-// single-domain selector uses (a 36 x 14 region: 504 of the 512 threads), the
-// general one otherwise
-template <bool SINGLE>
-const void *batch_kernel(int TX, int TY) {
-  if (SINGLE && TX == 32 && TY == 10) return (const void *)k_trop_batch<true, 32, 10>;
-  return (const void *)k_trop_batch<SINGLE>;
-}
-}  // namespace
-
 size_t trop_batch_smem(int TX, int TY) { return (size_t)B_COUNT * (TX + 4) * (TY + 4) * sizeof(double); }
 
-// co-resident CTAs of the multi-tile kernel for a tile shape (the smaller of
-// its single-domain and batched forms)
+// co-resident CTAs for a tile shape
 int trop_batch_max_blocks(int TX, int TY) {
-  int dev = 0, nsm = 0, best = 1 << 30;
+  int dev = 0, nsm = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const size_t smem = trop_batch_smem(TX, TY);
-  const void *fns[2] = {batch_kernel<true>(TX, TY), batch_kernel<false>(TX, TY)};
-  const int nth[2] = {batch_threads<true>(), batch_threads<false>()};
-  for (int f = 0; f < 2; ++f) {
-    int per = 0;
-    if (cudaFuncSetAttribute(fns[f], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fns[f], nth[f], smem) != cudaSuccess) return 0;
-    best = per < best ? per : best;
-  }
-  return best * nsm;
+  if (cudaFuncSetAttribute(k_trop_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trop_batch, kBatchThreads, smem) != cudaSuccess) return 0;
+  return per * nsm;
 }
 
-namespace {
-cudaError_t launch_batch_form(const void *fn, int nthreads, const Dev &P0, const Dev *dPs, const TileRef *dtiles,
-                              int ntiles, int TX, int TY, int nblocks, unsigned long long *cnt, int *err,
-                              cudaStream_t s) {
+cudaError_t launch_trop_batch(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nblocks,
+                              unsigned long long *cnt, int *err, cudaStream_t s) {
   const size_t smem = trop_batch_smem(TX, TY);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k_trop_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   // the barrier counter starts from zero in every launch
   e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  void *args[] = {(void *)&P0, (void *)&dPs, (void *)&dtiles, (void *)&ntiles, (void *)&TX, (void *)&TY,
-                  (void *)&cnt, (void *)&err};
-  return cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(nthreads), args, smem, s);
-}
-}  // namespace
-
-cudaError_t launch_trop_batch(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nblocks,
-                              unsigned long long *cnt, int *err, cudaStream_t s) {
-  const Dev none{};
-  return launch_batch_form(batch_kernel<false>(TX, TY), batch_threads<false>(), none, dPs, dtiles, ntiles, TX, TY,
-                           nblocks, cnt, err, s);
-}
-
-cudaError_t launch_trop_multi(const Dev &P, const TileRef *dtiles, int ntiles, int TX, int TY, int nblocks,
-                              unsigned long long *cnt, int *err, cudaStream_t s) {
-  return launch_batch_form(batch_kernel<true>(TX, TY), batch_threads<true>(), P, nullptr, dtiles, ntiles, TX, TY,
-                           nblocks, cnt, err, s);
+  void *args[] = {(void *)&dPs, (void *)&dtiles, (void *)&ntiles, (void *)&TX, (void *)&TY, (void *)&cnt, (void *)&err};
+  return cudaLaunchCooperativeKernel((const void *)k_trop_batch, dim3(nblocks), dim3(kBatchThreads), args, smem, s);
 }

@@ -359,9 +359,11 @@ struct pcom_handle {
   int n_ts = 0, n_uv = 0, n_w = 0, n_ch = 0, n_ssh = 0;
   int trop_tx = 24, trop_ty = 18, trop_blocks = 0;
   bool trop_resident = false;
-  // domains too large for the resident kernel: the multi-tile kernel over
-  // this domain's tile list (its Dev passed by value per launch)
+  // domains too large for the resident kernel: the multi-tile kernels
   bool trop_multi = false;
+  // FP64: packed coefficients and the state between substeps
+  unsigned char *ms_scratch = nullptr;
+  MultiTrop ms{};
   // mixed handles on the multi-tile path: FP32 coefficients and velocities
   unsigned char *mm_scratch = nullptr;
   MultiMixed mm{};
@@ -535,39 +537,60 @@ int pick_trop_config(pcom_handle *h) {
       }
     if (bx > 0 && trop_fast_max_blocks(bx, by) >= best_n) return take(bx, by, best_n);
   }
-  // too large to be resident: the multi-tile kernel (several tiles per CTA,
-  // coefficients from L2) over this domain's tiles
+  // too large to be resident: the multi-tile kernels
   if (h->trop_force == 1) return fail(PCOM_ERR_ARG, "the domain does not fit the resident barotropic kernel");
   if (h->D.separable && (h->trop_force == 0 || h->trop_force == 2)) {
-    const int tx = 32, ty = 10;
-    const int mb = trop_batch_max_blocks(tx, ty);
-    if (mb > 0) {
+    const int G = h->dims.glo_ni, nj = h->nj;
+    if (!h->d_cnt1) {
+      int rc = h->alloc(&h->d_cnt1, 1);
+      if (rc) return rc;
+    }
+    if (!h->mixed) {
+      // the compiled shape whose CTAs issue the fewest warps per substep
+      // (tiles per CTA x warps per tile)
+      long long best = 1LL << 60;
+      int bx = 0, by = 0, bb = 0;
+#define PCOM_TRY_SHAPE(x, y)                                                                        \
+  {                                                                                                 \
+    const int n_ = ((G + (x) - 1) / (x)) * ((nj + (y) - 1) / (y));                                  \
+    const int mb_ = std::min(n_, trop_multi_max_blocks((x), (y)));                                  \
+    const long long c_ = mb_ > 0 ? (long long)((n_ + mb_ - 1) / mb_) * ((((x) + 4) * ((y) + 4) + 31) / 32) : best; \
+    if (c_ < best) { best = c_; bx = (x); by = (y); bb = mb_; }                                     \
+  }
+      PCOM_MULTI_SHAPES(PCOM_TRY_SHAPE)
+#undef PCOM_TRY_SHAPE
+      if (bx > 0) {
+        if (!h->ms_scratch) {
+          int rc = h->alloc(&h->ms_scratch, trop_multi_scratch_bytes(G, nj, bx, by));
+          if (rc) return rc;
+          trop_multi_bind(h->ms, h->ms_scratch, G, nj, bx, by);
+        }
+        h->trop_multi = true;
+        h->trop_tx = bx;
+        h->trop_ty = by;
+        h->trop_blocks = bb;
+        return PCOM_OK;
+      }
+    } else {
+      const int tx = 32, ty = 10;
+      const int mmb = trop_multi_mixed_max_blocks(tx, ty);
+      if (mmb <= 0) return fail(PCOM_ERR_CUDA, "the mixed multi-tile barotropic kernel cannot be launched");
       std::vector<TileRef> t;
-      const int G = h->dims.glo_ni, nj = h->nj;
       for (int j0 = 1; j0 <= nj; j0 += ty)
         for (int r0 = 0; r0 < G; r0 += tx) t.push_back({0, r0, j0, std::min(tx, G - r0), std::min(ty, nj - j0 + 1)});
-      if (!h->d_cnt1) {
-        int rc = h->alloc(&h->d_cnt1, 1);
-        if (rc) return rc;
-      }
       int rc = h->alloc(&h->d_tiles1, t.size());
       if (rc) return rc;
       CK(cudaMemcpy(h->d_tiles1, t.data(), t.size() * sizeof(TileRef), cudaMemcpyHostToDevice));
       h->ntiles1 = (int)t.size();
+      if (!h->mm_scratch) {
+        rc = h->alloc(&h->mm_scratch, trop_multi_mixed_scratch_bytes(h->n2));
+        if (rc) return rc;
+        trop_multi_mixed_bind(h->mm, h->mm_scratch, h->n2);
+      }
       h->trop_multi = true;
       h->trop_tx = tx;
       h->trop_ty = ty;
-      h->trop_blocks = std::min(h->ntiles1, mb);
-      if (h->mixed) {
-        const int mmb = trop_multi_mixed_max_blocks(tx, ty);
-        if (mmb <= 0) return fail(PCOM_ERR_CUDA, "the mixed multi-tile barotropic kernel cannot be launched");
-        if (!h->mm_scratch) {
-          rc = h->alloc(&h->mm_scratch, trop_multi_mixed_scratch_bytes(h->n2));
-          if (rc) return rc;
-          trop_multi_mixed_bind(h->mm, h->mm_scratch, h->n2);
-        }
-        h->trop_blocks = std::min(h->ntiles1, mmb);
-      }
+      h->trop_blocks = std::min(h->ntiles1, mmb);
       return PCOM_OK;
     }
   }
@@ -665,8 +688,8 @@ int do_trop(pcom_handle *h) {
     e = launch_trop_multi_mixed(h->D, h->mm, h->d_tiles1, h->ntiles1, h->trop_tx, h->trop_ty, h->trop_blocks,
                                 h->d_cnt1, h->D.err, h->stream);
   } else if (h->trop_multi) {
-    e = launch_trop_multi(h->D, h->d_tiles1, h->ntiles1, h->trop_tx, h->trop_ty, h->trop_blocks, h->d_cnt1, h->D.err,
-                          h->stream);
+    h->launches++;  // its coefficient packing
+    e = launch_trop_multi(h->D, h->ms, h->trop_tx, h->trop_ty, h->trop_blocks, h->d_cnt1, h->stream);
   } else {
     e = launch_trop(h->D, h->trop_tx, h->trop_ty, h->trop_blocks, h->stream);
   }

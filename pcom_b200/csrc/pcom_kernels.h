@@ -81,13 +81,25 @@ int trop_multi_mixed_max_blocks(int TX, int TY);
 cudaError_t launch_trop_multi_mixed(const Dev &P, const MultiMixed &M, const TileRef *dtiles, int ntiles, int TX,
                                     int TY, int nblocks, unsigned long long *cnt, int *err, cudaStream_t s);
 
+// a batch's members too large for the resident form: several tiles per CTA
 size_t trop_batch_smem(int TX, int TY);
 int trop_batch_max_blocks(int TX, int TY);
 cudaError_t launch_trop_batch(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nblocks,
                               unsigned long long *cnt, int *err, cudaStream_t s);
-// the same kernel over the tiles of one domain P (passed by value)
-cudaError_t launch_trop_multi(const Dev &P, const TileRef *dtiles, int ntiles, int TX, int TY, int nblocks,
-                              unsigned long long *cnt, int *err, cudaStream_t s);
+// one FP64 domain with more tiles than SMs (k_trop_multi.cu): tile shapes it
+// is compiled for, and its scratch, which the handle allocates
+#define PCOM_MULTI_SHAPES(S) S(24, 14) S(20, 16) S(28, 12)
+struct MultiTrop {
+  int pitch;                       // columns of the packed grid: glo_ni and two wrapped ones at each end
+  double2 *cf;                     // coefficient pairs, planes of [nj][pitch]
+  double2 *st[2], *acc;            // state between substeps ([nj][pitch]), sums of ub, vb ([nj][ni])
+  double *xm, *ym;                 // metric vectors of every tile column and row
+};
+size_t trop_multi_scratch_bytes(int glo_ni, int nj, int TX, int TY);
+void trop_multi_bind(MultiTrop &M, void *scratch, int glo_ni, int nj, int TX, int TY);
+int trop_multi_max_blocks(int TX, int TY);
+cudaError_t launch_trop_multi(const Dev &P, const MultiTrop &M, int TX, int TY, int nblocks, unsigned long long *cnt,
+                              cudaStream_t s);
 // resident form: one tile per CTA, coefficients in registers (the fast
 // kernel over a tile list); all tiles of the group must be co-resident.  *cnt
 // is the sequence base, advanced by nstep before the launch
