@@ -13,7 +13,10 @@
 // the exceptions: one thread per column marches down the levels (k_ts_col,
 // k_readyc_col), and a point-parallel kernel forms int_ts's accumulations
 // (k_ts_acc).  Horizontal operators are evaluated point-wise from their
-// definitions in mod_op.f90 (halo conventions in pcom_dev.cuh).  Every
+// definitions in mod_op.f90 (halo conventions in pcom_dev.cuh).  Points below
+// a column's bottom (two thirds of a global grid's points, land included)
+// take an operator's masked result -- zero, or the value unchanged -- without
+// the operator.  Every
 // division by a static metric, a bottom pressure or a per-step 2-D field uses
 // its precomputed correctly rounded reciprocal with dvr (bitwise equal to the
 // IEEE quotient); the equation of state keeps its IEEE divisions.
@@ -89,25 +92,19 @@ __global__ void __launch_bounds__(512) k_alpha_tobot(const __grid_constant__ Dev
   for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
     if (!ok) continue;
     const long long q = q2 + P.n2 * (k - 1);
-    double al;
-    if (k <= lev) {
-      al = 1.0 / den_rho(P.c, P.tc[q], P.sc[q], ch * P.pr2[k]);
-      P.alpha[q] = alpha_store(P, al, k);
-    } else {
-      al = alpha_full(P, P.alpha[q], k);
-    }
-    tmp[(k - 1) * TB_X + tx] = al * P.dpr2[k] * (double)(k <= lev);
+    if (k > lev) break;  // below the bottom: alpha stays, nothing to integrate
+    const double al = 1.0 / den_rho(P.c, P.tc[q], P.sc[q], ch * P.pr2[k]);
+    P.alpha[q] = alpha_store(P, al, k);
+    tmp[(k - 1) * TB_X + tx] = al * P.dpr2[k];
   }
   __syncthreads();
   for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
     if (!ok) continue;
-    double v;
-    if (k < nk) {
+    double v = 0.0;
+    if (k <= lev) {
       double s = 0.0;
-      for (int kk = k + 1; kk <= nk; ++kk) s = s + tmp[(kk - 1) * TB_X + tx];
+      for (int kk = k + 1; kk <= lev; ++kk) s = s + tmp[(kk - 1) * TB_X + tx];
       v = tmp[(k - 1) * TB_X + tx] * 0.5 + s;
-    } else {
-      v = tmp[(nk - 1) * TB_X + tx] * 0.5;
     }
     P.adp[q2 + P.n2 * (k - 1)] = adp_store(P, v, k, q2);
   }
@@ -130,8 +127,12 @@ __global__ void __launch_bounds__(512) k_pgra2d(const __grid_constant__ DevT<R> 
   const int tx = threadIdx.x;
   const long long q2 = ok ? I2(P, i, j) : 0;
   const bool nrow = j <= P.njm;
-  for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
-    if (!ok) continue;
+  // the integrals run to the bottom of the U columns here and at cshift(-1)
+  // in j and in i
+  const int js = (j == 1) ? P.nj : j - 1;
+  const long long qs = ok ? I2(P, i, js) : 0, qw = q2 - 1;
+  const int kb = ok ? max(P.lev_u[q2], max(P.lev_u[qs], P.lev_u[qw])) : 0;
+  for (int k = threadIdx.y + 1; k <= kb; k += TB_K) {
     const long long q = q2 + P.n2 * (k - 1);
     const double dp = P.dpr2[k], pr = P.pr2[k];
     const double adc = adp_full(P, ld(P.adp, q), k, q2), ade = adp_full(P, ld(P.adp, q + 1), k, q2 + 1);
@@ -153,14 +154,12 @@ __global__ void __launch_bounds__(512) k_pgra2d(const __grid_constant__ DevT<R> 
   __syncthreads();
   const int which = threadIdx.y;  // 8 column sums, one per thread row
   if (!ok || which >= 8) return;
-  const int js = (j == 1) ? P.nj : j - 1;
-  const long long qs = I2(P, i, js), qw = q2 - 1;  // cshift(-1) in j and in i
   const double *base = (which < 2) ? bE : (which < 4) ? bN : (which < 6) ? bX : bY;
   // masks: own point, the point cshift(-1) in j (xs) or in i (yw)
   const long long qm = (which & 1) ? ((which == 1 || which == 5) ? qs : qw) : q2;
   const int lm = P.lev_u[qm];
   double s = 0.0;
-  for (int k = 1; k <= nk; ++k) s = s + base[(k - 1) * TB_X + tx] * (double)(lm >= k);
+  for (int k = 1; k <= lm; ++k) s = s + base[(k - 1) * TB_X + tx];
   const double v = dvr(s, ld(P.prh_u, qm), ld(P.rprh_u, qm));
   double *dst = (which < 4) ? P.bphi[which] : P.bgra[which - 4];
   st2(dst, P, i, q2, v);
@@ -250,8 +249,7 @@ __global__ void __launch_bounds__(512) k_upwelling(const __grid_constant__ DevT<
   const int lev = ok ? P.lev_t[q2] : 0;
   const bool srow = j >= 2;
   const long long qw = q2 - 1, qs = q2 - P.ni, qsw = qs - 1;
-  for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
-    if (!ok) continue;
+  for (int k = threadIdx.y + 1; k <= lev; k += TB_K) {
     const long long o = P.n2 * (k - 1);
     const R s_c = ld(P.sch_w, q2), s_w = ld(P.sch_w, qw);
     const R r_c = RH(3, j);
@@ -269,18 +267,17 @@ __global__ void __launch_bounds__(512) k_upwelling(const __grid_constant__ DevT<
     const R A = DIVX(tEc - tEw, 1, i);
     const R w = DIVARH(A + B, 1, j);
     wk[(k - 1) * UX + tx] = w;
-    tm[(k - 1) * UX + tx] = w * P.dpr2[k] * (R)(k <= lev);
+    tm[(k - 1) * UX + tx] = w * P.dpr2[k];
   }
   __syncthreads();
   if (ok && threadIdx.y == 0) {
     double s = 0.0;
-    for (int k = 1; k <= nk; ++k) s = s + tm[(k - 1) * UX + tx];
+    for (int k = 1; k <= lev; ++k) s = s + tm[(k - 1) * UX + tx];
     const double wk2d = -dvr(s, ld(P.prh_t, q2), ld(P.rprh_t, q2));
     double wprev = P.wm[q2];
     wmv[tx] = wprev;
-    for (int k = 2; k <= nk; ++k) {
-      double w = wprev + P.dpr2[k - 1] * (wk2d + wk[(k - 2) * UX + tx]);
-      w = w * (double)(k <= lev);
+    for (int k = 2; k <= lev; ++k) {
+      const double w = wprev + P.dpr2[k - 1] * (wk2d + wk[(k - 2) * UX + tx]);
       wmv[(k - 1) * UX + tx] = w;
       wprev = w;
     }
@@ -289,13 +286,28 @@ __global__ void __launch_bounds__(512) k_upwelling(const __grid_constant__ DevT<
   if (!ok) return;
   for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
     const long long q = q2 + P.n2 * (k - 1);
-    const double w = wmv[(k - 1) * UX + tx];
+    const double w = k <= max(lev, 1) ? wmv[(k - 1) * UX + tx] : 0.0;
     if (k >= 2) st2(P.wm, P, i, q, w);
-    if (with_acw) {
+    if (with_acw && k <= max(lev, 1)) {
       const double gm = P.c.g * ld(P.mch2, q2);
       st2(P.acw, P, i, q, P.acw[q] + dvr(w * alpha_full(P, ld(P.alpha, q), k), gm, ld(P.rgm2, q2)));
     }
   }
+}
+
+// int_readyc's 3-D results two or more levels below a U column's bottom: the
+// tendencies are masked and there is no stress (the level below the bottom
+// still takes the drag)
+template <typename R>
+__device__ __forceinline__ void readyc_dry(const DevT<R> &P, int i, long long q) {
+  st2(P.auc, P, i, q, (R)0);
+  st2(P.avc, P, i, q, (R)0);
+  if (P.ab3_mode == 1) {
+    st2(P.aup, P, i, q, (R)0); st2(P.aupp, P, i, q, (R)0);
+    st2(P.avp, P, i, q, (R)0); st2(P.avpp, P, i, q, (R)0);
+  }
+  st2(P.fx, P, i, q, (R)0);
+  st2(P.fy, P, i, q, (R)0);
 }
 
 // ----------------------------------------------------------------------------
@@ -322,6 +334,10 @@ __global__ void __launch_bounds__(512) k_readyc3d(const __grid_constant__ DevT<R
   const int lu = ok ? P.lev_u[q2] : 0;
   for (int k = threadIdx.y + 1; k <= nk && ok; k += TB_K) {
     const long long o = P.n2 * (k - 1);
+    if (k > lu + 1) {  // below the level that takes the bottom drag
+      readyc_dry(P, i, q2 + o);
+      continue;
+    }
     // per-column coefficients
     const R sch = ld(P.sch_r, q2), rsch = ld(P.rsch, q2);
     const R rsc_e = ld(P.rsch, qe), rsc_w = ld(P.rsch, qw);
@@ -459,185 +475,233 @@ __global__ void __launch_bounds__(512) k_readyc3d(const __grid_constant__ DevT<R
   if (!ok || threadIdx.y >= 2) return;
   const double *t = threadIdx.y == 0 ? tu : tv;
   double s = 0.0;
-  for (int k = 1; k <= nk; ++k) s = s + t[(k - 1) * TB_X + tx];
+  for (int k = 1; k <= lu; ++k) s = s + t[(k - 1) * TB_X + tx];
   st2(threadIdx.y == 0 ? P.ut : P.vt, P, i, q2, dvr(s, ld(P.prh_u, q2), ld(P.rprh_u, q2)));
 }
 
 // ----------------------------------------------------------------------------
-// int_readyc's 3-D part on the FP64 path, one thread per column marching
-// down the levels (the per-point arithmetic of k_readyc3d above, in the same
-// order).  The column's 2-D fields and metric factors are read once; u, v
-// at k-1 and k+1, w on U at k+1 (the next level's w at k) and km roll
-// through registers, so a level reads only the horizontal neighbours of u
-// and v, the four wm of the next level, am and km.  The depth integral of
-// the baroclinic tendency accumulates in registers in level order.
-constexpr int kRcX = 32, kRcY = 2;
-
-template <bool BATCH>
-__global__ void __launch_bounds__(kRcX * kRcY, 7) k_readyc_col(const __grid_constant__ DevT<double> P0,
-                                                              const DevT<double> *__restrict__ Ps) {
+// int_readyc's 3-D part on the FP64 path: threads march down the levels of a
+// column (the per-point arithmetic of k_readyc3d above, in the same order).
+// The column's 2-D fields and metric factors are read once; u, v, w on U and
+// the vertical fluxes between two levels (advection, and stress or drag: a
+// level's lower one is the next level's upper one) roll through registers, so
+// a level reads only the horizontal neighbours of u and v, the four wm of the
+// next level, am and km.
+//
+// What bounds it is the time of a level in a thread (~1,000 instructions, a
+// third of them FP64, and its loads' latency) times the levels in a row, so a
+// warp stops at its deepest bottom, fields are read at 32-bit offsets from a
+// level's uniform base, and with NC > 1 NC threads share a column's levels;
+// the terms of the depth integral then go to shared memory and one thread
+// adds them in level order.  The register limit is the one without spills:
+// more warps with fewer registers were slower at every size (1 degree: 116 us
+// at 128 registers, 137 at 80).
+constexpr int kColX = 32;
+template <bool BATCH, int NC>
+__global__ void __launch_bounds__(kColX * (NC == 1 ? 2 : NC), NC == 1 ? 6 : 3)
+    k_readyc_col(const __grid_constant__ DevT<double> P0, const DevT<double> *__restrict__ Ps) {
   using R = double;
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
-  const int x = blockIdx.x * kRcX + threadIdx.x;
-  const int j = blockIdx.y * kRcY + threadIdx.y + P.j_lo;
-  if (x >= P.glo_ni || j > P.j_hi) return;
+  extern __shared__ double sh[];  // NC > 1: [2][nk][kColX]
+  const int x = blockIdx.x * kColX + threadIdx.x;
+  const int j = blockIdx.y * (NC == 1 ? 2 : 1) + threadIdx.y + P.j_lo;
+  const int part = NC > 1 ? threadIdx.z : 0;
+  const bool in = x < P.glo_ni && j <= P.j_hi;
   const int i = x + 2;
-  const int nk = P.nk;
+  const int nk = P.nk, ni = P.ni;
   const long long n2 = P.n2;
-  const long long q2 = I2(P, i, j);
-  const int ni = P.ni;
-  const R g = P.c.g, a = P.c.a;
-  const R grho = g * P.c.rho0;
-  const bool nrow = j <= P.njm, srow = j >= 2;
-  const long long qe = q2 + 1, qw = q2 - 1, qn = q2 + ni, qs = q2 - ni;
-  const int lu = P.lev_u[q2];
-  // column constants (k_readyc3d: the per-point prologue)
-  const R sch = ld(P.sch_r, q2), rsch = ld(P.rsch, q2);
-  const R rsc_e = ld(P.rsch, qe), rsc_w = ld(P.rsch, qw);
-  const R sch_e = ld(P.sch_r, qe), sch_w = ld(P.sch_r, qw);
-  const R rh3 = RH(3, j), dx3 = MX(3, i), rdx3 = RMX(3, i), dy3 = MY(3, j), rdy3 = RMY(3, j);
-  const R arh3 = ARH(3, j), rarh3 = RARH(3, j);
-  const R sn = nrow ? ld(P.sch_r, qn) : 1.0, rsn = nrow ? ld(P.rsch, qn) : 1.0;
-  const R ss = srow ? ld(P.sch_r, qs) : 1.0, rss = srow ? ld(P.rsch, qs) : 1.0;
-  const R rh3n = nrow ? RH(3, j + 1) : 0.0, rh3s = srow ? RH(3, j - 1) : 0.0;
-  const R cv1 = ld(P.cv1, q2), cv2 = ld(P.cv2, q2);
-  const R dx4 = MX(4, i), dx4e = MX(4, i + 1), rdx4 = RMX(4, i), rdx4e = RMX(4, i + 1);
-  const R arh4 = ARH(4, j), rarh4 = RARH(4, j);
-  const R my2 = MY(2, j), rmy2 = RMY(2, j);
-  const R my2n = nrow ? MY(2, j + 1) : 1.0, rmy2n = nrow ? RMY(2, j + 1) : 1.0;
-  const R c00 = ld(P.chc, q2), c10 = ld(P.chc, qe);
-  const R c01 = nrow ? ld(P.chc, qn) : 0.0, c11 = nrow ? ld(P.chc, qn + 1) : 0.0;
-  const R chN0 = nrow ? 0.5 * (c00 + c01) : 0.0, chN1 = nrow ? 0.5 * (c10 + c11) : 0.0;
-  const R chE0 = 0.5 * (c00 + c10), chE1 = nrow ? 0.5 * (c01 + c11) : 0.0;
-  const R rh2 = RH(2, j), rh2n = nrow ? RH(2, j + 1) : 0.0;
-  const R dxc = a * RH(4, j) * (dx4 + dx4e);
-  const R rdxc = 1.0 / dxc;
-  const R rsch2 = ld(P.rsch2, q2);
-  const R tx_ = ld(P.taux, q2), ty_ = ld(P.tauy, q2);
-  const R pax = ld(P.pax, q2), pay = ld(P.pay, q2);
-  // w on U: ter_{T->U}(wm / chc) at level kk (rows j <= njm)
-  const R rc00 = ld(P.rchc, q2), rc01 = nrow ? ld(P.rchc, qn) : 1.0;
-  const R rc10 = ld(P.rchc, qe), rc11 = nrow ? ld(P.rchc, qn + 1) : 1.0;
-  auto wU = [&](int kk) -> R {
-    if (!nrow) return 0.0;
-    const long long ok_ = n2 * (kk - 1);
-    return (dvr(ld(P.wm, q2 + ok_), c00, rc00) + dvr(ld(P.wm, qn + ok_), c01, rc01) +
-            dvr(ld(P.wm, qe + ok_), c10, rc10) + dvr(ld(P.wm, qn + 1 + ok_), c11, rc11)) *
-           0.25;
+  // offsets within a plane fit 32 bits
+  const unsigned q2 = (unsigned)I2(P, in ? i : 2, in ? j : 1);
+  const int lu = in ? P.lev_u[q2] : 0;
+  // the warp marches to the level below its deepest bottom (which takes the
+  // bottom drag); what lies below is zero
+  const int deep = __reduce_max_sync(0xffffffffu, lu);
+  const int kw = min(nk, deep + 1);
+  const int per = (kw + NC - 1) / NC, ka = part * per + 1, kb = min(kw, (part + 1) * per);
+  const unsigned twin = i == 2 ? ni - 2 : (i == ni - 1 ? 2u - ni : 0u);  // to the halo twin (modulo 2^32)
+  auto put = [&](R *p, R v) {
+    p[q2] = v;
+    if (twin) p[q2 + twin] = v;
   };
-  const int lev1 = lu;
-  // rolling: u, v at k-1, k; w on U at k; km at k
-  R u_km = 0.0, v_km = 0.0;
-  R u_c = ld(P.uc, q2), v_c = ld(P.vc, q2);
-  R wUk = wU(1);
-  R km_k = ld(P.km, q2);
-  double su = 0.0, sv = 0.0;
-  for (int k = 1; k <= nk; ++k) {
-    const long long o = n2 * (k - 1);
-    const R mu_k = (R)(lu >= k), mu_k1 = (R)(lu >= k + 1), mu_km = (R)(lu >= k - 1);
-    auto U = [&](long long q) { return ld(P.uc, q + o); };
-    auto V = [&](long long q) { return ld(P.vc, q + o); };
-    // velocities at level k (unweighted wu = uc/sch, wv = vc/sch)
-    const R u_e = U(qe), u_w = U(qw);
-    const R v_e = V(qe), v_w = V(qw);
-    const R wu_c = dvr(u_c, sch, rsch), wu_e = dvr(u_e, sch_e, rsc_e), wu_w = dvr(u_w, sch_w, rsc_w);
-    const R wv_c = dvr(v_c, sch, rsch), wv_e = dvr(v_e, sch_e, rsc_e), wv_w = dvr(v_w, sch_w, rsc_w);
-    R u_n = 0, u_s = 0, v_n = 0, v_s = 0, wu_n = 0, wu_s = 0, wv_n = 0, wv_s = 0;
-    if (nrow) {
-      u_n = U(qn); v_n = V(qn);
-      wu_n = dvr(u_n, sn, rsn); wv_n = dvr(v_n, sn, rsn);
-    }
-    if (srow) {
-      u_s = U(qs); v_s = V(qs);
-      wu_s = dvr(u_s, ss, rss); wv_s = dvr(v_s, ss, rss);
-    }
-    // vertical neighbours at (i, j)
-    const R u_k1 = (k < nk) ? ld(P.uc, q2 + o + n2) : 0.0, v_k1 = (k < nk) ? ld(P.vc, q2 + o + n2) : 0.0;
-    // u on N (i, j), (i+1, j); v*cos on E (i, j), (i, j+1)
-    const R uN0 = 0.5 * (wu_w + wu_c), uN1 = 0.5 * (wu_c + wu_e);
-    const R vE0 = srow ? 0.5 * (wv_s * rh3s + wv_c * rh3) : 0.0;
-    const R vE1 = nrow ? 0.5 * (wv_c * rh3 + wv_n * rh3n) : 0.0;
-    const R wUk1 = wU(k + 1);  // wm has nkp levels
-    const R dm1 = dvr(uN1 - uN0, dx3, rdx3);
-    const R dm2 = nrow ? dvr(vE1 - vE0, dy3, rdy3) : 0.0;
-    const R dw = DIVDP(wUk - wUk1, k);
-    const R rdiv = dvr(dm1 + dm2, arh3, rarh3) + dw;
-    // op_adv(var)
-    auto adv = [&](R x_c, R x_e, R x_w, R x_n, R x_s, R x_km, R x_k1) {
-      const R wk1_0 = (0.5 * (x_w + x_c)) * uN0, wk1_1 = (0.5 * (x_c + x_e)) * uN1;
-      const R wk2_0 = srow ? (0.5 * (x_s + x_c)) * vE0 : 0.0;
-      const R wk2_1 = nrow ? (0.5 * (x_c + x_n)) * vE1 : 0.0;
-      const R wa = dvr(wk1_1 - wk1_0, dx3, rdx3);
-      const R wb = nrow ? dvr(wk2_1 - wk2_0, dy3, rdy3) : 0.0;
-      R ans = dvr(wa + wb, arh3, rarh3);
-      const R wkbp_k = (k >= 2) ? ((x_km + x_c) * 0.5 * wUk) * mu_km * mu_k : 0.0;
-      const R wkbp_k1 = (k < nk) ? ((x_c + x_k1) * 0.5 * wUk1) * mu_k * mu_k1 : 0.0;
-      ans = ans + DIVDP(wkbp_k - wkbp_k1, k);
-      ans = ans - 0.5 * x_c * rdiv;
-      return ans * mu_k;
-    };
-    const R auc = adv(u_c, u_e, u_w, u_n, u_s, u_km, u_k1);
-    const R avc = adv(v_c, v_e, v_w, v_n, v_s, v_km, v_k1);
-    // fri_r3d(ans, sch, v, vp, vc, tau)
-    const R am = ld(P.am, q2 + o);
-    const R km_k1 = ld(P.km, q2 + o + n2);  // km has nkp levels
-    auto fri = [&](R vc_, R ve_, R vw_, R vn_, R vs_, R vp_km, R vp_c, R vp_k1, R vce, R vcw, R v_bot_k,
-                   R vc_bot_k, R v_bot_km, R vc_bot_km, R tau) -> R {
-      const R wx0 = dvr(dvr(vc_ - vw_, dx4, rdx4), arh4, rarh4);
-      const R wx1 = dvr(dvr(ve_ - vc_, dx4e, rdx4e), arh4, rarh4);
-      const R wy0 = srow ? DIVA(dvr(vc_ - vs_, my2, rmy2)) : 0.0;
-      const R wy1 = nrow ? DIVA(dvr(vn_ - vc_, my2n, rmy2n)) : 0.0;
-      const R va0 = chN0 * wx0, va1 = chN1 * wx1;
-      const R vb0 = (chE0 * wy0) * rh2, vb1 = (chE1 * wy1) * rh2n;
-      const R A = dvr(va1 - va0, dx3, rdx3);
-      const R B = nrow ? dvr(vb1 - vb0, dy3, rdy3) : 0.0;
-      const R wka = dvr(A + B, arh3, rarh3);
-      R ans = dvr(am, sch, rsch) * wka;
-      ans = ans + am * cv1 * vp_c;
-      const R pxc = dvr(vce - vcw, dxc, rdxc);
-      ans = ans + am * cv2 * sch * pxc;
-      // wkp at kk = k and k+1: surface stress, bottom drag at lev+1, else
-      // the km-scaled pz (mod_op.f90:147-161)
-      auto wkp = [&](int kk, R vp_a, R vp_b, R v_bot, R vc_bot, R kmv) -> R {
-        if (kk == 1) return dvr(g * tau, sch, rsch);
-        if (lev1 > 0 && kk == lev1 + 1) {
-          const R mag = sqrt(v_bot * v_bot + vc_bot * vc_bot);
-          return dvr(v_bot * g * P.c.cdbot * mag, sch, rsch);
-        }
-        if (kk > nk) return 0.0;
-        const R pzv = dvr((vp_a - vp_b) * (R)(lev1 >= kk - 1) * (R)(lev1 >= kk), P.dz1[kk], P.rdz1[kk]);
-        return dvr(grho * kmv * pzv, sch * sch, rsch2);
-      };
-      const R wkp_k = wkp(k, vp_km, vp_c, v_bot_km, vc_bot_km, km_k);
-      const R wkp_k1 = wkp(k + 1, vp_c, vp_k1, v_bot_k, vc_bot_k, km_k1);
-      return ans * mu_k + DIVDP(wkp_k - wkp_k1, k);
-    };
-    // level k-1 values for a bottom drag at kk = k (lev = k-1)
-    R wu_km = 0.0, wv_km = 0.0;
-    if (k > 1 && lev1 == k - 1) { wu_km = dvr(u_km, sch, rsch); wv_km = dvr(v_km, sch, rsch); }
-    // fx = fri(v = uc/sch, vp = uc, vc = -(vc/sch), taux)
-    const R fx = fri(wu_c, wu_e, wu_w, wu_n, wu_s, u_km, u_c, u_k1, -wv_e, -wv_w, wu_c, -wv_c, wu_km, -wv_km, tx_);
-    // fy = fri(v = vc/sch, vp = vc, vc = uc/sch, tauy)
-    const R fy = fri(wv_c, wv_e, wv_w, wv_n, wv_s, v_km, v_c, v_k1, wu_e, wu_w, wv_c, wu_c, wv_km, wu_km, ty_);
-    const long long q = q2 + o;
-    st2(P.auc, P, i, q, auc);
-    st2(P.avc, P, i, q, avc);
+  auto put3 = [&](long long o, R auc, R avc, R fx, R fy) {
+    put(P.auc + o, auc);
+    put(P.avc + o, avc);
     if (P.ab3_mode == 1) {
-      st2(P.aup, P, i, q, auc); st2(P.aupp, P, i, q, auc);
-      st2(P.avp, P, i, q, avc); st2(P.avpp, P, i, q, avc);
+      put(P.aup + o, auc); put(P.aupp + o, auc);
+      put(P.avp + o, avc); put(P.avpp + o, avc);
     }
-    st2(P.fx, P, i, q, fx);
-    st2(P.fy, P, i, q, fy);
-    const R wx = -auc - sch * P.c.a0 * pax + fx;
-    const R wy = -avc - sch * P.c.a0 * pay + fy;
-    su = su + (double)wx * P.dpr2[k] * (double)mu_k;
-    sv = sv + (double)wy * P.dpr2[k] * (double)mu_k;
-    u_km = u_c; u_c = u_k1; v_km = v_c; v_c = v_k1;
-    wUk = wUk1;
-    km_k = km_k1;
+    put(P.fx + o, fx);
+    put(P.fy + o, fy);
+  };
+  const R g = P.c.g;
+  double su = 0.0, sv = 0.0;
+  if (in && deep == 0) {
+    // land: the surface stress at level 1 only
+    if (part == 0) {
+      const R sch = ld(P.sch_r, q2), rsch = ld(P.rsch, q2);
+      const R fx = DIVDP(dvr(g * ld(P.taux, q2), sch, rsch), 1), fy = DIVDP(dvr(g * ld(P.tauy, q2), sch, rsch), 1);
+      put3(0, 0.0, 0.0, fx, fy);
+    }
+  } else if (in && ka <= kb) {
+    const R a = P.c.a;
+    const R grho = g * P.c.rho0;
+    const bool nrow = j <= P.njm, srow = j >= 2;
+    // (rows past the domain: any value, every use is guarded by nrow or srow)
+    const unsigned qe = q2 + 1, qw = q2 - 1, qn = nrow ? q2 + ni : q2, qs = srow ? q2 - ni : q2, qne = qn + 1;
+    const int jn = nrow ? j + 1 : j, js = srow ? j - 1 : j;
+    // column constants (k_readyc3d: the per-point prologue)
+    const R sch = ld(P.sch_r, q2), rsch = ld(P.rsch, q2);
+    const R rsc_e = ld(P.rsch, qe), rsc_w = ld(P.rsch, qw);
+    const R sch_e = ld(P.sch_r, qe), sch_w = ld(P.sch_r, qw);
+    const R rh3 = RH(3, j), dx3 = MX(3, i), rdx3 = RMX(3, i), dy3 = MY(3, j), rdy3 = RMY(3, j);
+    const R arh3 = ARH(3, j), rarh3 = RARH(3, j);
+    const R sn = ld(P.sch_r, qn), rsn = ld(P.rsch, qn), ss = ld(P.sch_r, qs), rss = ld(P.rsch, qs);
+    const R rh3n = RH(3, jn), rh3s = RH(3, js);
+    const R cv1 = ld(P.cv1, q2), cv2 = ld(P.cv2, q2);
+    const R dx4 = MX(4, i), dx4e = MX(4, i + 1), rdx4 = RMX(4, i), rdx4e = RMX(4, i + 1);
+    const R arh4 = ARH(4, j), rarh4 = RARH(4, j);
+    const R my2 = MY(2, j), rmy2 = RMY(2, j), my2n = MY(2, jn), rmy2n = RMY(2, jn);
+    const R c00 = ld(P.chc, q2), c10 = ld(P.chc, qe), c01 = ld(P.chc, qn), c11 = ld(P.chc, qne);
+    const R chN0 = nrow ? 0.5 * (c00 + c01) : 0.0, chN1 = nrow ? 0.5 * (c10 + c11) : 0.0;
+    const R chE0 = 0.5 * (c00 + c10), chE1 = nrow ? 0.5 * (c01 + c11) : 0.0;
+    const R rh2 = RH(2, j), rh2n = nrow ? RH(2, jn) : 0.0;
+    const R dxc = a * RH(4, j) * (dx4 + dx4e);
+    const R rdxc = 1.0 / dxc;
+    const R rsch2 = ld(P.rsch2, q2);
+    const R pgx = sch * P.c.a0 * ld(P.pax, q2), pgy = sch * P.c.a0 * ld(P.pay, q2);
+    // w on U: ter_{T->U}(wm / chc) at level kk (rows j <= njm)
+    const R rc00 = ld(P.rchc, q2), rc01 = ld(P.rchc, qn), rc10 = ld(P.rchc, qe), rc11 = ld(P.rchc, qne);
+    auto wU = [&](int kk) -> R {
+      const R *w = P.wm + n2 * (kk - 1);
+      const R v = (dvr(ld(w, q2), c00, rc00) + dvr(ld(w, qn), c01, rc01) + dvr(ld(w, qe), c10, rc10) +
+                   dvr(ld(w, qne), c11, rc11)) *
+                  0.25;
+      return nrow ? v : 0.0;
+    };
+    // vertical advective flux at the top of level kk >= 2: values above and
+    // below, w there
+    auto vadv = [&](int kk, R xm, R xc, R w) -> R { return lu >= kk ? (xm + xc) * 0.5 * w : 0.0; };
+    // vertical stress at the top of level kk >= 2: bottom drag at lev + 1
+    // (from the unweighted velocities above), else the km-scaled pz
+    // (mod_op.f90:147-161)
+    auto stress = [&](int kk, R vp_a, R vp_b, R v_bot, R vc_bot, R kmv) -> R {
+      R r = 0.0;
+      if (lu > 0 && kk == lu + 1) {
+        const R mag = sqrt(v_bot * v_bot + vc_bot * vc_bot);
+        r = dvr(v_bot * g * P.c.cdbot * mag, sch, rsch);
+      } else if (lu >= kk) {
+        const R pzv = dvr(vp_a - vp_b, P.dz1[kk], P.rdz1[kk]);
+        r = dvr(grho * kmv * pzv, sch * sch, rsch2);
+      }
+      return r;
+    };
+    // level ka: u, v, w on U, and the fluxes through its top
+    const R *uk = P.uc + n2 * (ka - 1), *vk = P.vc + n2 * (ka - 1);
+    R u_c = ld(uk, q2), v_c = ld(vk, q2);
+    R wUk = wU(ka);
+    R adv_u = 0.0, adv_v = 0.0, str_u, str_v;
+    if (ka == 1) {
+      str_u = dvr(g * ld(P.taux, q2), sch, rsch);
+      str_v = dvr(g * ld(P.tauy, q2), sch, rsch);
+    } else {
+      const R u_m = ld(uk - n2, q2), v_m = ld(vk - n2, q2), km_k = ld(P.km + n2 * (ka - 1), q2);
+      const R wu_m = dvr(u_m, sch, rsch), wv_m = dvr(v_m, sch, rsch);
+      adv_u = vadv(ka, u_m, u_c, wUk);
+      adv_v = vadv(ka, v_m, v_c, wUk);
+      str_u = stress(ka, u_m, u_c, wu_m, -wv_m, km_k);
+      str_v = stress(ka, v_m, v_c, wv_m, wu_m, km_k);
+    }
+    for (int k = ka; k <= kb; ++k) {
+      const long long o = n2 * (k - 1);
+      const R *u = P.uc + o, *v = P.vc + o;
+      const bool wet = lu >= k, more = k < kw;  // (below kw every flux is masked)
+      const R u_e = ld(u, qe), u_w = ld(u, qw), u_n = ld(u, qn), u_s = ld(u, qs);
+      const R v_e = ld(v, qe), v_w = ld(v, qw), v_n = ld(v, qn), v_s = ld(v, qs);
+      const R u_k1 = more ? ld(u + n2, q2) : 0.0, v_k1 = more ? ld(v + n2, q2) : 0.0;
+      const R wUk1 = wU(k + 1);                                                // wm has nkp levels
+      const R am = ld(P.am + o, q2), km_k1 = ld(P.km + o + n2, q2);            // km has nkp levels
+      // unweighted velocities (wu = uc/sch, wv = vc/sch)
+      const R wu_c = dvr(u_c, sch, rsch), wu_e = dvr(u_e, sch_e, rsc_e), wu_w = dvr(u_w, sch_w, rsc_w);
+      const R wv_c = dvr(v_c, sch, rsch), wv_e = dvr(v_e, sch_e, rsc_e), wv_w = dvr(v_w, sch_w, rsc_w);
+      const R wu_n = dvr(u_n, sn, rsn), wv_n = dvr(v_n, sn, rsn);
+      const R wu_s = dvr(u_s, ss, rss), wv_s = dvr(v_s, ss, rss);
+      // u on N (i, j), (i+1, j); v*cos on E (i, j), (i, j+1)
+      const R uN0 = 0.5 * (wu_w + wu_c), uN1 = 0.5 * (wu_c + wu_e);
+      const R vE0 = srow ? 0.5 * (wv_s * rh3s + wv_c * rh3) : 0.0;
+      const R vE1 = nrow ? 0.5 * (wv_c * rh3 + wv_n * rh3n) : 0.0;
+      const R dm1 = dvr(uN1 - uN0, dx3, rdx3);
+      const R dm2 = nrow ? dvr(vE1 - vE0, dy3, rdy3) : 0.0;
+      const R dw = DIVDP(wUk - wUk1, k);
+      const R rdiv = dvr(dm1 + dm2, arh3, rarh3) + dw;
+      // op_adv(var); top: the flux through the level's top, then its bottom's
+      auto adv = [&](R x_c, R x_e, R x_w, R x_n, R x_s, R x_k1, R &top) {
+        const R wk1_0 = (0.5 * (x_w + x_c)) * uN0, wk1_1 = (0.5 * (x_c + x_e)) * uN1;
+        const R wk2_0 = srow ? (0.5 * (x_s + x_c)) * vE0 : 0.0;
+        const R wk2_1 = nrow ? (0.5 * (x_c + x_n)) * vE1 : 0.0;
+        const R wa = dvr(wk1_1 - wk1_0, dx3, rdx3);
+        const R wb = nrow ? dvr(wk2_1 - wk2_0, dy3, rdy3) : 0.0;
+        R ans = dvr(wa + wb, arh3, rarh3);
+        const R bot = vadv(k + 1, x_c, x_k1, wUk1);
+        ans = ans + DIVDP(top - bot, k);
+        top = bot;
+        ans = ans - 0.5 * x_c * rdiv;
+        return wet ? ans : 0.0;
+      };
+      const R auc = adv(u_c, u_e, u_w, u_n, u_s, u_k1, adv_u);
+      const R avc = adv(v_c, v_e, v_w, v_n, v_s, v_k1, adv_v);
+      // fri_r3d(ans, sch, v, vp, vc, tau)
+      const R ams = dvr(am, sch, rsch);
+      auto fri = [&](R vc_, R ve_, R vw_, R vn_, R vs_, R vp_c, R vce, R vcw, R &top, R bot) -> R {
+        const R wx0 = dvr(dvr(vc_ - vw_, dx4, rdx4), arh4, rarh4);
+        const R wx1 = dvr(dvr(ve_ - vc_, dx4e, rdx4e), arh4, rarh4);
+        const R wy0 = srow ? DIVA(dvr(vc_ - vs_, my2, rmy2)) : 0.0;
+        const R wy1 = nrow ? DIVA(dvr(vn_ - vc_, my2n, rmy2n)) : 0.0;
+        const R va0 = chN0 * wx0, va1 = chN1 * wx1;
+        const R vb0 = (chE0 * wy0) * rh2, vb1 = (chE1 * wy1) * rh2n;
+        const R A = dvr(va1 - va0, dx3, rdx3);
+        const R B = nrow ? dvr(vb1 - vb0, dy3, rdy3) : 0.0;
+        const R wka = dvr(A + B, arh3, rarh3);
+        R ans = ams * wka;
+        ans = ans + am * cv1 * vp_c;
+        const R pxc = dvr(vce - vcw, dxc, rdxc);
+        ans = ans + am * cv2 * sch * pxc;
+        const R r = (wet ? ans : 0.0) + DIVDP(top - bot, k);
+        top = bot;
+        return r;
+      };
+      // fx = fri(v = uc/sch, vp = uc, vc = -(vc/sch), taux)
+      const R fx = fri(wu_c, wu_e, wu_w, wu_n, wu_s, u_c, -wv_e, -wv_w, str_u, stress(k + 1, u_c, u_k1, wu_c, -wv_c, km_k1));
+      // fy = fri(v = vc/sch, vp = vc, vc = uc/sch, tauy)
+      const R fy = fri(wv_c, wv_e, wv_w, wv_n, wv_s, v_c, wu_e, wu_w, str_v, stress(k + 1, v_c, v_k1, wv_c, wu_c, km_k1));
+      put3(o, auc, avc, fx, fy);
+      const R wx = -auc - pgx + fx;
+      const R wy = -avc - pgy + fy;
+      const double tu = wet ? wx * P.dpr2[k] : 0.0, tv = wet ? wy * P.dpr2[k] : 0.0;
+      if (NC > 1) {
+        sh[(k - 1) * kColX + threadIdx.x] = tu;
+        sh[(nk + k - 1) * kColX + threadIdx.x] = tv;
+      } else {
+        su = su + tu;
+        sv = sv + tv;
+      }
+      u_c = u_k1; v_c = v_k1;
+      wUk = wUk1;
+    }
   }
-  st2(P.ut, P, i, q2, dvr(su, ld(P.prh_u, q2), ld(P.rprh_u, q2)));
-  st2(P.vt, P, i, q2, dvr(sv, ld(P.prh_u, q2), ld(P.rprh_u, q2)));
+  if (in)
+    for (int k = kw + 1 + part; k <= nk; k += NC) put3(n2 * (k - 1), 0.0, 0.0, 0.0, 0.0);
+  if (NC > 1) {
+    __syncthreads();
+    if (part == 0 && in)
+      for (int k = 1; k <= lu; ++k) {
+        su = su + sh[(k - 1) * kColX + threadIdx.x];
+        sv = sv + sh[(nk + k - 1) * kColX + threadIdx.x];
+      }
+  }
+  if (part == 0 && in) {
+    put(P.ut, dvr(su, ld(P.prh_u, q2), ld(P.rprh_u, q2)));
+    put(P.vt, dvr(sv, ld(P.prh_u, q2), ld(P.rprh_u, q2)));
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -665,6 +729,11 @@ __global__ void __launch_bounds__(512, 2) k_clin(const __grid_constant__ DevT<R>
   const long long qe = q2 + 1, qn = q2 + ni;
   const double bc = (double)P.bc;
   for (int k = threadIdx.y + 1; k <= nk && ok; k += TB_K) {
+    if (k > lu) {  // below the bottom: no tendency
+      uns[(k - 1) * TB_X + tx] = (double)P.up[q2 + P.n2 * (k - 1)];
+      vns[(k - 1) * TB_X + tx] = (double)P.vp[q2 + P.n2 * (k - 1)];
+      continue;
+    }
     const double sch = ld(P.schc, q2);
     // gra(mch) on E (i, j), (i, j+1) and on N (i, j), (i+1, j)
     auto gE = [&](const double *f, long long q, int jj) { return DIVARH(DIVX(ld(f, q + 1) - ld(f, q), 2, i), 2, jj); };
@@ -714,21 +783,20 @@ __global__ void __launch_bounds__(512, 2) k_clin(const __grid_constant__ DevT<R>
     p2 = w2 - w * w1;
     w = 1 + w * w;
     const double rw = ld(P.rwc, q2);
-    const double mu = (double)(lu >= k);
-    p1 = dvr(p1 * mu, w, rw);
-    p2 = dvr(p2 * mu, w, rw);
+    p1 = dvr(p1, w, rw);
+    p2 = dvr(p2, w, rw);
     const double un = P.up[q] + p1 * bc;
     const double vn = P.vp[q] + p2 * bc;
     uns[(k - 1) * TB_X + tx] = (double)(R)un;
     vns[(k - 1) * TB_X + tx] = (double)(R)vn;
-    t1s[(k - 1) * TB_X + tx] = un * P.dpr2[k] * mu;
-    t2s[(k - 1) * TB_X + tx] = vn * P.dpr2[k] * mu;
+    t1s[(k - 1) * TB_X + tx] = un * P.dpr2[k];
+    t2s[(k - 1) * TB_X + tx] = vn * P.dpr2[k];
   }
   __syncthreads();
   if (ok && threadIdx.y < 2) {
     const double *t = threadIdx.y == 0 ? t1s : t2s;
     double s = 0.0;
-    for (int k = 1; k <= nk; ++k) s = s + t[(k - 1) * TB_X + tx];
+    for (int k = 1; k <= lu; ++k) s = s + t[(k - 1) * TB_X + tx];
     wsum[threadIdx.y * TB_X + tx] = dvr(s, ld(P.prh_u, q2), ld(P.rprh_u, q2));
   }
   __syncthreads();
@@ -807,21 +875,16 @@ __global__ void __launch_bounds__(512) k_ssh(const __grid_constant__ DevT<R> P0,
   const long long q2 = ok ? I2(P, i, j) : 0;
   const int lev = ok ? P.lev_t[q2] : 0;
   const double mch = ok ? P.mch[q2] : 0.0;
-  for (int k = threadIdx.y + 1; k <= nk && ok; k += TB_K) {
+  for (int k = threadIdx.y + 1; k <= lev; k += TB_K) {
     const long long q = q2 + P.n2 * (k - 1);
-    double al;
-    if (k <= lev) {
-      al = 1.0 / den_rho(P.c, P.tp[q], P.sp[q], mch * P.pr2[k]);
-      P.alpha[q] = alpha_store(P, al, k);
-    } else {
-      al = alpha_full(P, P.alpha[q], k);
-    }
-    sh[(k - 1) * TB_X + tx] = al * P.dpr2[k] * mch * (double)(k <= lev);
+    const double al = 1.0 / den_rho(P.c, P.tp[q], P.sp[q], mch * P.pr2[k]);
+    P.alpha[q] = alpha_store(P, al, k);
+    sh[(k - 1) * TB_X + tx] = al * P.dpr2[k] * mch;
   }
   __syncthreads();
   if (!ok || threadIdx.y != 0) return;
   double s = 0.0;
-  for (int k = 1; k <= nk; ++k) s = s + sh[(k - 1) * TB_X + tx];
+  for (int k = 1; k <= lev; ++k) s = s + sh[(k - 1) * TB_X + tx];
   double ssh = dvr(s, P.c.g, P.rg);
   ssh = dvr(P.phih_t[q2], P.c.g, P.rg) + ssh;
   P.acssh[q2] = P.acssh[q2] + ssh;
@@ -927,7 +990,15 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1) k_ts(const __grid
     const R c2c = nrow ? 0.5 * (mc + mn) : 0.0, c2s = srow ? 0.5 * (ms + mc) : 0.0;
     const R bc = (R)P.bc;
     const long long o = P.n2 * (k - 1), q = q2 + o;
-    const R m_c = (R)(lev >= k), m_w = (R)(lw >= k), m_e = (R)(le >= k);
+    if (k > lev) {  // below the bottom: T and S stay
+      tcs[(k - 1) * TB_X + tx] = (double)ld(P.tp, q);
+      scs[(k - 1) * TB_X + tx] = (double)ld(P.sp, q);
+      const auto pr = P.prho[q];
+      p1s[(k - 1) * TB_X + tx] = pr.x;
+      p2s[(k - 1) * TB_X + tx] = pr.y;
+      continue;
+    }
+    const R m_c = 1.0, m_w = (R)(lw >= k), m_e = (R)(le >= k);
     const R m_n = (R)(ln >= k), m_s = (R)(ls >= k);
     const R m_k1 = (R)(lev >= k + 1), m_km = (R)(lev >= k - 1);
     // mass-weighted velocity: um1 = uc*sch on U, um2 = vc*sch*rh3
@@ -1052,7 +1123,6 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1) k_ts(const __grid
 //
 // k_ts_acc: point-parallel, the halo twins of the new T, S and the
 // act/acs/acr accumulations (acr through the equation of state).
-constexpr int kColX = 32, kColY = 2;
 
 // one column of T, S and prho copied to local arrays, levels 1..nlev (+1 for prho)
 struct ColL {
@@ -1063,136 +1133,162 @@ struct ColL {
   __device__ double P2(int k) const { return p2[k - 1]; }
 };
 
-template <bool BATCH>
-__global__ void __launch_bounds__(kColX * kColY, 7) k_ts_col(const __grid_constant__ DevT<double> P0,
-                                                            const DevT<double> *__restrict__ Ps) {
+// NC > 1: NC threads share a column's levels, as in k_readyc_col; the
+// stability test across their borders and the adjustment follow after a CTA
+// barrier.
+template <bool BATCH, int NC>
+__global__ void __launch_bounds__(kColX * (NC == 1 ? 2 : NC), NC == 1 ? 6 : 3)
+    k_ts_col(const __grid_constant__ DevT<double> P0, const DevT<double> *__restrict__ Ps) {
   using R = double;
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
+  __shared__ int s_unstable[kColX];
   const int x = blockIdx.x * kColX + threadIdx.x;
-  const int j = blockIdx.y * kColY + threadIdx.y + P.j_lo;
-  if (x >= P.glo_ni || j > P.j_hi) return;
+  const int j = blockIdx.y * (NC == 1 ? 2 : 1) + threadIdx.y + P.j_lo;
+  const int part = NC > 1 ? threadIdx.z : 0;
+  const bool in = x < P.glo_ni && j <= P.j_hi;
   const int i = x + 2;
-  const int nk = P.nk;
+  const int nk = P.nk, ni = P.ni;
   const long long n2 = P.n2;
-  const long long q2 = I2(P, i, j);
-  const int ni = P.ni;
-  const R g = P.c.g;
-  const R grho = g * P.c.rho0;
-  const bool nrow = j <= P.njm, srow = j >= 2;
-  const long long qw = q2 - 1, qs = q2 - ni, qsw = qs - 1, qe = q2 + 1, qn = q2 + ni;
-  const int lev = P.lev_t[q2];
-  // column constants (k_ts: the per-point prologue)
-  const int lw = P.lev_t[qw], le = P.lev_t[qe], ln = nrow ? P.lev_t[qn] : 0, ls = srow ? P.lev_t[qs] : 0;
-  const R rh4c = RH(4, j), rh4s = srow ? RH(4, j - 1) : 0.0;
-  const R sc_c = ld(P.sch_r, q2), sc_w = ld(P.sch_r, qw);
-  const R sc_s = srow ? ld(P.sch_r, qs) : 0.0, sc_sw = srow ? ld(P.sch_r, qsw) : 0.0;
-  const R r3c = RH(3, j), r3s = srow ? RH(3, j - 1) : 0.0;
-  const R mc = ld(P.mch, q2), me = ld(P.mch, qe), mw = ld(P.mch, qw);
-  const R mn = nrow ? ld(P.mch, qn) : 0.0, ms = srow ? ld(P.mch, qs) : 0.0;
-  const R c1c = 0.5 * (mc + me), c1w = 0.5 * (mw + mc);
-  const R c2c = nrow ? 0.5 * (mc + mn) : 0.0, c2s = srow ? 0.5 * (ms + mc) : 0.0;
-  const R bc = (R)P.bc;
-  const double rmc = ld(P.rmch, q2);
-  // metric factors of the divisions (the DIVX/DIVY/DIVARH operands)
-  const R mx2c = MX(2, i), rmx2c = RMX(2, i), mx2w = MX(2, i - 1), rmx2w = RMX(2, i - 1);
-  const R mx1c = MX(1, i), rmx1c = RMX(1, i);
-  const R my4c = MY(4, j), rmy4c = RMY(4, j), my1c = MY(1, j), rmy1c = RMY(1, j);
-  const R my4s = srow ? MY(4, j - 1) : 1.0, rmy4s = srow ? RMY(4, j - 1) : 1.0;
-  const R arh1 = ARH(1, j), rarh1 = RARH(1, j), arh2 = ARH(2, j), rarh2 = RARH(2, j);
-  // rolling vertical neighbours: x(k-1), x(k)
-  R tc_m = 0, tc_c = ld(P.tc, q2), sc_m = 0, sc_cc = ld(P.sc, q2);
-  R tp_m = 0, tp_c = ld(P.tp, q2), sp_m = 0, sp_c = ld(P.sp, q2);
-  R wm_c = ld(P.wm, q2), kh_c = ld(P.kh, q2);
-  double t_prev = 0.0, s_prev = 0.0;
+  const unsigned q2 = (unsigned)I2(P, in ? i : 2, in ? j : 1);
+  const int lev = in ? P.lev_t[q2] : 0;
+  // the warp marches to its deepest bottom; below, T and S stay
+  const int kw = __reduce_max_sync(0xffffffffu, lev);
+  const int per = (kw + NC - 1) / NC, ka = part * per + 1, kb = min(kw, (part + 1) * per);
   bool unstable = false;
-  for (int k = 1; k <= nk; ++k) {
-    const long long o = n2 * (k - 1), q = q2 + o;
-    const R m_c = (R)(lev >= k), m_w = (R)(lw >= k), m_e = (R)(le >= k);
-    const R m_n = (R)(ln >= k), m_s = (R)(ls >= k);
-    const R m_k1 = (R)(lev >= k + 1), m_km = (R)(lev >= k - 1);
-    // mass-weighted velocity: um1 = uc*sch on U, um2 = vc*sch*rh3
-    const R um1c = ld(P.uc, q) * sc_c, um1w = ld(P.uc, qw + o) * sc_w;
-    const R um1s = srow ? ld(P.uc, qs + o) * sc_s : 0.0, um1sw = srow ? ld(P.uc, qsw + o) * sc_sw : 0.0;
-    const R um2c = ld(P.vc, q) * sc_c * r3c, um2w = ld(P.vc, qw + o) * sc_w * r3c;
-    const R um2s = srow ? ld(P.vc, qs + o) * sc_s * r3s : 0.0;
-    const R um2sw = srow ? ld(P.vc, qsw + o) * sc_sw * r3s : 0.0;
-    const R wa1c = srow ? 0.5 * (um1s + um1c) : 0.0, wa1w = srow ? 0.5 * (um1sw + um1w) : 0.0;
-    const R wa2c = 0.5 * (um2w + um2c), wa2s = srow ? 0.5 * (um2sw + um2s) : 0.0;
-    const R wmk = wm_c, wmk1 = ld(P.wm, q + n2);  // wm has nkp levels
-    const R khk = kh_c, khk1 = (k < nk) ? ld(P.kh, q + n2) : 0.0;
-    auto adv = [&](const R *var, R xc, R xkm, R xk1) -> R {
-      const R xe = ld(var, qe + o), xw = ld(var, qw + o);
-      const R xn = nrow ? ld(var, qn + o) : 0.0, xs = srow ? ld(var, qs + o) : 0.0;
-      const R w1c = dvr(xe - xc, mx2c, rmx2c), w1w = dvr(xc - xw, mx2w, rmx2w);
-      const R wb1 = 0.5 * (wa1w * w1w + wa1c * w1c);
-      R ans = dvr(wb1, arh1, rarh1);
-      const R w2c = nrow ? dvr(xn - xc, my4c, rmy4c) : 0.0;
-      R wb2 = 0.0;
-      if (srow) {
-        const R w2s = dvr(xc - xs, my4s, rmy4s);
-        wb2 = 0.5 * (wa2s * w2s + wa2c * w2c);
-      }
-      ans = ans + dvr(wb2, arh1, rarh1);
-      const R wmp_k = (k >= 2) ? wmk * (xkm - xc) : wmk * 0.0;
-      const R wmp_k1 = (k < nk) ? wmk1 * (xc - xk1) : wmk1 * 0.0;
-      ans = ans + DIVDP((wmp_k + wmp_k1) * 0.5, k);
-      return ans;
+  if (NC > 1) {
+    if (part == 0) s_unstable[threadIdx.x] = 0;
+    __syncthreads();
+  }
+  if (in && ka <= kb) {
+    const R grho = P.c.g * P.c.rho0;
+    const bool nrow = j <= P.njm, srow = j >= 2;
+    // (rows past the domain: any value, every use is guarded by nrow or srow)
+    const unsigned qw = q2 - 1, qe = q2 + 1, qn = nrow ? q2 + ni : q2, qs = srow ? q2 - ni : q2, qsw = qs - 1;
+    const int js = srow ? j - 1 : j;
+    // column constants (k_ts: the per-point prologue)
+    const int lw = P.lev_t[qw], le = P.lev_t[qe], ln = nrow ? P.lev_t[qn] : 0, ls = srow ? P.lev_t[qs] : 0;
+    const R rh4c = RH(4, j), rh4s = RH(4, js);
+    const R sc_c = ld(P.sch_r, q2), sc_w = ld(P.sch_r, qw), sc_s = ld(P.sch_r, qs), sc_sw = ld(P.sch_r, qsw);
+    const R r3c = RH(3, j), r3s = RH(3, js);
+    const R mc = ld(P.mch, q2), me = ld(P.mch, qe), mw = ld(P.mch, qw), mn = ld(P.mch, qn), ms = ld(P.mch, qs);
+    const R c1c = 0.5 * (mc + me), c1w = 0.5 * (mw + mc), c2c = 0.5 * (mc + mn), c2s = 0.5 * (ms + mc);
+    const R bc = (R)P.bc;
+    const double rmc = ld(P.rmch, q2);
+    // metric factors of the divisions (the DIVX/DIVY/DIVARH operands)
+    const R mx2c = MX(2, i), rmx2c = RMX(2, i), mx2w = MX(2, i - 1), rmx2w = RMX(2, i - 1);
+    const R mx1c = MX(1, i), rmx1c = RMX(1, i);
+    const R my4c = MY(4, j), rmy4c = RMY(4, j), my1c = MY(1, j), rmy1c = RMY(1, j);
+    const R my4s = MY(4, js), rmy4s = RMY(4, js);
+    const R arh1 = ARH(1, j), rarh1 = RARH(1, j), arh2 = ARH(2, j), rarh2 = RARH(2, j);
+    // level ka: values and the vertical terms at its top.  wm dx3(var) of
+    // op_adv_ts (at the surface wm times 0), kh pz of op_dif
+    const long long oa = n2 * (ka - 1);
+    R tc_c = ld(P.tc + oa, q2), sc_cc = ld(P.sc + oa, q2), tp_c = ld(P.tp + oa, q2), sp_c = ld(P.sp + oa, q2);
+    auto dif3 = [&](int kk, R xa, R xb, R kh) -> R {
+      return lev >= kk ? grho * kh * dvr(xa - xb, P.dz1[kk], P.rdz1[kk]) : 0.0;
     };
-    auto dif = [&](const R *var, R xc, R xkm, R xk1) -> R {
-      const R xe = ld(var, qe + o), xw = ld(var, qw + o);
-      const R xn = nrow ? ld(var, qn + o) : 0.0, xs = srow ? ld(var, qs + o) : 0.0;
-      const R w1c = dvr(dvr((xe - xc) * m_e * m_c, mx2c, rmx2c), arh2, rarh2);
-      const R w1w = dvr(dvr((xc - xw) * m_c * m_w, mx2w, rmx2w), arh2, rarh2);
-      const R A = dvr(c1c * w1c - c1w * w1w, mx1c, rmx1c);
-      const R w2c = nrow ? DIVA(dvr((xn - xc) * m_n * m_c, my4c, rmy4c)) : 0.0;
-      R B = 0.0;
-      if (srow) {
-        const R w2s = DIVA(dvr((xc - xs) * m_c * m_s, my4s, rmy4s));
-        B = dvr((c2c * w2c) * rh4c - (c2s * w2s) * rh4s, my1c, rmy1c);
-      }
-      R ans = P.c.ah_c * dvr(A + B, arh1, rarh1);
-      R wkp_k = 0.0, wkp_k1 = 0.0;
-      if (k >= 2) {
-        const R pz = dvr((xkm - xc) * m_km * m_c, P.dz1[k], P.rdz1[k]);
-        wkp_k = grho * khk * pz;
-      }
-      if (k < nk) {
-        const R pz = dvr((xc - xk1) * m_c * m_k1, P.dz1[k + 1], P.rdz1[k + 1]);
-        wkp_k1 = grho * khk1 * pz;
-      }
-      ans = ans + DIVDP(wkp_k - wkp_k1, k);
-      return ans;
-    };
-    const R tc_k1 = (k < nk) ? ld(P.tc, q + n2) : 0.0, sc_k1 = (k < nk) ? ld(P.sc, q + n2) : 0.0;
-    const R tp_k1 = (k < nk) ? ld(P.tp, q + n2) : 0.0, sp_k1 = (k < nk) ? ld(P.sp, q + n2) : 0.0;
-    const R at = adv(P.tc, tc_c, tc_m, tc_k1), as = adv(P.sc, sc_cc, sc_m, sc_k1);
-    const R dt_ = dif(P.tp, tp_c, tp_m, tp_k1), ds_ = dif(P.sp, sp_c, sp_m, sp_k1);
-    R p1 = -at, p2 = -as;
-    p1 = p1 + dt_;
-    p2 = p2 + ds_;
-    if (k == 1) {
-      p1 = p1 + DIVDP(P.c.gamma_t * (ld(P.bnd_t, q2) - tc_c) * m_c, 1);
-      p2 = p2 + P.c.gamma_s * (ld(P.bnd_s, q2) - sc_cc) * m_c * mc;
+    const R wma = ld(P.wm + oa, q2);
+    R adv_t = wma * 0.0, adv_s = adv_t, dif_t = 0.0, dif_s = 0.0;
+    if (ka > 1) {
+      const R kh = ld(P.kh + oa, q2);
+      adv_t = wma * (ld(P.tc + oa - n2, q2) - tc_c);
+      adv_s = wma * (ld(P.sc + oa - n2, q2) - sc_cc);
+      dif_t = dif3(ka, ld(P.tp + oa - n2, q2), tp_c, kh);
+      dif_s = dif3(ka, ld(P.sp + oa - n2, q2), sp_c, kh);
     }
-    double tn = (double)tp_c + dvr((double)(p1 * bc * m_c), (double)mc, rmc);
-    const double sn = (double)sp_c + dvr((double)(p2 * bc * m_c), (double)mc, rmc);
-    if (m_c > 0 && tn < P.c.tice) tn = P.c.tice;
-    P.tn_[q] = tn;
-    P.sn_[q] = sn;
-    // convect's trigger: rhob(k-1) > rhoa(k) for 1 <= k-1 < lev
-    if (k >= 2 && k <= lev) {
+    double t_prev = 0.0, s_prev = 0.0;
+    for (int k = ka; k <= kb; ++k) {
+      const long long o = n2 * (k - 1);
+      const R *uo = P.uc + o, *vo = P.vc + o;
+      const bool more = k < kw;  // (at k = kw < nk the terms with the level below are masked, or w = 0 there)
+      const bool b_c = lev >= k, b_w = lw >= k, b_e = le >= k, b_n = ln >= k, b_s = ls >= k;
+      const R u_c = ld(uo, q2), u_w = ld(uo, qw), u_s = ld(uo, qs), u_sw = ld(uo, qsw);
+      const R v_c = ld(vo, q2), v_w = ld(vo, qw), v_s = ld(vo, qs), v_sw = ld(vo, qsw);
+      const R wmk1 = ld(P.wm + o + n2, q2);  // wm has nkp levels
+      const R khk1 = more ? ld(P.kh + o + n2, q2) : 0.0;
+      // mass-weighted velocity: um1 = uc*sch on U, um2 = vc*sch*rh3
+      const R um1c = u_c * sc_c, um1w = u_w * sc_w, um1s = u_s * sc_s, um1sw = u_sw * sc_sw;
+      const R um2c = v_c * sc_c * r3c, um2w = v_w * sc_w * r3c;
+      const R um2s = v_s * sc_s * r3s, um2sw = v_sw * sc_sw * r3s;
+      const R wa1c = srow ? 0.5 * (um1s + um1c) : 0.0, wa1w = srow ? 0.5 * (um1sw + um1w) : 0.0;
+      const R wa2c = 0.5 * (um2w + um2c), wa2s = srow ? 0.5 * (um2sw + um2s) : 0.0;
+      auto adv = [&](const R *var, R xc, R xk1, R &top) -> R {
+        const R xe = ld(var, qe), xw = ld(var, qw), xn = ld(var, qn), xs = ld(var, qs);
+        const R w1c = dvr(xe - xc, mx2c, rmx2c), w1w = dvr(xc - xw, mx2w, rmx2w);
+        const R wb1 = 0.5 * (wa1w * w1w + wa1c * w1c);
+        R ans = dvr(wb1, arh1, rarh1);
+        const R w2c = nrow ? dvr(xn - xc, my4c, rmy4c) : 0.0;
+        const R w2s = dvr(xc - xs, my4s, rmy4s);
+        const R wb2 = srow ? 0.5 * (wa2s * w2s + wa2c * w2c) : 0.0;
+        ans = ans + dvr(wb2, arh1, rarh1);
+        const R bot = more ? wmk1 * (xc - xk1) : wmk1 * 0.0;
+        ans = ans + DIVDP((top + bot) * 0.5, k);
+        top = bot;
+        return ans;
+      };
+      auto dif = [&](const R *var, R xc, R xk1, R &top) -> R {
+        const R xe = ld(var, qe), xw = ld(var, qw), xn = ld(var, qn), xs = ld(var, qs);
+        const R w1c = dvr(dvr(b_e && b_c ? xe - xc : 0.0, mx2c, rmx2c), arh2, rarh2);
+        const R w1w = dvr(dvr(b_c && b_w ? xc - xw : 0.0, mx2w, rmx2w), arh2, rarh2);
+        const R A = dvr(c1c * w1c - c1w * w1w, mx1c, rmx1c);
+        const R w2c = DIVA(dvr(b_n && b_c ? xn - xc : 0.0, my4c, rmy4c));
+        const R w2s = DIVA(dvr(b_c && b_s ? xc - xs : 0.0, my4s, rmy4s));
+        const R B = srow ? dvr((c2c * w2c) * rh4c - (c2s * w2s) * rh4s, my1c, rmy1c) : 0.0;
+        R ans = P.c.ah_c * dvr(A + B, arh1, rarh1);
+        const R bot = more ? dif3(k + 1, xc, xk1, khk1) : 0.0;
+        ans = ans + DIVDP(top - bot, k);
+        top = bot;
+        return ans;
+      };
+      const R tc_k1 = more ? ld(P.tc + o + n2, q2) : 0.0, sc_k1 = more ? ld(P.sc + o + n2, q2) : 0.0;
+      const R tp_k1 = more ? ld(P.tp + o + n2, q2) : 0.0, sp_k1 = more ? ld(P.sp + o + n2, q2) : 0.0;
+      const R at = adv(P.tc + o, tc_c, tc_k1, adv_t), as = adv(P.sc + o, sc_cc, sc_k1, adv_s);
+      const R dt_ = dif(P.tp + o, tp_c, tp_k1, dif_t), ds_ = dif(P.sp + o, sp_c, sp_k1, dif_s);
+      R p1 = -at, p2 = -as;
+      p1 = p1 + dt_;
+      p2 = p2 + ds_;
+      if (k == 1) {
+        const R m_c = b_c ? 1.0 : 0.0;
+        p1 = p1 + DIVDP(P.c.gamma_t * (ld(P.bnd_t, q2) - tc_c) * m_c, 1);
+        p2 = p2 + P.c.gamma_s * (ld(P.bnd_s, q2) - sc_cc) * m_c * mc;
+      }
+      double tn = tp_c + (b_c ? dvr(p1 * bc, mc, rmc) : 0.0);
+      const double sn = sp_c + (b_c ? dvr(p2 * bc, mc, rmc) : 0.0);
+      if (b_c && tn < P.c.tice) tn = P.c.tice;
+      P.tn_[q2 + o] = tn;
+      P.sn_[q2 + o] = sn;
+      // convect's trigger: rhob(k-1) > rhoa(k) for 1 <= k-1 < lev
+      if (k > ka && b_c) {
+        const double2 pr = P.prho[q2 + o];
+        const double rb = pr.x * t_prev + pr.y * s_prev;
+        const double ra = pr.x * tn + pr.y * sn;
+        if (rb > ra) unstable = true;
+      }
+      t_prev = tn;
+      s_prev = sn;
+      tc_c = tc_k1; sc_cc = sc_k1; tp_c = tp_k1; sp_c = sp_k1;
+    }
+  }
+  if (in)
+    for (int k = kw + 1 + part; k <= nk; k += NC) {
+      const long long o = n2 * (k - 1);
+      P.tn_[q2 + o] = ld(P.tp + o, q2);
+      P.sn_[q2 + o] = ld(P.sp + o, q2);
+    }
+  if (NC > 1) {
+    __syncthreads();  // the column's new T, S are in memory
+    if (in && ka > 1 && ka <= kb && ka <= lev) {  // against the part above
+      const long long q = q2 + n2 * (ka - 1);
       const double2 pr = P.prho[q];
-      const double rb = pr.x * t_prev + pr.y * s_prev;
-      const double ra = pr.x * tn + pr.y * sn;
+      const double rb = pr.x * P.tn_[q - n2] + pr.y * P.sn_[q - n2];
+      const double ra = pr.x * P.tn_[q] + pr.y * P.sn_[q];
       if (rb > ra) unstable = true;
     }
-    t_prev = tn;
-    s_prev = sn;
-    tc_m = tc_c; tc_c = tc_k1; sc_m = sc_cc; sc_cc = sc_k1;
-    tp_m = tp_c; tp_c = tp_k1; sp_m = sp_c; sp_c = sp_k1;
-    wm_c = wmk1; kh_c = khk1;
+    if (unstable) s_unstable[threadIdx.x] = 1;
+    __syncthreads();
+    unstable = part == 0 && s_unstable[threadIdx.x];
   }
-  if (lev > 1 && unstable) {
+  if (in && lev > 1 && unstable) {
     // convect reads prho one level below the adjusted range
     double t[PCOM_MAXK], s_[PCOM_MAXK], p1[PCOM_MAXK], p2[PCOM_MAXK];
     const int np = lev < nk ? lev + 1 : nk;
@@ -1282,6 +1378,32 @@ static inline size_t sm3(int nk, int planes) { return (size_t)planes * nk * TB_X
 // k_clin: four level planes (column-sum terms, new u and v) and the two sums
 static inline size_t clin_smem(int nk) { return sm3(nk, 4) + 2 * TB_X * sizeof(double); }
 
+// The column kernels' threads per column: 4 while the grid's columns are about
+// what the SMs hold at once (2^17: 148 SMs x 384 threads x 2.3), where the time
+// is that of one thread's levels; 1 beyond, where 4 prologues per column
+// cost more (int_readyc and int_ts, us, 4 against 1: 128 x 64 box 17 + 33
+// against 39 + 52, 360 x 160 66 + 143 against 78 + 155, 420 x 190 66 + 119 against
+// 73 + 131, 720 x 320 165 + 295 against 147 + 268, 1440 x 640 717 + 1491 against
+// 578 + 1296; the point-serial forms before: 58 + 63, 138 + 160, .., 1582 + 1672)
+constexpr int kParts = 4;
+static inline bool split_columns(int nx, int ny, int nz) { return (long long)nx * ny * nz <= 1 << 17; }
+template <bool BATCH>
+static void launch_readyc_col(const Dev &P, const Dev *Ps, int nx, int ny, int nk, int nz, cudaStream_t s) {
+  const int gx = (nx + kColX - 1) / kColX;
+  if (split_columns(nx, ny, nz))
+    k_readyc_col<BATCH, kParts><<<dim3(gx, ny, nz), dim3(kColX, 1, kParts), (size_t)2 * nk * kColX * sizeof(double), s>>>(P, Ps);
+  else
+    k_readyc_col<BATCH, 1><<<dim3(gx, (ny + 1) / 2, nz), dim3(kColX, 2), 0, s>>>(P, Ps);
+}
+template <bool BATCH>
+static void launch_ts_col(const Dev &P, const Dev *Ps, int nx, int ny, int nz, cudaStream_t s) {
+  const int gx = (nx + kColX - 1) / kColX;
+  if (split_columns(nx, ny, nz))
+    k_ts_col<BATCH, kParts><<<dim3(gx, ny, nz), dim3(kColX, 1, kParts), 0, s>>>(P, Ps);
+  else
+    k_ts_col<BATCH, 1><<<dim3(gx, (ny + 1) / 2, nz), dim3(kColX, 2), 0, s>>>(P, Ps);
+}
+
 template <typename R>
 void launch_alpha_tobot(const DevT<R> &P, cudaStream_t s) { k_alpha_tobot<R, false><<<g3(P.ni, wrows(P), 1), kBlock3, sm3(P.nk, 1), s>>>(P, nullptr); }
 template <typename R>
@@ -1299,7 +1421,7 @@ void launch_upwelling(const DevT<R> &P, int with_acw, cudaStream_t s) {
 template <typename R>
 void launch_readyc3d(const DevT<R> &P, cudaStream_t s) {
   if constexpr (std::is_same<R, double>::value)
-    k_readyc_col<false><<<dim3((P.glo_ni + kRcX - 1) / kRcX, (wrows(P) + kRcY - 1) / kRcY), dim3(kRcX, kRcY), 0, s>>>(P, nullptr);
+    launch_readyc_col<false>(P, nullptr, P.glo_ni, wrows(P), P.nk, 1, s);
   else
     k_readyc3d<R, false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, sm3(P.nk, 2), s>>>(P, nullptr);
 }
@@ -1323,7 +1445,7 @@ void launch_ssh(const DevT<R> &P, cudaStream_t s) { k_ssh<R, false><<<g3(P.ni, w
 template <typename R>
 void launch_ts(const DevT<R> &P, cudaStream_t s) {
   if constexpr (std::is_same<R, double>::value) {
-    k_ts_col<false><<<dim3((P.glo_ni + kColX - 1) / kColX, (wrows(P) + kColY - 1) / kColY), dim3(kColX, kColY), 0, s>>>(P, nullptr);
+    launch_ts_col<false>(P, nullptr, P.glo_ni, wrows(P), 1, s);
     k_ts_acc<false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, 0, s>>>(P, nullptr);
   } else {
     k_ts<R, false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, sm3(P.nk, 4), s>>>(P, nullptr);
@@ -1362,7 +1484,7 @@ void launch_batch(int kernel, const Dev *dPs, const BatchShape &b, int arg, cuda
     break;
   }
   case BK_READYC3D:
-    k_readyc_col<true><<<dim3((b.glo_ni + kRcX - 1) / kRcX, (b.nj + kRcY - 1) / kRcY, n), dim3(kRcX, kRcY), 0, s>>>(none, dPs);
+    launch_readyc_col<true>(none, dPs, b.glo_ni, b.nj, b.nk, n, s);
     break;
   case BK_CLIN: {
     static const cudaError_t attr = cudaFuncSetAttribute(k_clin<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1374,7 +1496,7 @@ void launch_batch(int kernel, const Dev *dPs, const BatchShape &b, int arg, cuda
   case BK_SMAG: k_smag<double, true><<<dim3((b.glo_ni + 31) / 32, (b.nj + 3) / 4, n), dim3(32, 4), 0, s>>>(none, dPs); break;
   case BK_SSH: k_ssh<double, true><<<g3(b.ni, b.nj, n), kBlock3, sm3(b.nk, 1), s>>>(none, dPs); break;
   case BK_TS:
-    k_ts_col<true><<<dim3((b.glo_ni + kColX - 1) / kColX, (b.nj + kColY - 1) / kColY, n), dim3(kColX, kColY), 0, s>>>(none, dPs);
+    launch_ts_col<true>(none, dPs, b.glo_ni, b.nj, n, s);
     k_ts_acc<true><<<g3(b.glo_ni, b.nj, n), kBlock3, 0, s>>>(none, dPs);
     break;
   case BK_DEN_PRHO: k_den_prho<double, true><<<g3(b.ni, b.nj, n), kBlock3, 0, s>>>(none, dPs); break;
