@@ -46,7 +46,10 @@ typedef struct pcom_model pcom_model;
 int pcom_model_create(const pcom_case *c, int32_t flags, pcom_model **out);
 int pcom_model_destroy(pcom_model *m);
 pcom_handle *pcom_model_handle(pcom_model *m);
-/* n passes of the time loop body (main.f90:158-238, without output()). */
+/* n passes of the time loop body (main.f90:158-238, without output()).  The
+ * steps are enqueued one behind the other and awaited before the call
+ * returns; a device-side failure (PCOM_ERR_TIMEOUT) is reported by the next
+ * wait, after the steps enqueued behind it. */
 int pcom_model_run(pcom_model *m, int64_t nsteps);
 /* One pass split open, for drivers that put their own work between the
  * subroutines of the step (the halo exchanges of a domain split into row

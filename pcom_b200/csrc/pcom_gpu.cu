@@ -446,13 +446,15 @@ unsigned long long message_space() {
 }
 
 int sync_check(pcom_handle *h) {
+  // the flags' copy is the wait for the stream (a copy to pageable memory
+  // returns when it is done): one round trip instead of two
+  int err[2] = {0, 0};
+  CK(cudaMemcpyAsync(err, h->D.err, sizeof err, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   if (h->side) CK(cudaStreamSynchronize(h->side));
   if (h->copy) CK(cudaStreamSynchronize(h->copy));
   if (h->copy_out) CK(cudaStreamSynchronize(h->copy_out));
   CK(cudaGetLastError());
-  int err[2] = {0, 0};
-  CK(cudaMemcpy(err, h->D.err, sizeof err, cudaMemcpyDeviceToHost));
   if (err[0]) {
     cudaMemsetAsync(h->D.err, 0, sizeof err, h->stream);
     cudaMemsetAsync(h->D.bar, 0, 2 * sizeof(unsigned), h->stream);

@@ -14,6 +14,8 @@
 
 #include "../../include/pcom_host.h"
 
+int pcom_set_error(int code, const char *msg);  // pcom_gpu.cu
+
 namespace {
 
 // default-REAL literal: REAL(4) rounding (gfortran) or REAL(8) (ifort -r8)
@@ -457,15 +459,26 @@ int pcom_model_end_step(pcom_model *M) {
 int pcom_model_run(pcom_model *M, int64_t nsteps) {
   if (!M) return PCOM_ERR_ARG;
   if (!M->h) return PCOM_ERR_STATE;
-  for (int64_t n = 0; n < nsteps; ++n) {
+  // the steps are enqueued without waiting and awaited once at the end (the
+  // daily calls wait too): a wait per step left the GPU idle for its round
+  // trip and for the next step's first launches.  A step that fails is
+  // reported by the wait that follows it
+  int rc = PCOM_OK;
+  for (int64_t n = 0; n < nsteps && !rc; ++n) {
     int64_t it = 0;
     int32_t day = 0;
-    int rc = pcom_model_begin_step(M, &it, &day);
-    if (!rc) rc = pcom_gpu_step(M->h, it);
-    if (rc) return rc;
-    pcom_model_end_step(M);
+    rc = pcom_model_begin_step(M, &it, &day);
+    if (!rc) rc = pcom_gpu_step_async(M->h, it);
+    if (!rc) pcom_model_end_step(M);
   }
-  return PCOM_OK;
+  if (nsteps <= 0) return rc;
+  if (rc) {  // keep the first failure's message
+    char msg[512] = {0};
+    pcom_gpu_last_error(msg, sizeof msg);
+    pcom_gpu_sync(M->h);
+    return pcom_set_error(rc, msg);
+  }
+  return pcom_gpu_sync(M->h);
 }
 
 int pcom_model_run_batch(pcom_model *const *ms, int32_t n, pcom_batch *b, int64_t nsteps) {
