@@ -700,6 +700,9 @@ int trop_res_max_blocks(int TX, int TY) {
 template <bool GROUP, int CTX, int CTY>
 constexpr int fast_threads() { return !GROUP && CTX > 0 && (CTX + 4) * (CTY + 4) <= 256 ? ((CTX + 4) * (CTY + 4) + 31) / 32 * 32 : kResThreads; }
 
+template <bool GROUP, int CTX, int CTY>
+__host__ __device__ constexpr bool fast_mreg() { return !GROUP && CTX > 0 && (CTX + 4) * (CTY + 4) <= 256; }
+
 template <bool GROUP, int CTX = 0, int CTY = 0>
 __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
     k_trop_fast(const __grid_constant__ Dev P0, const Dev *__restrict__ Ps, const TileRef *__restrict__ tiles,
@@ -769,8 +772,8 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
   }
   // (where sqrt(ter()) is not formed it is 1, 2 sqrt(ter()) = sqrt(4): land,
   // and points that need none)
-  const TropPoint T{fs + p, vx, vy, W, H, RS, lx, ly, inR, nrow, srow, inS2 && levu > 0 && nrow, inS6 && levu > 0 && nrow,
-                    levu > 0 && !nrow};
+  TropPoint<fast_mreg<GROUP, CTX, CTY>()> T{
+      fs + p, vx, vy, W, H, RS, lx, ly, inR, nrow, srow, inS2 && levu > 0 && nrow, inS6 && levu > 0 && nrow, levu > 0 && !nrow};
   double vs0u = 0.0, vs0v = 0.0;
   // accumulators (mod_int.f90:176-180)
   double acc_m = 0, acc_m2 = 0, acc_u = 0, acc_v = 0;
@@ -786,6 +789,7 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
   }
   if (inR) { T.S(X_CH, 0) = s.c0; T.S(X_UB, 0) = s.u0; T.S(X_VB, 0) = s.v0; }
   __syncthreads();
+  T.load_metrics();
 
   for (int nt = 1; nt <= nstep; ++nt) {
     ulonglong2 *const out = P.xch + (long long)(nt & 1) * 3 * P.n2 + q;  // this substep's words of this point

@@ -63,17 +63,34 @@ struct TropCoef {
   bool sea_u, sea_t;
 };
 
-// where a thread's point is, its fields and its metrics
+// where a thread's point is, its fields and its metrics.  MREG: the metrics
+// are kept in registers (27 pairs; tiles whose threads can have the
+// registers): from shared memory they were half of a small tile's loads (int_trop
+// of the 128 x 64 box 278 -> 272 us)
+template <bool MREG>
 struct TropPoint {
   double *f;              // &field[0][point]
-  const double *vx, *vy;  // [kXVecs][W], [kYVecs][H]
+  const double *vx, *vy;  // [kXVecs][W], [kYVecs][H] in shared memory
   int W, H, RS, lx, ly;
   bool inR;               // the thread has a point of the region
   bool nrow, srow;        // j <= njm, j >= 2
   bool s2sea, s6sea, s2zero;  // sqrt(ter()) of ch / of pred is formed; it is 0 (row nj)
+  double xr[MREG ? kXVecs : 1], yr[MREG ? kYVecs : 1], yn[MREG ? 2 : 1];
   PD double &S(int F, int o) const { return f[F * RS + o]; }
-  PD double X(int n) const { return vx[n * W + lx]; }
-  PD double Y(int n) const { return vy[n * H + ly]; }
+  PD double X(int n) const { return MREG ? xr[n] : vx[n * W + lx]; }
+  PD double Y(int n) const { return MREG ? yr[n] : vy[n * H + ly]; }
+  // vectors 14 and 15 of the next row
+  PD double Yn(int n) const { return MREG ? yn[n - 14] : vy[n * H + ly + 1]; }
+  PD void load_metrics() {
+    if constexpr (MREG) {
+      #pragma unroll
+      for (int n = 0; n < kXVecs; ++n) xr[n] = vx[n * W + lx];
+      #pragma unroll
+      for (int n = 0; n < kYVecs; ++n) yr[n] = vy[n * H + ly];
+      yn[0] = vy[14 * H + ly + 1];
+      yn[1] = vy[15 * H + ly + 1];
+    }
+  }
 };
 
 struct TropState {
@@ -86,7 +103,8 @@ struct TropState {
 
 // S2: sch = sqrt(ter(ch)) on U and the fluxes supb; the viscosity's
 // differences p1(ub)/rh4 on N and p2(ub) rh2 on E
-PD void trop_s2(const TropPoint &T, const TropCoef &K, TropState &s) {
+template <class Pt>
+PD void trop_s2(const Pt &T, const TropCoef &K, TropState &s) {
   const int W = T.W;
   const double w = s.c0 + T.S(X_CH, W) + T.S(X_CH, 1) + T.S(X_CH, W + 1);
   double sch = sqrt(T.s2sea ? w : 4.0);
@@ -113,7 +131,8 @@ PD void trop_s2(const TropPoint &T, const TropCoef &K, TropState &s) {
 
 // divergence of the staged fluxes (the ter U->E and U->N means formed here;
 // rows >= 2)
-PD double trop_div(const TropPoint &T, const TropState &s) {
+template <class Pt>
+PD double trop_div(const Pt &T, const TropState &s) {
   const int W = T.W;
   double A = dvr((T.S(X_S1, -W) + s.s1) - (T.S(X_S1, -W - 1) + T.S(X_S1, -1)), T.X(0), T.X(4));
   double B = dvr((T.S(X_X2, -1) + s.x2) - (T.S(X_X2, -W - 1) + T.S(X_X2, -W)), T.Y(0), T.Y(4));
@@ -123,7 +142,8 @@ PD double trop_div(const TropPoint &T, const TropState &s) {
 
 // S4: predictor ch (land_ch: ch on land); the viscosity's change since the
 // first substep (vs0u, vs0v; set where `first`)
-PD void trop_s4(const TropPoint &T, const TropCoef &K, TropState &s, double bt, double gamma_b, double land_ch, bool first,
+template <class Pt>
+PD void trop_s4(const Pt &T, const TropCoef &K, TropState &s, double bt, double gamma_b, double land_ch, bool first,
                 double &vs0u, double &vs0v) {
   const int W = T.W;
   const double div = trop_div(T, s);
@@ -143,7 +163,8 @@ PD void trop_s4(const TropPoint &T, const TropCoef &K, TropState &s, double bt, 
 // S6: sqrt(ter(pred)), the gradients and means of pred on E (rows j and
 // j + 1) and N (columns i and i + 1), all from the same four values, and the
 // corrector velocity (pressure gradient, Coriolis adjustment); its fluxes
-PD void trop_s6(const TropPoint &T, const TropCoef &K, TropState &s, double bt, double a, double ra) {
+template <class Pt>
+PD void trop_s6(const Pt &T, const TropCoef &K, TropState &s, double bt, double a, double ra) {
   const int W = T.W;
   const double pe = T.S(X_PRED, 1), pn = T.S(X_PRED, W), pne = T.S(X_PRED, W + 1), pred = s.pred;
   const double w = pred + pn + pe + pne;
@@ -151,7 +172,7 @@ PD void trop_s6(const TropPoint &T, const TropCoef &K, TropState &s, double bt, 
   if (T.s2zero) sch = 0.0;
   const double dx2 = T.X(1), rdx2 = T.X(5), dy4 = T.Y(3), rdy4 = T.Y(7);
   const double gx0 = dvr(dvr(pe - pred, dx2, rdx2), T.Y(14), T.Y(15));
-  const double gx1 = dvr(dvr(pne - pn, dx2, rdx2), T.vy[14 * T.H + T.ly + 1], T.vy[15 * T.H + T.ly + 1]);
+  const double gx1 = dvr(dvr(pne - pn, dx2, rdx2), T.Yn(14), T.Yn(15));
   const double gy0 = dvr(dvr(pn - pred, dy4, rdy4), a, ra), gy1 = dvr(dvr(pne - pe, dy4, rdy4), a, ra);
   double t1 = (gx0 * K.bxn + gx1 * K.bxs) + ((pred + pe) * K.gxn + (pn + pne) * K.gxs);
   double t2 = (gy0 * K.bye + gy1 * K.byw) + ((pred + pn) * K.gye + (pe + pne) * K.gyw);
@@ -175,6 +196,7 @@ PD void trop_s6(const TropPoint &T, const TropCoef &K, TropState &s, double bt, 
 }
 
 // S8: corrector ch
-PD double trop_s8(const TropPoint &T, const TropCoef &K, const TropState &s, double bt) {
+template <class Pt>
+PD double trop_s8(const Pt &T, const TropCoef &K, const TropState &s, double bt) {
   return s.c0 - dvr(trop_div(T, s) * (K.sea_t ? bt : 0.0), K.prh_t, K.rprh_t);
 }
