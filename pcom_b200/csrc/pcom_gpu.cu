@@ -348,7 +348,7 @@ struct pcom_handle {
   double *stage = nullptr;     // FP64 staging for host copies of FP32 fields
   bool ref_set = false;        // reference profile of the anomalies fixed
   double *d_sums = nullptr;    // global-sum partials and result
-  std::vector<int> lev_t_host;
+  std::vector<int> lev_t_host, lev_u_host;
   std::vector<void *> allocs;
   double *ab_u[3] = {}, *ab_v[3] = {};  // AB3 ring buffers: [ic], [ip], [ipp]
   int ic = 0, ip = 1, ipp = 2;
@@ -364,6 +364,7 @@ struct pcom_handle {
   // FP64: packed coefficients and the state between substeps
   unsigned char *ms_scratch = nullptr;
   MultiTrop ms{};
+  std::vector<int> ms_tiles;  // its tiles, those with sea first
   // mixed handles on the multi-tile path: FP32 coefficients and velocities
   unsigned char *mm_scratch = nullptr;
   MultiMixed mm{};
@@ -499,6 +500,27 @@ int apply_staged_forcing(pcom_handle *h) {
   return PCOM_OK;
 }
 
+// the tiles TX x TY of a domain, row by row, those with sea (a point with
+// lev_t >= 1 or lev_u >= 1) first; returns their number
+int sea_first(const pcom_handle *h, int TX, int TY, std::vector<int> &list) {
+  const int G = h->dims.glo_ni, nj = h->nj, ntx = (G + TX - 1) / TX, nty = (nj + TY - 1) / TY;
+  std::vector<int> land;
+  list.clear();
+  for (int t = 0; t < ntx * nty; ++t) {
+    bool sea = h->lev_t_host.empty();
+    const int r0 = t % ntx * TX, j0 = t / ntx * TY;
+    for (int j = j0; j < std::min(j0 + TY, nj) && !sea; ++j)
+      for (int r = r0; r < std::min(r0 + TX, G) && !sea; ++r) {
+        const size_t q = (size_t)j * h->ni + r + 1;
+        sea = h->lev_t_host[q] >= 1 || h->lev_u_host[q] >= 1;
+      }
+    (sea ? list : land).push_back(t);
+  }
+  const int n = (int)list.size();
+  list.insert(list.end(), land.begin(), land.end());
+  return n;
+}
+
 int pick_trop_config(pcom_handle *h) {
   // resident kernel: one tile per CTA, one region point per thread
   h->trop_resident = false;
@@ -549,24 +571,26 @@ int pick_trop_config(pcom_handle *h) {
     }
     if (!h->mixed) {
       // the compiled shape whose CTAs issue the fewest warps per substep
-      // (tiles per CTA x warps per tile)
+      // (tiles with sea per CTA x warps per tile)
       long long best = 1LL << 60;
-      int bx = 0, by = 0, bb = 0;
+      int bx = 0, by = 0, bb = 0, bw = 0;
+      std::vector<int> list;
 #define PCOM_TRY_SHAPE(x, y)                                                                        \
   {                                                                                                 \
-    const int n_ = ((G + (x) - 1) / (x)) * ((nj + (y) - 1) / (y));                                  \
-    const int mb_ = std::min(n_, trop_multi_max_blocks((x), (y)));                                  \
-    const long long c_ = mb_ > 0 ? (long long)((n_ + mb_ - 1) / mb_) * ((((x) + 4) * ((y) + 4) + 31) / 32) : best; \
-    if (c_ < best) { best = c_; bx = (x); by = (y); bb = mb_; }                                     \
+    const int w_ = sea_first(h, (x), (y), list), mb_ = std::max(1, std::min(w_, trop_multi_max_blocks((x), (y)))); \
+    const long long c_ = (long long)((w_ + mb_ - 1) / mb_) * ((((x) + 4) * ((y) + 4) + 31) / 32);   \
+    if (c_ < best) { best = c_; bx = (x); by = (y); bb = mb_; bw = w_; h->ms_tiles = list; }        \
   }
       PCOM_MULTI_SHAPES(PCOM_TRY_SHAPE)
 #undef PCOM_TRY_SHAPE
-      if (bx > 0) {
+      if (trop_multi_max_blocks(bx, by) > 0) {
         if (!h->ms_scratch) {
-          int rc = h->alloc(&h->ms_scratch, trop_multi_scratch_bytes(G, nj, bx, by));
+          int rc = h->alloc(&h->ms_scratch, trop_multi_scratch_bytes(G, nj));
           if (rc) return rc;
-          trop_multi_bind(h->ms, h->ms_scratch, G, nj, bx, by);
         }
+        trop_multi_bind(h->ms, h->ms_scratch, G, nj, bx, by);
+        h->ms.nwet = bw;
+        CK(cudaMemcpyAsync(h->ms.tiles, h->ms_tiles.data(), h->ms_tiles.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
         h->trop_multi = true;
         h->trop_tx = bx;
         h->trop_ty = by;
@@ -1317,6 +1341,7 @@ int pcom_gpu_upload_static(pcom_handle *h, const pcom_static *s) {
     CK(cudaMemcpy((void *)D.kh, s->kh, h->n3p * sizeof(double), cudaMemcpyHostToDevice));
   }
   h->lev_t_host.assign(s->lev_t, s->lev_t + n2);
+  h->lev_u_host.assign(s->lev_u, s->lev_u + n2);
   if (!s->pr2 || !s->dpr2 || !s->dz1) return fail(PCOM_ERR_ARG, "vertical grid missing");
   for (int k = 1; k <= nk; ++k) { D.pr2[k] = s->pr2[k - 1]; D.dpr2[k] = s->dpr2[k - 1]; D.rdpr2[k] = 1.0 / s->dpr2[k - 1]; }
   for (int k = 1; k <= nkp; ++k) { D.dz1[k] = s->dz1[k - 1]; D.rdz1[k] = 1.0 / s->dz1[k - 1]; }

@@ -94,8 +94,9 @@ struct MultiTrop {
   double2 *cf;                     // coefficient pairs, planes of [nj][pitch]
   double2 *st[2], *acc;            // state between substeps ([nj][pitch]), sums of ub, vb ([nj][ni])
   double *xm, *ym;                 // metric vectors of every tile column and row
+  int *tiles, nwet;                // tile numbers (row * columns + column): those with sea (nwet), those without
 };
-size_t trop_multi_scratch_bytes(int glo_ni, int nj, int TX, int TY);
+size_t trop_multi_scratch_bytes(int glo_ni, int nj);
 void trop_multi_bind(MultiTrop &M, void *scratch, int glo_ni, int nj, int TX, int TY);
 int trop_multi_max_blocks(int TX, int TY);
 cudaError_t launch_trop_multi(const Dev &P, const MultiTrop &M, int TX, int TY, int nblocks, unsigned long long *cnt,
