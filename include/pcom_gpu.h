@@ -304,7 +304,7 @@ int pcom_gpu_batch_sync(pcom_batch *b);
 int pcom_gpu_batch_den_prho(pcom_batch *b);
 /* Replay captured CUDA graphs (default on) or launch kernel by kernel. */
 int pcom_gpu_batch_use_graphs(pcom_batch *b, int32_t enable);
-/* Time candidate tile shapes of the batched barotropic kernel on the
+/* Time candidate tile sizes of the batched barotropic kernel on the
  * members' current state (which it saves and restores) and keep the fastest;
  * a one-line report of the trials goes to `report`. */
 int pcom_gpu_batch_autotune(pcom_batch *b, char *report, int32_t len);

@@ -408,6 +408,7 @@ enum {
 }  // namespace
 
 constexpr int kResThreads = 640;
+constexpr int kFreeSide = kResThreads / 5;  // longest side of a region (5 points and more the other way)
 
 __global__ void __launch_bounds__(kResThreads, 1)
     k_trop_res(const __grid_constant__ Dev P, int TX, int TY, int ntx) {
@@ -692,8 +693,14 @@ int trop_res_max_blocks(int TX, int TY) {
 //
 // CTX, CTY > 0: the same kernel compiled for one tile shape, so that the
 // region's row length and plane size are constants and every shared-memory
-// operand is a fixed offset from the thread's own point (fewer instructions
-// and registers per substep than the general form, CTX = CTY = 0).
+// operand is a fixed offset from the thread's own point.  CTX = CTY = 0: any
+// shape.  Its fields lie kResThreads apart and a point's metric vectors next
+// to each other, so that only the neighbouring rows' addresses depend on the
+// shape: a launch of 608-point tiles takes 0.46 ms either way.  The group
+// kernel is this form: every member of a batch has its own tile shape
+// (fit_tiles), which takes fewer launches than one shape for all (24 box
+// members and smaller basins: 1.75 ms in 4 launches of 16 x 12 tiles, the
+// best of 11 shapes, 1.38 ms in 3).
 // threads of a CTA: a fixed single-domain shape's own count, so that small
 // tiles get the registers that let a stage's chains overlap (a group packs
 // several small tiles on an SM)
@@ -707,17 +714,14 @@ template <bool GROUP, int CTX = 0, int CTY = 0>
 __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
     k_trop_fast(const __grid_constant__ Dev P0, const Dev *__restrict__ Ps, const TileRef *__restrict__ tiles,
                 int TX, int TY, int ntx, unsigned long long seq0, const unsigned long long *gseq, int *gerr) {
-  if (CTX > 0) { TX = CTX; TY = CTY; }
+  constexpr bool FREE = CTX == 0;
+  if (!FREE) { TX = CTX; TY = CTY; }
   extern __shared__ double sm[];
   const TileRef tile = GROUP ? tiles[blockIdx.x] : TileRef{0, 0, 0, 0, 0};
   const Dev &P = GROUP ? Ps[tile.m] : P0;
   const unsigned long long seq = GROUP ? *gseq : seq0;
   int *const err = GROUP ? gerr : P.err;
   const int ni = P.ni, nj = P.nj, njm = P.njm, G = P.glo_ni;
-  const int W = TX + 4, H = TY + 4, RS = W * H;
-  double *const fs = sm + x_pad(W);
-  double *vx = fs + X_COUNT * RS + x_pad(W) + 32;  // dxx[1..4], 1/dxx[1..4] over lx: 8*W
-  double *vy = vx + 8 * W;                         // 19 vectors over ly (see below)
   const double a = P.c.a, bt = (double)P.bt, gamma_b = P.c.gamma_b;
   const int nstep = P.nstep;
   const int tid = threadIdx.x;
@@ -731,16 +735,24 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
   }
   const int rr0 = R0 - 2, jj0 = J0 - 2;
   auto ring_i = [&](int r) { r %= G; if (r < 0) r += G; return r + 2; };
-
-  for (int l = tid; l < kXVecs * W; l += blockDim.x) vx[l] = trop_xvec(P, l / W, ring_i(rr0 + l % W));
-  for (int l = tid; l < kYVecs * H; l += blockDim.x) vy[l] = trop_yvec(P, l / H, min(max(jj0 + l % H, 1), nj));
+  // the region, and where its fields and metric vectors lie: a compiled
+  // shape's vectors one after the other; a free shape's by column and by row
+  // (rows of 9: the 16 lanes of a 64-bit access meet 32 banks)
+  const int W = (FREE ? tw : TX) + 4, H = (FREE ? th : TY) + 4, N = W * H;
+  const int RS = FREE ? kResThreads : N, pad = FREE ? x_pad(kFreeSide) : x_pad(W);
+  const int XS = FREE ? 1 : W, XC = FREE ? kXVecs + 1 : 1, YS = FREE ? 1 : H, YR = FREE ? kYVecs : 1;
+  double *const fs = sm + pad;
+  double *vx = fs + X_COUNT * RS + pad + 32, *vy = vx + (FREE ? XC : kXVecs) * W;
+  for (int l = tid; l < kXVecs * W; l += blockDim.x) vx[l / W * XS + l % W * XC] = trop_xvec(P, l / W, ring_i(rr0 + l % W));
+  for (int l = tid; l < kYVecs * H; l += blockDim.x)
+    vy[l / H * YS + l % H * YR] = trop_yvec(P, l / H, min(max(jj0 + l % H, 1), nj));
 
   const double ra = P.ra;
   // this thread's region point
   const int p = tid;
   const int ly = min(p / W, H - 1), lx = p - ly * W < W ? p - ly * W : 0;
   const int j = jj0 + ly;
-  const bool inR = p < RS;
+  const bool inR = p < N;
   const bool active = inR && j >= 1 && j <= nj;
   const int i = active ? ring_i(rr0 + lx) : 2;
   const long long q = active ? I2(P, i, j) : 0;
@@ -773,7 +785,7 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
   // (where sqrt(ter()) is not formed it is 1, 2 sqrt(ter()) = sqrt(4): land,
   // and points that need none)
   TropPoint<fast_mreg<GROUP, CTX, CTY>()> T{
-      fs + p, vx, vy, W, H, RS, lx, ly, inR, nrow, srow, inS2 && levu > 0 && nrow, inS6 && levu > 0 && nrow, levu > 0 && !nrow};
+      fs + p, vx + lx * XC, vy + ly * YR, W, RS, XS, YS, YR, inR, nrow, srow, inS2 && levu > 0 && nrow, inS6 && levu > 0 && nrow, levu > 0 && !nrow};
   double vs0u = 0.0, vs0v = 0.0;
   // accumulators (mod_int.f90:176-180)
   double acc_m = 0, acc_m2 = 0, acc_u = 0, acc_v = 0;
@@ -915,8 +927,22 @@ cudaError_t launch_trop_floor(const Dev &P, int TX, int TY, unsigned long long s
   return cudaLaunchCooperativeKernel((const void *)k_trop_floor, dim3(ntx * nty), dim3(nthreads), args, smem, s);
 }
 
+namespace {
+bool compiled_shape(int TX, int TY) {
+#define PCOM_FAST_SHAPE(x, y) \
+  if (TX == (x) && TY == (y)) return true;
+  PCOM_TROP_SHAPES(PCOM_FAST_SHAPE)
+#undef PCOM_FAST_SHAPE
+  return false;
+}
+// 9 W + 19 (H + 1) doubles of metric vectors are most for W = 5, H = 128
+constexpr size_t kFreeSmem =
+    ((size_t)X_COUNT * kResThreads + 2 * x_pad(kFreeSide) + 32 + (kXVecs + 1) * 5 + kYVecs * (kFreeSide + 1)) * sizeof(double);
+}  // namespace
+
 size_t trop_fast_smem_bytes(int TX, int TY) {
   const int W = TX + 4, H = TY + 4;
+  if (!compiled_shape(TX, TY)) return kFreeSmem;
   return ((size_t)X_COUNT * W * H + 2 * x_pad(W) + 32 + 8 * W + 19 * H + 1) * sizeof(double);  // (+ 1: row ly + 1 of the last vector)
 }
 
@@ -929,18 +955,6 @@ const void *fast_kernel(int TX, int TY) {
   PCOM_TROP_SHAPES(PCOM_FAST_SHAPE)
 #undef PCOM_FAST_SHAPE
   return (const void *)k_trop_fast<false>;
-}
-// the group kernel for a tile shape: a fixed-shape form for each tile shape
-// the batch autotuner tries (pcom_gpu_batch_autotune), the general one
-// otherwise
-const void *group_kernel(int TX, int TY) {
-#define PCOM_GROUP_SHAPE(x, y) \
-  if (TX == (x) && TY == (y)) return (const void *)k_trop_fast<true, (x), (y)>;
-  PCOM_GROUP_SHAPE(12, 12) PCOM_GROUP_SHAPE(16, 8) PCOM_GROUP_SHAPE(16, 12) PCOM_GROUP_SHAPE(16, 16)
-  PCOM_GROUP_SHAPE(24, 12) PCOM_GROUP_SHAPE(20, 16) PCOM_GROUP_SHAPE(24, 18) PCOM_GROUP_SHAPE(32, 8)
-  PCOM_GROUP_SHAPE(32, 12) PCOM_GROUP_SHAPE(28, 16) PCOM_GROUP_SHAPE(48, 8) PCOM_GROUP_SHAPE(64, 6)
-#undef PCOM_GROUP_SHAPE
-  return (const void *)k_trop_fast<true>;
 }
 }  // namespace
 
@@ -961,43 +975,41 @@ cudaError_t launch_trop_fast(const Dev &P, int TX, int TY, unsigned long long se
 }
 
 namespace {
-template <bool GROUP>
-int fast_max_blocks(int TX, int TY) {
+int resident_blocks(const void *fn, int nthreads, size_t smem) {
   int dev = 0, nsm = 0, per = 0;
-  if ((TX + 4) * (TY + 4) > kResThreads) return 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = trop_fast_smem_bytes(TX, TY);
-  const void *fn = GROUP ? group_kernel(TX, TY) : fast_kernel(TX, TY);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-  const int nthreads = ((TX + 4) * (TY + 4) + 31) / 32 * 32;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, nthreads, smem) != cudaSuccess) return 0;
   return per * nsm;
 }
 }  // namespace
 
-int trop_fast_max_blocks(int TX, int TY) { return fast_max_blocks<false>(TX, TY); }
-int trop_group_max_blocks(int TX, int TY) { return fast_max_blocks<true>(TX, TY); }
+int trop_fast_max_blocks(int TX, int TY) {
+  if (!trop_res_fits(TX, TY)) return 0;
+  return resident_blocks(fast_kernel(TX, TY), ((TX + 4) * (TY + 4) + 31) / 32 * 32, trop_fast_smem_bytes(TX, TY));
+}
+int trop_group_max_blocks(int nthreads) {
+  return nthreads > kResThreads ? 0 : resident_blocks((const void *)k_trop_fast<true>, nthreads, kFreeSmem);
+}
 
 namespace {
 __global__ void k_advance(unsigned long long *cnt, int n) { *cnt += (unsigned long long)n; }
 }  // namespace
 
-cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nstep,
+cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int nthreads, int nstep,
                               unsigned long long *cnt, int *err, cudaStream_t s) {
-  const size_t smem = trop_fast_smem_bytes(TX, TY);
-  const void *fn = group_kernel(TX, TY);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const void *fn = (const void *)k_trop_fast<true>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFreeSmem);
   if (e != cudaSuccess) return e;
   // sequence numbers no message of an earlier launch carries (the launch may
   // be a node of a graph that is replayed, so they come from device memory)
   k_advance<<<1, 1, 0, s>>>(cnt, nstep);
-  const int nthreads = ((TX + 4) * (TY + 4) + 31) / 32 * 32;
   Dev none{};
-  const int ntx = 0;
+  const int TX = 0, TY = 0, ntx = 0;
   const unsigned long long seq = 0;
   const unsigned long long *ccnt = cnt;
   void *args[] = {(void *)&none, (void *)&dPs, (void *)&dtiles, (void *)&TX, (void *)&TY, (void *)&ntx, (void *)&seq,
                   (void *)&ccnt, (void *)&err};
-  return cudaLaunchCooperativeKernel(fn, dim3(ntiles), dim3(nthreads), args, smem, s);
+  return cudaLaunchCooperativeKernel(fn, dim3(ntiles), dim3(nthreads), args, kFreeSmem, s);
 }

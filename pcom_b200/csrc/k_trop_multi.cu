@@ -246,7 +246,7 @@ __global__ void __launch_bounds__((ms_threads<TX, TY>()), 1)
       const int fl = active ? (int)flag : 0;
       K.sea_u = fl & 1;
       K.sea_t = fl & 2;
-      const TropPoint<false> T{fs + p, vec + b * NV, vec + b * NV + kXVecs * W, W, H, RS, lx, ly, inR, nrow, j >= 2,
+      const TropPoint<false> T{fs + p, vec + b * NV + lx, vec + b * NV + kXVecs * W + ly, W, RS, W, H, 1, inR, nrow, j >= 2,
                                inS2 && K.sea_u && nrow, inS6 && K.sea_u && nrow, K.sea_u && !nrow};
       if (inR) { T.S(X_CH, 0) = s.c0; T.S(X_UB, 0) = s.u0; T.S(X_VB, 0) = s.v0; }
       if (__syncthreads_or(!ok)) {

@@ -1860,11 +1860,11 @@ struct pcom_batch {
   // to be resident go to one group of the multi-tile kernel
   struct TropGroup {
     TileRef *d;
-    int ntiles, nblocks;
+    int ntiles, nblocks, nthreads;
     bool resident;
   };
   std::vector<TropGroup> groups;
-  int TX = 24, TY = 18;
+  int TX = 24, TY = 18;  // tiles of the multi-tile kernel
   int max_resident = 0;  // > 0: cap on the tiles of one resident group
   int64_t launches = 0;  // kernels this batch launched
   // [0] barrier arrivals of the multi-tile kernel, [1] sequence base of the
@@ -1896,9 +1896,73 @@ void member_tiles(const pcom_handle *h, int m, int TX, int TY, std::vector<TileR
     for (int r0 = 0; r0 < G; r0 += TX) t.push_back({m, r0, j0, std::min(TX, G - r0), std::min(TY, nj - j0 + 1)});
 }
 
-// plan the barotropic launches for tile shape TX x TY: first-fit decreasing
-// packing of the members' tile lists into groups of at most `cap` tiles
-int batch_tiles(pcom_batch *b, int TX, int TY) {
+// a member's own tile shape: the fewest tiles whose regions have at most
+// `points` points, then the smallest
+void fit_tiles(const pcom_handle *h, int points, int &TX, int &TY) {
+  const int G = h->dims.glo_ni, nj = h->nj;
+  long long best = 1LL << 60;
+  for (int ny = 1; ny <= nj; ++ny) {
+    const int y = (nj + ny - 1) / ny, most = std::min(G, points / (y + 4) - 4);
+    if (most < std::min(G, 4)) continue;
+    if (y < std::min(nj, 4)) break;
+    const int nx = (G + most - 1) / most, x = (G + nx - 1) / nx;
+    const long long c = ((long long)nx * ((nj + y - 1) / y) << 16) + (x + 4) * (y + 4);
+    if (c < best) { best = c; TX = x; TY = y; }
+  }
+}
+
+// the barotropic launches of a batch: every member's tiles, of one shape or
+// (points > 0) of the member's own, packed first-fit decreasing into groups
+// of co-resident tiles
+struct BatchPlan {
+  std::vector<std::vector<TileRef>> res;  // resident groups
+  std::vector<TileRef> big;               // members that cannot be resident
+  int nthreads = 0;                       // a CTA of a resident group
+  double cost = 0.0;                      // modelled microseconds of a substep of the resident groups
+};
+BatchPlan batch_plan(const pcom_batch *b, int TX, int TY, int points) {
+  BatchPlan p;
+  const int n = (int)b->hs.size();
+  std::vector<std::vector<TileRef>> mt(n);
+  int most = 0;
+  for (int m = 0; m < n; ++m) {
+    int x = TX, y = TY;
+    if (points > 0) fit_tiles(b->hs[m], points, x, y);
+    member_tiles(b->hs[m], m, x, y, mt[m]);
+    most = std::max(most, (std::min(x, b->hs[m]->dims.glo_ni) + 4) * (std::min(y, b->hs[m]->nj) + 4));
+  }
+  p.nthreads = (most + 31) / 32 * 32;
+  int cap = trop_group_max_blocks(p.nthreads);
+  if (b->max_resident > 0) cap = std::min(cap, b->max_resident);
+  std::vector<int> order(n);
+  for (int m = 0; m < n; ++m) order[m] = m;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return mt[x].size() > mt[y].size(); });
+  for (int m : order) {
+    const int nt = (int)mt[m].size();
+    if (nt > cap || !b->hs[m]->D.xch) {
+      member_tiles(b->hs[m], m, TX, TY, p.big);
+      continue;
+    }
+    bool placed = false;
+    for (auto &g : p.res)
+      if ((int)(g.size() + nt) <= cap) {
+        g.insert(g.end(), mt[m].begin(), mt[m].end());
+        placed = true;
+        break;
+      }
+    if (!placed) p.res.push_back(mt[m]);
+  }
+  // a substep of a group: the messages' way and the stages' latency, and
+  // every warp's instructions (5 warps on an SM took 2.2 us, 20 took 3.95)
+  int nsm = 1;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->hs[0]->device);
+  for (auto &g : p.res) p.cost += 1.62 + 0.117 * (((int)g.size() + nsm - 1) / nsm * (p.nthreads / 32));
+  return p;
+}
+
+// plan the barotropic launches for tile shape TX x TY, or for the members'
+// own shapes of at most `points` points
+int batch_tiles(pcom_batch *b, int TX, int TY, int points) {
   for (pcom_batch::TropGroup &g : b->groups) {
     cudaFree(g.d);
     b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void *)g.d));
@@ -1906,33 +1970,9 @@ int batch_tiles(pcom_batch *b, int TX, int TY) {
   b->groups.clear();
   for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
   b->graphs.clear();
-  int cap = trop_group_max_blocks(TX, TY);
-  if (b->max_resident > 0) cap = std::min(cap, b->max_resident);
-  const int n = (int)b->hs.size();
-  std::vector<std::vector<TileRef>> mt(n);
-  for (int m = 0; m < n; ++m) member_tiles(b->hs[m], m, TX, TY, mt[m]);
-  std::vector<int> order(n);
-  for (int m = 0; m < n; ++m) order[m] = m;
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return mt[x].size() > mt[y].size(); });
-  std::vector<std::vector<TileRef>> res;  // resident groups
-  std::vector<TileRef> big;               // members that cannot be resident
-  for (int m : order) {
-    const int nt = (int)mt[m].size();
-    if (nt > cap || !b->hs[m]->D.xch) {
-      big.insert(big.end(), mt[m].begin(), mt[m].end());
-      continue;
-    }
-    bool placed = false;
-    for (auto &g : res)
-      if ((int)(g.size() + nt) <= cap) {
-        g.insert(g.end(), mt[m].begin(), mt[m].end());
-        placed = true;
-        break;
-      }
-    if (!placed) res.push_back(mt[m]);
-  }
+  const BatchPlan p = batch_plan(b, TX, TY, points);
   auto add = [&](const std::vector<TileRef> &t, bool resident) -> int {
-    pcom_batch::TropGroup g{nullptr, (int)t.size(), 0, resident};
+    pcom_batch::TropGroup g{nullptr, (int)t.size(), 0, p.nthreads, resident};
     CK(cudaMalloc(&g.d, t.size() * sizeof(TileRef)));
     b->allocs.push_back(g.d);
     CK(cudaMemcpy(g.d, t.data(), t.size() * sizeof(TileRef), cudaMemcpyHostToDevice));
@@ -1946,12 +1986,12 @@ int batch_tiles(pcom_batch *b, int TX, int TY) {
     b->groups.push_back(g);
     return PCOM_OK;
   };
-  for (auto &g : res) {
+  for (auto &g : p.res) {
     int rc = add(g, true);
     if (rc) return rc;
   }
-  if (!big.empty()) {
-    int rc = add(big, false);
+  if (!p.big.empty()) {
+    int rc = add(p.big, false);
     if (rc) return rc;
   }
   b->TX = TX;
@@ -1959,10 +1999,22 @@ int batch_tiles(pcom_batch *b, int TX, int TY) {
   return PCOM_OK;
 }
 
+// the tile sizes a batch may take (points of a region), the cheapest by the
+// model first (24 box members and basins: 608 points modelled 1.39 ms, 1.38
+// measured; 640: 1.42, 1.42; 320, two tiles on an SM: 1.76, 1.70)
+std::vector<int> batch_sizes(const pcom_batch *b) {
+  std::vector<std::pair<double, int>> v;
+  for (int points = 640; points >= 128; points -= 32) v.push_back({batch_plan(b, 24, 18, points).cost, points});
+  std::stable_sort(v.begin(), v.end(), [](const auto &x, const auto &y) { return x.first < y.first; });
+  std::vector<int> s;
+  for (auto &c : v) s.push_back(c.second);
+  return s;
+}
+
 // the barotropic subcycles of all members
 cudaError_t batch_trop(pcom_batch *b, const Dev *dP) {
   for (const pcom_batch::TropGroup &g : b->groups) {
-    cudaError_t e = g.resident ? launch_trop_group(dP, g.d, g.ntiles, b->TX, b->TY, b->nstep, b->cnt + 1, b->err, b->stream)
+    cudaError_t e = g.resident ? launch_trop_group(dP, g.d, g.ntiles, g.nthreads, b->nstep, b->cnt + 1, b->err, b->stream)
                                : launch_trop_batch(dP, g.d, g.ntiles, b->TX, b->TY, g.nblocks, b->cnt, b->err, b->stream);
     if (e != cudaSuccess) return e;
   }
@@ -2078,7 +2130,7 @@ int pcom_gpu_batch_create(pcom_handle *const *hs, int32_t n, pcom_batch **out) {
   const unsigned long long cnt0[2] = {0, message_space()};
   if (e == cudaSuccess) e = cudaMemcpy(b->cnt, cnt0, sizeof cnt0, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) { delete b; return fail(PCOM_ERR_CUDA, "batch scratch: %s", cudaGetErrorString(e)); }
-  int rc = batch_tiles(b, 24, 18);
+  int rc = batch_tiles(b, 24, 18, batch_sizes(b)[0]);
   if (rc) { delete b; return rc; }
   *out = b;
   return PCOM_OK;
@@ -2184,7 +2236,7 @@ int pcom_gpu_batch_set_tiles(pcom_batch *b, int32_t tx, int32_t ty, int32_t max_
     return fail(PCOM_ERR_ARG, "tile %dx%d: need tx, ty >= 1 and (tx+4)*(ty+4) <= 640", tx, ty);
   CK(cudaStreamSynchronize(b->stream));
   b->max_resident = max_resident > 0 ? max_resident : 0;
-  return batch_tiles(b, tx, ty);
+  return batch_tiles(b, tx, ty, 0);
 }
 
 int64_t pcom_gpu_batch_launch_count(pcom_batch *b) { return b ? b->launches : 0; }
@@ -2201,14 +2253,14 @@ int pcom_gpu_batch_step(pcom_batch *b, int64_t tctr_i) {
 }
 
 // Autotuner: time the barotropic launches of the whole batch for candidate
-// tile shapes on the members' current state (the 2-D fields they change are
+// tile sizes on the members' current state (the 2-D fields they change are
 // saved and restored around every trial) and keep the fastest.  The choice
 // is cached per set of member grid sizes, so later batches of the same
 // shapes skip the trials.
 int pcom_gpu_batch_autotune(pcom_batch *b, char *report, int32_t len) {
   if (!b) return fail(PCOM_ERR_ARG, "null batch");
   static std::mutex cache_mu;
-  static std::map<std::string, std::pair<int, int>> cache;
+  static std::map<std::string, int> cache;  // points of a region
   std::vector<std::string> dims;
   for (pcom_handle *h : b->hs) dims.push_back(std::to_string(h->dims.glo_ni) + "x" + std::to_string(h->dims.glo_nj));
   std::sort(dims.begin(), dims.end());
@@ -2218,15 +2270,16 @@ int pcom_gpu_batch_autotune(pcom_batch *b, char *report, int32_t len) {
     std::lock_guard<std::mutex> lk(cache_mu);
     auto it = cache.find(sig);
     if (it != cache.end()) {
-      int rc = batch_tiles(b, it->second.first, it->second.second);
+      int rc = batch_tiles(b, 24, 18, it->second);
       if (rc) return rc;
-      std::string rep = "cached -> " + std::to_string(b->TX) + "x" + std::to_string(b->TY);
+      std::string rep = "cached -> " + std::to_string(it->second) + " points";
       if (report && len > 0) { strncpy(report, rep.c_str(), (size_t)len - 1); report[len - 1] = 0; }
       return PCOM_OK;
     }
   }
-  static const int cand[][2] = {{12, 12}, {16, 8},  {16, 12}, {16, 16}, {24, 12}, {20, 16},
-                                {24, 18}, {32, 8},  {32, 12}, {28, 16}, {48, 8},  {64, 6}};
+  // the sizes the model finds cheapest (it is within some percent)
+  std::vector<int> cand = batch_sizes(b);
+  cand.resize(6);
   for (cudaStream_t s : b->member_streams) CK(cudaStreamSynchronize(s));
   CK(cudaStreamSynchronize(b->stream));
   // save the 2-D fields the subcycle writes
@@ -2252,15 +2305,14 @@ int pcom_gpu_batch_autotune(pcom_batch *b, char *report, int32_t len) {
   Dev *dP = nullptr;
   if (!rc) rc = batch_dev_array(b, phase_key(b->hs[0]), &dP);
   double best = 1e30;
-  int bx = b->TX, by = b->TY;
+  int points = cand[0];
   std::string rep;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  for (auto &c : cand) {
+  for (int c : cand) {
     if (rc) break;
-    if (trop_group_max_blocks(c[0], c[1]) <= 0) continue;
-    rc = batch_tiles(b, c[0], c[1]);
+    rc = batch_tiles(b, 24, 18, c);
     if (rc) break;
     float ms = 0.f, tot = 0.f;
     for (int rep_i = 0; rep_i < 3 && !rc; ++rep_i) {
@@ -2277,23 +2329,23 @@ int pcom_gpu_batch_autotune(pcom_batch *b, char *report, int32_t len) {
     int res = 0, tiles = 0;
     for (auto &g : b->groups) { res += g.resident; tiles += g.ntiles; }
     char line[128];
-    snprintf(line, sizeof line, "%dx%d:%.3fms(%d tiles,%d launches,%d resident) ", c[0], c[1], t, tiles,
+    snprintf(line, sizeof line, "%d points:%.3fms(%d tiles,%d launches,%d resident) ", c, t, tiles,
              (int)b->groups.size(), res);
     rep += line;
-    if (!rc && t < best) { best = t; bx = c[0]; by = c[1]; }
+    if (!rc && t < best) { best = t; points = c; }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   for (double *c : saved) cudaFree(c);
   if (rc) return rc;
-  rc = batch_tiles(b, bx, by);
+  rc = batch_tiles(b, 24, 18, points);
   if (rc) return rc;
   {
     std::lock_guard<std::mutex> lk(cache_mu);
-    cache[sig] = {bx, by};
+    cache[sig] = points;
   }
   char line[96];
-  snprintf(line, sizeof line, "-> %dx%d", bx, by);
+  snprintf(line, sizeof line, "-> %d points", points);
   rep += line;
   if (report && len > 0) { strncpy(report, rep.c_str(), (size_t)len - 1); report[len - 1] = 0; }
   return PCOM_OK;

@@ -104,8 +104,8 @@ cudaError_t launch_trop_multi(const Dev &P, const MultiTrop &M, int TX, int TY, 
 // resident form: one tile per CTA, coefficients in registers (the fast
 // kernel over a tile list); all tiles of the group must be co-resident.  *cnt
 // is the sequence base, advanced by nstep before the launch
-int trop_group_max_blocks(int TX, int TY);
-cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nstep,
+int trop_group_max_blocks(int nthreads);
+cudaError_t launch_trop_group(const Dev *dPs, const TileRef *dtiles, int ntiles, int nthreads, int nstep,
                               unsigned long long *cnt, int *err, cudaStream_t s);
 
 // the model constants (literal precision per PCOM_LIT_R8)

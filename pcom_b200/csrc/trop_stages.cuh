@@ -70,25 +70,26 @@ struct TropCoef {
 template <bool MREG>
 struct TropPoint {
   double *f;              // &field[0][point]
-  const double *vx, *vy;  // [kXVecs][W], [kYVecs][H] in shared memory
-  int W, H, RS, lx, ly;
+  const double *vx, *vy;  // this column's and this row's metrics in shared memory
+  int W, RS;              // row length of the region, size of a field
+  int XS, YS, YR;         // from one column vector to the next, one row vector to the next, one row to the next
   bool inR;               // the thread has a point of the region
   bool nrow, srow;        // j <= njm, j >= 2
   bool s2sea, s6sea, s2zero;  // sqrt(ter()) of ch / of pred is formed; it is 0 (row nj)
   double xr[MREG ? kXVecs : 1], yr[MREG ? kYVecs : 1], yn[MREG ? 2 : 1];
   PD double &S(int F, int o) const { return f[F * RS + o]; }
-  PD double X(int n) const { return MREG ? xr[n] : vx[n * W + lx]; }
-  PD double Y(int n) const { return MREG ? yr[n] : vy[n * H + ly]; }
+  PD double X(int n) const { return MREG ? xr[n] : vx[n * XS]; }
+  PD double Y(int n) const { return MREG ? yr[n] : vy[n * YS]; }
   // vectors 14 and 15 of the next row
-  PD double Yn(int n) const { return MREG ? yn[n - 14] : vy[n * H + ly + 1]; }
+  PD double Yn(int n) const { return MREG ? yn[n - 14] : vy[n * YS + YR]; }
   PD void load_metrics() {
     if constexpr (MREG) {
       #pragma unroll
-      for (int n = 0; n < kXVecs; ++n) xr[n] = vx[n * W + lx];
+      for (int n = 0; n < kXVecs; ++n) xr[n] = vx[n * XS];
       #pragma unroll
-      for (int n = 0; n < kYVecs; ++n) yr[n] = vy[n * H + ly];
-      yn[0] = vy[14 * H + ly + 1];
-      yn[1] = vy[15 * H + ly + 1];
+      for (int n = 0; n < kYVecs; ++n) yr[n] = vy[n * YS];
+      yn[0] = vy[14 * YS + YR];
+      yn[1] = vy[15 * YS + YR];
     }
   }
 };

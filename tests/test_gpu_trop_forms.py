@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from pcom_b200 import _lib as L
-from pcom_b200.model import Model
+from pcom_b200.model import Batch, Model
 from pcom_b200.synth import make_case
 from parity_util import STATE_FIELDS, compare
 
@@ -50,3 +50,24 @@ def test_forms_agree_bit_for_bit(size, land):
         for f in STATE_FIELDS:
             r = compare(got[form][f], got[3][f])
             assert r["unequal"] == 0, f"form {form}, {f}: {r['unequal']} values differ"
+
+
+@pytest.mark.parametrize("sizes", [[(10, 8), (13, 9), (37, 23)], [(211, 97), (12, 90), (150, 9)], [(128, 66)] * 5],
+                         ids=["small", "long", "several launches"])
+def test_batch_of_fitted_tiles(sizes):
+    """A batch gives each member tiles of its own shape, packed into launches."""
+    cases = [_case(ni, nj, 3, "band") for ni, nj in sizes]
+    ms = [Model(c) for c in cases]
+    b = Batch(ms)
+    b.run(4)
+    for c, m in zip(cases, ms):
+        r = Model(c)
+        L.check(r.lib.pcom_gpu_set_trop_kernel(r.handle, 3), "set_trop_kernel")
+        r.run(4)
+        for f in STATE_FIELDS:
+            d = compare(m.field(f), r.field(f))
+            assert d["unequal"] == 0, f"{c['itn'].shape}, {f}: {d['unequal']} values differ"
+        r.close()
+    b.close()
+    for m in ms:
+        m.close()
