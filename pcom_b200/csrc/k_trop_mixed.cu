@@ -20,7 +20,7 @@
 
 namespace {
 
-constexpr int kThreads = 640;
+constexpr int kThreads = 640, kSide = kThreads / 5;  // threads; longest side of a region
 
 enum { D_CH, D_PRED, D_COUNT };                                         // FP64 region fields
 enum { F_UB, F_VB, F_S1, F_X2, F_A1U, F_A1V, F_A2U, F_A2V, F_COUNT };  // FP32 region fields
@@ -40,19 +40,16 @@ __device__ __forceinline__ void unpack_uv(double w, float &u, float &v) {
 
 }  // namespace
 
-// CTX, CTY > 0: compiled for one tile shape (constant region strides, as in
-// k_trop_fast); CTX = CTY = 0: any shape
+// CTX, CTY > 0: compiled for one tile shape (constant region strides);
+// CTX = CTY = 0: any shape, laid out as in k_trop_fast (19 warps in rows of 32
+// points for 360 x 162: 339 -> 323 us; 211 x 99: 248 -> 233)
 template <int CTX = 0, int CTY = 0>
 __global__ void __launch_bounds__(kThreads, 1)
     k_trop_mixed(const __grid_constant__ Dev P, int TX, int TY, int ntx, unsigned long long seq) {
-  if (CTX > 0) { TX = CTX; TY = CTY; }
+  constexpr bool FREE = CTX == 0;
+  if (!FREE) { TX = CTX; TY = CTY; }
   extern __shared__ double smd[];
   const int nj = P.nj, njm = P.njm, ni = P.ni, G = P.glo_ni;
-  const int W = TX + 4, H = TY + 4, RS = W * H;
-  double *const ds = smd + pad(W);
-  float *const fs = reinterpret_cast<float *>(ds + D_COUNT * RS + pad(W) + 32) + pad(W);
-  float *vx = fs + F_COUNT * RS + pad(W) + 32;
-  float *vy = vx + kVx * W;
   const float ra = (float)P.ra, bt = (float)P.bt, gamma_b = (float)P.c.gamma_b;
   const int nstep = P.nstep;
   const int tid = threadIdx.x;
@@ -62,33 +59,41 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int rr0 = R0 - 2, jj0 = J0 - 2;
   auto ring_i = [&](int r) { r %= G; if (r < 0) r += G; return r + 2; };
 
+  // (the layout of k_trop_fast)
+  const int W = (FREE ? tw : TX) + 4, H = (FREE ? th : TY) + 4, N = W * H;
+  const int RS = FREE ? kThreads : N, margin = FREE ? pad(kSide) : pad(W);
+  const int XS = FREE ? 1 : W, XC = FREE ? kVx + 1 : 1, YS = FREE ? 1 : H, YR = FREE ? kVy : 1;
+  double *const ds = smd + margin;
+  float *const fs = reinterpret_cast<float *>(ds + D_COUNT * RS + margin + 32) + margin;
+  float *vx = fs + F_COUNT * RS + margin + 32, *vy = vx + (FREE ? XC : kVx) * W;
   for (int l = tid; l < W; l += blockDim.x) {
     const int i = ring_i(rr0 + l);
     for (int g = 1; g <= 4; ++g) {
-      vx[(g - 1) * W + l] = (float)ld(P.dxx1d[g], i - 1);
-      vx[(4 + g - 1) * W + l] = (float)ld(P.rdxx1d[g], i - 1);
+      vx[l * XC + (g - 1) * XS] = (float)ld(P.dxx1d[g], i - 1);
+      vx[l * XC + (4 + g - 1) * XS] = (float)ld(P.rdxx1d[g], i - 1);
     }
   }
   for (int l = tid; l < H; l += blockDim.x) {
     const int j = min(max(jj0 + l, 1), nj);
+    float *const v = vy + l * YR;
     for (int g = 1; g <= 4; ++g) {
-      vy[(g - 1) * H + l] = (float)ld(P.dxy1d[g], j - 1);
-      vy[(4 + g - 1) * H + l] = (float)ld(P.rdxy1d[g], j - 1);
-      vy[(8 + g - 1) * H + l] = (float)ld(P.rh1d[g], j - 1);
+      v[(g - 1) * YS] = (float)ld(P.dxy1d[g], j - 1);
+      v[(4 + g - 1) * YS] = (float)ld(P.rdxy1d[g], j - 1);
+      v[(8 + g - 1) * YS] = (float)ld(P.rh1d[g], j - 1);
     }
-    vy[12 * H + l] = (float)ld(P.arh1d[1], j - 1);
-    vy[13 * H + l] = (float)ld(P.rarh1d[1], j - 1);
-    vy[14 * H + l] = (float)ld(P.arh1d[2], j - 1);
-    vy[15 * H + l] = (float)ld(P.rarh1d[2], j - 1);
-    vy[16 * H + l] = (float)ld(P.rrh1d[4], j - 1);
-    vy[17 * H + l] = (float)ld(P.aarh3, j - 1);
-    vy[18 * H + l] = (float)ld(P.raarh3, j - 1);
+    v[12 * YS] = (float)ld(P.arh1d[1], j - 1);
+    v[13 * YS] = (float)ld(P.rarh1d[1], j - 1);
+    v[14 * YS] = (float)ld(P.arh1d[2], j - 1);
+    v[15 * YS] = (float)ld(P.rarh1d[2], j - 1);
+    v[16 * YS] = (float)ld(P.rrh1d[4], j - 1);
+    v[17 * YS] = (float)ld(P.aarh3, j - 1);
+    v[18 * YS] = (float)ld(P.raarh3, j - 1);
   }
 
   const int p = tid;
   const int ly = min(p / W, H - 1), lx = p - ly * W < W ? p - ly * W : 0;
   const int j = jj0 + ly;
-  const bool inR = p < RS;
+  const bool inR = p < N;
   const bool active = inR && j >= 1 && j <= nj;
   const int i = active ? ring_i(rr0 + lx) : 2;
   const long long q = active ? I2(P, i, j) : 0;
@@ -134,9 +139,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   float *const ff = fs + p;
 #define SD(F, o) fd[(F) * RS + (o)]
 #define SF(F, o) ff[(F) * RS + (o)]
-#define RDXX(g) vx[(4 + (g) - 1) * W + lx]
-#define RDXY(g) vy[(4 + (g) - 1) * H + ly]
-#define RH(g) vy[(8 + (g) - 1) * H + ly]
+  vx += lx * XC;
+  vy += ly * YR;
+#define RDXX(g) vx[(4 + (g) - 1) * XS]
+#define RDXY(g) vy[(4 + (g) - 1) * YS]
+#define RH(g) vy[(8 + (g) - 1) * YS]
   if (inR) { SD(D_CH, 0) = c0; SF(F_UB, 0) = u0; SF(F_VB, 0) = v0; }
   __syncthreads();
 
@@ -156,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const float ps = prh_u * sch;
       s1 = __fmul_rn(ps, u0);
       x2 = __fmul_rn(ps * v0, RH(3));
-      const float rdx4 = RDXX(4), rrh4 = vy[16 * H + ly];
+      const float rdx4 = RDXX(4), rrh4 = vy[16 * YS];
       a1u = __fmul_rn((u0 - SF(F_UB, -1)) * rdx4, rrh4);
       a1v = __fmul_rn((v0 - SF(F_VB, -1)) * rdx4, rrh4);
       const float rdy2 = RDXY(2), rh2 = RH(2);
@@ -183,10 +190,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       const float A = __fmul_rn(tEc - tEw, RDXX(1));
       float B = __fmul_rn(tNc - tNs, RDXY(1));
       if (!srow) B = 0.f;
-      const float div = __fadd_rn(A, B) * vy[13 * H + ly];
+      const float div = __fadd_rn(A, B) * vy[13 * YS];
       pred = c0 - (double)(div * bt * gamma_b * rprh_t);
       if (levt <= 0) pred = nt == 1 ? land_ch0 : c0;
-      const float rdx3 = RDXX(3), rdy3 = RDXY(3), raarh = vy[18 * H + ly];
+      const float rdx3 = RDXX(3), rdy3 = RDXY(3), raarh = vy[18 * YS];
       const float L1u = __fmul_rn(SF(F_A1U, 1) - a1u, rdx3), L1v = __fmul_rn(SF(F_A1V, 1) - a1v, rdx3);
       float L2u = __fmul_rn(SF(F_A2U, W) - a2u, rdy3), L2v = __fmul_rn(SF(F_A2V, W) - a2v, rdy3);
       if (!nrow) L2u = L2v = 0.f;
@@ -206,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       float sch = sqrtf(s6sea ? (float)w : 1.f);
       if (s2zero) sch = 0.f;
       const float rdx2 = RDXX(2), rdy4 = RDXY(4);
-      const float gx0 = (float)(pe - pred) * rdx2 * vy[15 * H + ly], gx1 = (float)(pne - pn) * rdx2 * vy[15 * H + ly + 1];
+      const float gx0 = (float)(pe - pred) * rdx2 * vy[15 * YS], gx1 = (float)(pne - pn) * rdx2 * vy[15 * YS + YR];
       const float gy0 = (float)(pn - pred) * rdy4 * ra, gy1 = (float)(pne - pe) * rdy4 * ra;
       const double ce0 = 0.5 * (pred + pe), ce1 = 0.5 * (pn + pne), cn0 = 0.5 * (pred + pn), cn1 = 0.5 * (pe + pne);
       float gi1 = 0.5f * __fmaf_rn(gx0, bxn, __fmul_rn(gx1, bxs)), gi2 = 0.5f * __fmaf_rn(gy0, bye, __fmul_rn(gy1, byw));
@@ -241,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const float A = __fmul_rn(tEc - tEw, RDXX(1));
       float B = __fmul_rn(tNc - tNs, RDXY(1));
       if (!srow) B = 0.f;
-      const float div = __fadd_rn(A, B) * vy[13 * H + ly];
+      const float div = __fadd_rn(A, B) * vy[13 * YS];
       c0 = c0 - (double)(mskt1 * div * bt * rprh_t);
       if (border && nt < nstep) xch_put(out, c0, seq + nt);
       u0 = ubc; v0 = vbc;
@@ -295,16 +302,22 @@ namespace {
 const void *mixed_kernel(int TX, int TY) {
 #define PCOM_MIXED_SHAPE(x, y) \
   if (TX == (x) && TY == (y)) return (const void *)k_trop_mixed<(x), (y)>;
-  PCOM_TROP_SHAPES(PCOM_MIXED_SHAPE)
+  PCOM_TROP_SMALL(PCOM_MIXED_SHAPE)
 #undef PCOM_MIXED_SHAPE
   return (const void *)k_trop_mixed<>;
 }
 }  // namespace
 
 size_t trop_mixed_smem_bytes(int TX, int TY) {
+  bool free = true;
+#define PCOM_MIXED_SHAPE(x, y) \
+  if (TX == (x) && TY == (y)) free = false;
+  PCOM_TROP_SMALL(PCOM_MIXED_SHAPE)
+#undef PCOM_MIXED_SHAPE
   const int W = TX + 4, H = TY + 4;
-  const size_t rs = (size_t)W * H, margin = 2 * (size_t)pad(W) + 32;
-  return (D_COUNT * rs + margin) * sizeof(double) + (F_COUNT * rs + margin + kVx * W + kVy * H + 1) * sizeof(float);
+  const size_t rs = free ? kThreads : (size_t)W * H, margin = 2 * (size_t)pad(free ? kSide : W) + 32;
+  return (D_COUNT * rs + margin) * sizeof(double) +
+         (F_COUNT * rs + margin + (kVx + free) * W + kVy * (H + 1)) * sizeof(float);
 }
 
 int trop_mixed_max_blocks(int TX, int TY) {

@@ -534,10 +534,10 @@ int pick_trop_config(pcom_handle *h) {
       h->trop_blocks = n;
       return PCOM_OK;
     };
-    // the compiled shape with the fewest warps per CTA whose tiles fit one
-    // per SM, then the fewest tiles: a substep's stages issue every warp's
-    // instructions on one SM, while its messages cost the same whatever the
-    // number of tiles
+    // tiles that fit one per SM.  A shape compiled for small tiles, where one
+    // covers the domain: the fewest warps per CTA, then the fewest tiles (a
+    // substep's stages issue every warp's instructions on one SM, while its
+    // messages cost the same whatever the number of tiles)
     int nsm = 0, best_w = 1 << 30, best_n = 0, bx = 0, by = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
 #define PCOM_TRY_SHAPE(x, y)                                                                   \
@@ -545,20 +545,19 @@ int pick_trop_config(pcom_handle *h) {
     const int n_ = tiles((x), (y)), w_ = (((x) + 4) * ((y) + 4) + 31) / 32;                    \
     if (n_ <= nsm && (w_ < best_w || (w_ == best_w && n_ < best_n))) { best_w = w_; best_n = n_; bx = (x); by = (y); } \
   }
-    PCOM_TROP_SHAPES(PCOM_TRY_SHAPE)
+    PCOM_TROP_SMALL(PCOM_TRY_SHAPE)
 #undef PCOM_TRY_SHAPE
-    if (bx > 0 && trop_fast_max_blocks(bx, by) >= best_n) return take(bx, by, best_n);
-    // a domain that only another shape covers: the fewest tiles
-    best_n = 1 << 30;
-    bx = by = 0;
-    const int mb = trop_fast_max_blocks(24, 18);
-    for (int ty = 6; ty <= 40; ++ty)
-      for (int tx = 6; tx <= 60; ++tx) {
-        if (!trop_res_fits(tx, ty)) continue;
-        const int nt = tiles(tx, ty);
-        if (nt > mb) continue;
-        if (nt < best_n || (nt == best_n && (tx + 4) * (ty + 4) < (bx + 4) * (by + 4))) { best_n = nt; bx = tx; by = ty; }
-      }
+    // larger domains: any shape by the same rule, where rows of 32 points (a
+    // warp's messages and loads are one row's) count as 1.5 warps less.
+    // int_trop of 300 x 152 points in us: 16 warps in rows of 32 397, of 28
+    // 417, of 24 420, 18 warps in rows of 28 443; of 360 x 162: 19 in rows of
+    // 32 444, of 27 442, 20 in rows of 32 450, of 28 467
+    if (bx == 0)
+      for (int ty = 6; ty <= 40; ++ty)
+        for (int tx = 6; tx <= 60; ++tx) {
+          const int n = tiles(tx, ty), c = ((tx + 4) * (ty + 4) + 31) / 32 * 2 - (tx == 28 ? 3 : 0);
+          if (trop_res_fits(tx, ty) && n <= nsm && (c < best_w || (c == best_w && n < best_n))) { best_w = c; best_n = n; bx = tx; by = ty; }
+        }
     if (bx > 0 && trop_fast_max_blocks(bx, by) >= best_n) return take(bx, by, best_n);
   }
   // too large to be resident: the multi-tile kernels

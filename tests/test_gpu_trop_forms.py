@@ -12,6 +12,7 @@ from pcom_b200 import _lib as L
 from pcom_b200.model import Batch, Model
 from pcom_b200.synth import make_case
 from parity_util import STATE_FIELDS, compare
+from test_gpu_mixed import BOUNDS, errors
 
 pytestmark = pytest.mark.gpu
 
@@ -69,5 +70,21 @@ def test_batch_of_fitted_tiles(sizes):
             assert d["unequal"] == 0, f"{c['itn'].shape}, {f}: {d['unequal']} values differ"
         r.close()
     b.close()
+    for m in ms:
+        m.close()
+
+
+@pytest.mark.parametrize("size", [(24, 14, 3), (150, 100, 3), (211, 97, 3)], ids=lambda s: "x".join(map(str, s)))
+def test_mixed_resident_shapes(size):
+    """The mixed resident kernel at a compiled shape and at shapes of the
+    domain's own does the multi-tile mixed kernel's arithmetic in code compiled
+    apart: half the mixed bounds, as on the 1-degree domain."""
+    c = make_case("basin", noise=0.01, glo_ni=size[0], glo_nj=size[1], nk=size[2])
+    ms = [Model(c, flags=L.PCOM_PREC_MIXED) for _ in range(2)]
+    L.check(ms[1].lib.pcom_gpu_set_trop_kernel(ms[1].handle, 2), "set_trop_kernel")
+    for m in ms:
+        m.run(6)
+    for f, e in errors(ms[0], ms[1]).items():
+        assert e <= 0.5 * BOUNDS[f], f"{f} rel RMS {e:.3e}"
     for m in ms:
         m.close()
