@@ -30,7 +30,12 @@
 // end in a serial column pass by one or two warps, and smaller blocks let
 // more of them per SM overlap that pass with other blocks' loads (1-degree
 // FP64 step 1.240 -> 1.188 ms).  k_pgra2d needs TB_K >= 8 (one column sum per
-// thread row).
+// thread row).  These kernels wait for loads, and threads to wait with are
+// worth more than registers: k_clin with 64, 80, 128 registers takes 236, 263,
+// 350 us on 720 x 320 x 30 points, k_upwelling with 40, 48, 64 60, 66, 70 us
+// (less does not pay: 48 for k_clin 265, 32 for k_upwelling 64).  What a loop
+// adds to is loaded ahead of the loop's stores, behind which the compiler has
+// to leave it (k_clin 257 -> 236 us, k_ts_acc 149 -> 99).
 #define TB_X 32
 #define TB_K 8
 static_assert(TB_K >= 8, "k_pgra2d computes one of its 8 column sums per thread row");
@@ -115,7 +120,7 @@ __global__ void __launch_bounds__(512) k_alpha_tobot(const __grid_constant__ Dev
 // E/N-averaged geopotential and of the adp gradient (op_vint_ns/op_vint_ew,
 // mod_op.f90:946-981, incl. their cshift(-1) masks).
 template <typename R, bool BATCH>
-__global__ void __launch_bounds__(512) k_pgra2d(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
+__global__ void __launch_bounds__(TB_X * TB_K, 4) k_pgra2d(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
   constexpr bool MIXED = std::is_same<R, float>::value;
   (void)MIXED;
@@ -234,7 +239,7 @@ __host__ __device__ constexpr int upw_cols() { return std::is_same<R, double>::v
 // wm(k) = (wm(k-1) + dpr(k-1) (wk3d(k-1) - vint(wk3d))) msk(k).
 // with_acw: also int_ts's acw accumulation (mod_int.f90:458-461).
 template <typename R, bool BATCH>
-__global__ void __launch_bounds__(512) k_upwelling(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps, int with_acw) {
+__global__ void __launch_bounds__(upw_cols<R>() * TB_K, sizeof(R) == 8 ? 12 : 4) k_upwelling(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps, int with_acw) {
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
   constexpr bool MIXED = std::is_same<R, float>::value;
   (void)MIXED;
@@ -286,11 +291,13 @@ __global__ void __launch_bounds__(512) k_upwelling(const __grid_constant__ DevT<
   if (!ok) return;
   for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
     const long long q = q2 + P.n2 * (k - 1);
+    const bool acc = with_acw && k <= max(lev, 1);
+    const double aw = acc ? P.acw[q] : 0.0;  // (ahead of the store of wm)
     const double w = k <= max(lev, 1) ? wmv[(k - 1) * UX + tx] : 0.0;
     if (k >= 2) st2(P.wm, P, i, q, w);
-    if (with_acw && k <= max(lev, 1)) {
+    if (acc) {
       const double gm = P.c.g * ld(P.mch2, q2);
-      st2(P.acw, P, i, q, P.acw[q] + dvr(w * alpha_full(P, ld(P.alpha, q), k), gm, ld(P.rgm2, q2)));
+      st2(P.acw, P, i, q, aw + dvr(w * alpha_full(P, ld(P.alpha, q), k), gm, ld(P.rgm2, q2)));
     }
   }
 }
@@ -708,7 +715,7 @@ __global__ void __launch_bounds__(kColX * (NC == 1 ? 2 : NC), NC == 1 ? 6 : 3)
 // int_clin (mod_int.f90:298-396): baroclinic momentum, barotropic
 // replacement, unweighted velocity and its accumulation.  smag runs after.
 template <typename R, bool BATCH>
-__global__ void __launch_bounds__(512, 2) k_clin(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
+__global__ void __launch_bounds__(TB_X * TB_K, 4) k_clin(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
   constexpr bool MIXED = std::is_same<R, float>::value;
   (void)MIXED;
@@ -807,6 +814,8 @@ __global__ void __launch_bounds__(512, 2) k_clin(const __grid_constant__ DevT<R>
   for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
     const long long q = q2 + P.n2 * (k - 1);
     double un = uns[(k - 1) * TB_X + tx], vn = vns[(k - 1) * TB_X + tx];
+    // (ahead of the stores, which the compiler must keep them behind)
+    const double au = P.acu[q], av = P.acv[q];
     if (lu >= k) {
       un = un - w1 + ubc;
       vn = vn - w2 + vbc;
@@ -818,8 +827,8 @@ __global__ void __launch_bounds__(512, 2) k_clin(const __grid_constant__ DevT<R>
     const double uu = dvr(un * schu, mch2, rmch2), vv = dvr(vn * schu, mch2, rmch2);
     st2(P.uu, P, i, q, uu);
     st2(P.vv, P, i, q, vv);
-    st2(P.acu, P, i, q, P.acu[q] + uu);
-    st2(P.acv, P, i, q, P.acv[q] + vv);
+    st2(P.acu, P, i, q, au + uu);
+    st2(P.acv, P, i, q, av + vv);
   }
 }
 
@@ -827,7 +836,7 @@ __global__ void __launch_bounds__(512, 2) k_clin(const __grid_constant__ DevT<R>
 // smag (mod_int.f90:403-440): Smagorinsky viscosity, rows 2..nj-1.
 constexpr int kSmagK = 4;  // levels per thread of a single-domain launch
 template <typename R, bool BATCH>
-__global__ void k_smag(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
+__global__ void __launch_bounds__(128, 12) k_smag(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
   constexpr bool MIXED = std::is_same<R, float>::value;
   (void)MIXED;
@@ -863,7 +872,7 @@ __global__ void k_smag(const __grid_constant__ DevT<R> P0, const DevT<R> *__rest
 // ----------------------------------------------------------------------------
 // int_ssh (mod_int.f90:602-624): alpha from (tp, sp, mch), SSH accumulation.
 template <typename R, bool BATCH>
-__global__ void __launch_bounds__(512) k_ssh(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
+__global__ void __launch_bounds__(TB_X * TB_K, 4) k_ssh(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
   constexpr bool MIXED = std::is_same<R, float>::value;
   (void)MIXED;
@@ -1309,8 +1318,11 @@ __global__ void __launch_bounds__(kColX * (NC == 1 ? 2 : NC), NC == 1 ? 6 : 3)
   }
 }
 
+// Its time is the loads' latency: with every load ahead of the iteration's
+// stores, and the next level's in flight behind this one's equation of state
+// (32 us at 1 degree; one load after the other 47).
 template <bool BATCH>
-__global__ void __launch_bounds__(512, 2) k_ts_acc(const __grid_constant__ DevT<double> P0,
+__global__ void __launch_bounds__(TB_X * TB_K, 4) k_ts_acc(const __grid_constant__ DevT<double> P0,
                                                 const DevT<double> *__restrict__ Ps) {
   const DevT<double> &P = BATCH ? Ps[blockIdx.z] : P0;
   int i, j;
@@ -1321,19 +1333,33 @@ __global__ void __launch_bounds__(512, 2) k_ts_acc(const __grid_constant__ DevT<
   const int ni = P.ni;
   const bool twin = i == 2 || i == ni - 1;
   const long long dq = i == 2 ? (long long)(ni - 2) : -(long long)(ni - 2);
-  for (int k = threadIdx.y + 1; k <= P.nk; k += TB_K) {
+  struct Level {
+    double t, s, at, as, ar;
+  };
+  auto load = [&](int k) {
     const long long q = q2 + P.n2 * (k - 1);
-    const double tn = P.tn_[q], sn = P.sn_[q];
+    return Level{P.tn_[q], P.sn_[q], P.act[q], P.acs[q], k <= lev ? P.acr[q] : 0.0};
+  };
+  int k = threadIdx.y + 1;
+  if (k > P.nk) return;
+  #pragma unroll 1
+  for (Level v = load(k);; k += TB_K) {
+    const bool more = k + TB_K <= P.nk;
+    Level next{};
+    if (more) next = load(k + TB_K);
+    const long long q = q2 + P.n2 * (k - 1);
     if (twin) {
-      P.tn_[q + dq] = tn;
-      P.sn_[q + dq] = sn;
+      P.tn_[q + dq] = v.t;
+      P.sn_[q + dq] = v.s;
     }
-    st2(P.act, P, i, q, P.act[q] + tn);
-    st2(P.acs, P, i, q, P.acs[q] + sn);
+    st2(P.act, P, i, q, v.at + v.t);
+    st2(P.acs, P, i, q, v.as + v.s);
     if (k <= lev) {
-      const double w = 1.0 / den_rho(P.c, tn, sn, chc * P.pr2[k]);
-      st2(P.acr, P, i, q, P.acr[q] + 1.0 / w);
+      const double w = 1.0 / den_rho(P.c, v.t, v.s, chc * P.pr2[k]);
+      st2(P.acr, P, i, q, v.ar + 1.0 / w);
     }
+    if (!more) return;
+    v = next;
   }
 }
 
