@@ -35,7 +35,8 @@
 // 350 us on 720 x 320 x 30 points, k_upwelling with 40, 48, 64 60, 66, 70 us
 // (less does not pay: 48 for k_clin 265, 32 for k_upwelling 64).  What a loop
 // adds to is loaded ahead of the loop's stores, behind which the compiler has
-// to leave it (k_clin 257 -> 236 us, k_ts_acc 149 -> 99).
+// to leave it (k_clin 257 -> 236 us, k_ts_acc 149 -> 99,
+// the mixed k_ts 323 -> 298).
 #define TB_X 32
 #define TB_K 8
 static_assert(TB_K >= 8, "k_pgra2d computes one of its 8 column sums per thread row");
@@ -322,7 +323,7 @@ __device__ __forceinline__ void readyc_dry(const DevT<R> &P, int i, long long q)
 // (mod_op.f90:224-278), op_fri -> fri_r3d for both components
 // (mod_op.f90:103-184) and the depth integral of the baroclinic tendency.
 template <typename R, bool BATCH>
-__global__ void __launch_bounds__(512) k_readyc3d(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
+__global__ void __launch_bounds__(TB_X * TB_K, 4) k_readyc3d(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
   constexpr bool MIXED = std::is_same<R, float>::value;
   (void)MIXED;
@@ -964,9 +965,7 @@ __device__ void ts_convect(const DevT<R> &P, long long q2, int nlev, C c) {
 }
 
 template <typename R, bool BATCH>
-// (FP32 storage: registers for two CTAs per SM)
-__global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1) k_ts(const __grid_constant__ DevT<R> P0,
-                                                                    const DevT<R> *__restrict__ Ps) {
+__global__ void __launch_bounds__(TB_X * TB_K, 4) k_ts(const __grid_constant__ DevT<R> P0, const DevT<R> *__restrict__ Ps) {
   const DevT<R> &P = BATCH ? Ps[blockIdx.z] : P0;
   constexpr bool MIXED = std::is_same<R, float>::value;
   (void)MIXED;
@@ -1106,13 +1105,14 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1) k_ts(const __grid
   for (int k = threadIdx.y + 1; k <= nk; k += TB_K) {
     const long long q = q2 + P.n2 * (k - 1);
     const double tn = tcs[(k - 1) * TB_X + tx], sn = scs[(k - 1) * TB_X + tx];
+    const double at = P.act[q], as = P.acs[q], ar = k <= lev ? P.acr[q] : 0.0;
     st2(P.tn_, P, i, q, tn);
     st2(P.sn_, P, i, q, sn);
-    st2(P.act, P, i, q, P.act[q] + tn);
-    st2(P.acs, P, i, q, P.acs[q] + sn);
+    st2(P.act, P, i, q, at + tn);
+    st2(P.acs, P, i, q, as + sn);
     if (k <= lev) {
       const double w = 1.0 / den_rho(P.c, tn, sn, chc * P.pr2[k]);
-      st2(P.acr, P, i, q, P.acr[q] + 1.0 / w);
+      st2(P.acr, P, i, q, ar + 1.0 / w);
     }
   }
 }
