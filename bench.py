@@ -296,7 +296,7 @@ def run_ours(args):
     clk.__exit__(None, None, None)
 
     # the barotropic subcycle's latency floor: its synchronisation skeleton
-    # (same grid, block, barriers, ring reload and stores; no arithmetic),
+    # (same grid, block, barriers and messages; no arithmetic),
     # the median of 3 launches after 2; None where the handle does not run
     # the resident FP64 kernel
     floor_ms = None
@@ -386,8 +386,8 @@ def run_ours(args):
                          # the barotropic subcycle keeps its state on chip: its
                          # time is the latency of 120 dependent substeps
                          "us_per_substep": round(avg_s * 1e6 / nstep, 3) if kname == "int_trop" else None,
-                         # against the latency floor: the kernel's barriers,
-                         # ring reload and stores without its arithmetic
+                         # against the latency floor: the kernel's barriers
+                         # and messages without its arithmetic
                          "latency_floor": ({"us_per_substep": round(floor_ms * 1e3 / nstep, 3),
                                             "floor_over_actual": round(floor_ms * 1e-3 / avg_s, 3),
                                             "measured": "pcom_gpu_trop_floor: the resident kernel's synchronisation "

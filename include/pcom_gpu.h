@@ -210,11 +210,12 @@ int pcom_gpu_set_trop_kernel(pcom_handle *h, int32_t which);
  * either way; 0 issues every launch on the handle's stream in phase order.
  * pcom_gpu_phase always runs serially.  No counterpart in the reference. */
 int pcom_gpu_set_overlap(pcom_handle *h, int32_t enable);
-/* Longest a device-side wait (a grid barrier of the barotropic kernels) may
- * take before the kernel gives up, returns early and the next synchronising
- * call reports PCOM_ERR_TIMEOUT (default 2 s; the barriers normally take
- * microseconds).  The handle stays usable after a timeout: its barrier
- * counters are reset, the state of the interrupted step is not meaningful.
+/* Longest a device-side wait of the barotropic kernels (for a neighbouring
+ * tile's message, or at the multi-tile kernels' grid barrier) may take before
+ * the kernel gives up, returns early and the next synchronising call reports
+ * PCOM_ERR_TIMEOUT (default 2 s; the waits normally take microseconds).  The
+ * handle stays usable after a timeout; the state of the interrupted step is
+ * not meaningful.
  * No counterpart in the reference. */
 int pcom_gpu_set_wait_limit(pcom_handle *h, double seconds);
 /* Global sums over the wet T cells of the interior: out3[0] = volume (m^3),
@@ -229,12 +230,11 @@ int pcom_gpu_set_stream(pcom_handle *h, void *stream);
 int pcom_gpu_sync(pcom_handle *h);
 /* Latency floor of the barotropic subcycle: one launch of the resident FP64
  * kernel's synchronisation skeleton.  It has the same grid, block and
- * shared memory, and per substep the same ring reload, the seven CTA
- * barriers, the interior stores and the grid barrier, without the
- * arithmetic.  Its device time in milliseconds for the handle's nstep
+ * shared memory, and per substep the same four CTA barriers and the same
+ * messages to and from the neighbouring tiles, without the arithmetic.  Its device time in milliseconds for the handle's nstep
  * substeps goes to *ms (CUDA events; the call synchronises the handle's
  * stream).  The model state is unchanged: the skeleton writes only the
- * subcycle's scratch buffers.  PCOM_ERR_STATE unless the handle runs the
+ * message buffer.  PCOM_ERR_STATE unless the handle runs the
  * resident FP64 kernel.  No counterpart in the reference. */
 int pcom_gpu_trop_floor(pcom_handle *h, double *ms);
 /* Per-kernel device timing with CUDA events (off by default).  When on,

@@ -1,5 +1,7 @@
 // k_trop.cu -- the barotropic predictor/corrector subcycle of int_trop
-// (mod_int.f90:153-296) as ONE persistent cooperative kernel.
+// (mod_int.f90:153-296) as ONE persistent cooperative kernel.  k_trop_fast,
+// further down, is the form that lat-lon domains of up to one tile per SM and
+// batches run; what follows here describes the general one.
 //
 // The 2-D domain (interior columns x all rows) is cut into TX x TY tiles.
 // Each CTA owns tiles; for every substep it stages a (TX+4) x (TY+4) region of

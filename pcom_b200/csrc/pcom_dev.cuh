@@ -78,7 +78,7 @@ struct DevCommon {
   // too large to be resident
   ulonglong2 *xch;
   int *err;        // [0] timeout flag, [1] watchdog flag
-  // longest a device-side wait (the barotropic kernels' grid barriers) may
+  // longest a device-side wait (the barotropic kernels' messages and grid barriers) may
   // take before it gives up and sets err[0] (ns of global time)
   unsigned long long wait_ns = 2000000000ULL;
   // lat-lon (separable) metrics: dx?x depends on i only, dx?y and rh? on j

@@ -460,7 +460,7 @@ int sync_check(pcom_handle *h) {
     cudaMemsetAsync(h->D.err, 0, sizeof err, h->stream);
     cudaMemsetAsync(h->D.bar, 0, 2 * sizeof(unsigned), h->stream);
     cudaStreamSynchronize(h->stream);
-    return fail(PCOM_ERR_TIMEOUT, "a device-side grid barrier gave up waiting (bounded spin)");
+    return fail(PCOM_ERR_TIMEOUT, "a device-side wait of a barotropic kernel gave up (bounded spin)");
   }
   return PCOM_OK;
 }
@@ -2090,7 +2090,7 @@ int batch_sync(pcom_batch *b) {
   if (err) {
     cudaMemsetAsync(b->err, 0, sizeof(int), b->stream);
     cudaStreamSynchronize(b->stream);
-    return fail(PCOM_ERR_TIMEOUT, "a device-side grid barrier of the batch gave up waiting (bounded spin)");
+    return fail(PCOM_ERR_TIMEOUT, "a device-side wait of the batch's barotropic kernels gave up (bounded spin)");
   }
   return PCOM_OK;
 }
