@@ -75,10 +75,12 @@ __global__ void k_mm_prep(const __grid_constant__ Dev P, MultiMixed M) {
 
 }  // namespace
 
-template <int CTX = 0, int CTY = 0>
+// SKIP: the tiles from number nwet on are without sea (a form of its own: it
+// costs the other 1 %)
+template <bool SKIP, int CTX = 0, int CTY = 0>
 __global__ void __launch_bounds__(kThreads) k_trop_multi_mixed(const __grid_constant__ Dev P, const MultiMixed M,
-                                                               const TileRef *__restrict__ tiles, int ntiles, int TX,
-                                                               int TY, unsigned long long *cnt, int *err) {
+                                                               const TileRef *__restrict__ tiles, int ntiles, int nwet,
+                                                               int TX, int TY, unsigned long long *cnt, int *err) {
   if (CTX > 0) { TX = CTX; TY = CTY; }
   extern __shared__ double smd[];
   const int W = TX + 4, RS = W * (TY + 4);
@@ -114,7 +116,10 @@ __global__ void __launch_bounds__(kThreads) k_trop_multi_mixed(const __grid_cons
     // the velocity ping-pong, selected without indexing the parameter array
     const float *src_ub = d ? M.ub[0] : M.ub[1], *src_vb = d ? M.vb[0] : M.vb[1];
     float *dst_ub = d ? M.ub[1] : M.ub[0], *dst_vb = d ? M.vb[1] : M.vb[0];
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    // tiles without sea keep their state: two substeps put it into both
+    // buffers that their neighbours read, the rest skip them (int_trop of a
+    // 1440 x 640 globe with 28 % of such tiles: 9.72 -> 7.67 ms)
+    for (int t = blockIdx.x; t < (!SKIP || nt <= 2 ? ntiles : nwet); t += gridDim.x) {
       const TileRef T = tiles[t];
       const int tw = T.tw, th = T.th, rr0 = T.r0 - 2, jj0 = T.j0 - 2;
       auto ring_i = [&](int r) { r %= G; if (r < 0) r += G; return r + 2; };
@@ -308,8 +313,16 @@ __global__ void __launch_bounds__(kThreads) k_trop_multi_mixed(const __grid_cons
     for (int p = tid; p < T.tw * T.th; p += nth) {
       const int i = T.r0 + p % T.tw + 2, j = T.j0 + p / T.tw;
       const long long q = I2(P, i, j);
-      const double ub = P.tr_acc[2][q] / (nstep + 1), vb = P.tr_acc[3][q] / (nstep + 1);
-      const double mch = P.tr_acc[0][q] / (nstep / 2 + 1), mch2 = P.tr_acc[1][q] / (nstep + 1);
+      double a0 = P.tr_acc[0][q], a1 = P.tr_acc[1][q], a2 = P.tr_acc[2][q], a3 = P.tr_acc[3][q];
+      if (SKIP && t >= nwet) {  // the sums of the substeps it was skipped in
+        const double c = P.tr_ch[1][q], u = (double)M.ub[1][q], v = (double)M.vb[1][q];
+        for (int nt = 3; nt <= nstep / 2; ++nt) a0 = a0 + c;
+        for (int nt = 3; nt <= nstep; ++nt) a1 = a1 + c;
+        for (int nt = 3; nt <= nstep; ++nt) a2 = a2 + u;
+        for (int nt = 3; nt <= nstep; ++nt) a3 = a3 + v;
+      }
+      const double ub = a2 / (nstep + 1), vb = a3 / (nstep + 1);
+      const double mch = a0 / (nstep / 2 + 1), mch2 = a1 / (nstep + 1);
       st2(P.ubc, P, i, q, ub);
       st2(P.vbc, P, i, q, vb);
       st2(P.ubp, P, i, q, ub);
@@ -326,9 +339,10 @@ __global__ void __launch_bounds__(kThreads) k_trop_multi_mixed(const __grid_cons
 namespace {
 // the fixed-shape form for the 32 x 10 tiles the single-domain multi-tile
 // path uses
-const void *mm_kernel(int TX, int TY) {
-  if (TX == 32 && TY == 10) return (const void *)k_trop_multi_mixed<32, 10>;
-  return (const void *)k_trop_multi_mixed<>;
+const void *mm_kernel(int TX, int TY, bool skip) {
+  if (TX == 32 && TY == 10)
+    return skip ? (const void *)k_trop_multi_mixed<true, 32, 10> : (const void *)k_trop_multi_mixed<false, 32, 10>;
+  return skip ? (const void *)k_trop_multi_mixed<true> : (const void *)k_trop_multi_mixed<false>;
 }
 }  // namespace
 
@@ -359,25 +373,25 @@ int trop_multi_mixed_max_blocks(int TX, int TY) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const size_t smem = trop_multi_mixed_smem(TX, TY);
-  const void *fn = mm_kernel(TX, TY);
+  const void *fn = mm_kernel(TX, TY, true);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kThreads, smem) != cudaSuccess) return 0;
   return per * nsm;
 }
 
-cudaError_t launch_trop_multi_mixed(const Dev &P, const MultiMixed &M, const TileRef *dtiles, int ntiles, int TX,
-                                    int TY, int nblocks, unsigned long long *cnt, int *err, cudaStream_t s) {
+cudaError_t launch_trop_multi_mixed(const Dev &P, const MultiMixed &M, const TileRef *dtiles, int ntiles, int nwet,
+                                    int TX, int TY, int nblocks, unsigned long long *cnt, int *err, cudaStream_t s) {
   k_mm_prep<<<592, 256, 0, s>>>(P, M);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const size_t smem = trop_multi_mixed_smem(TX, TY);
-  const void *fn = mm_kernel(TX, TY);
+  const void *fn = mm_kernel(TX, TY, nwet < ntiles);
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   // the barrier counter starts from zero in every launch
   e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  void *args[] = {(void *)&P, (void *)&M, (void *)&dtiles, (void *)&ntiles, (void *)&TX, (void *)&TY, (void *)&cnt,
+  void *args[] = {(void *)&P, (void *)&M, (void *)&dtiles, (void *)&ntiles, (void *)&nwet, (void *)&TX, (void *)&TY, (void *)&cnt,
                   (void *)&err};
   return cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(kThreads), args, smem, s);
 }

@@ -74,12 +74,13 @@ def test_batch_of_fitted_tiles(sizes):
         m.close()
 
 
+@pytest.mark.parametrize("land", ["none", "band"])
 @pytest.mark.parametrize("size", [(24, 14, 3), (150, 100, 3), (211, 97, 3)], ids=lambda s: "x".join(map(str, s)))
-def test_mixed_resident_shapes(size):
+def test_mixed_resident_shapes(size, land):
     """The mixed resident kernel at a compiled shape and at shapes of the
     domain's own does the multi-tile mixed kernel's arithmetic in code compiled
     apart: half the mixed bounds, as on the 1-degree domain."""
-    c = make_case("basin", noise=0.01, glo_ni=size[0], glo_nj=size[1], nk=size[2])
+    c = dict(_case(*size, land), dtbt=60, dtbc=3600)
     ms = [Model(c, flags=L.PCOM_PREC_MIXED) for _ in range(2)]
     L.check(ms[1].lib.pcom_gpu_set_trop_kernel(ms[1].handle, 2), "set_trop_kernel")
     for m in ms:
