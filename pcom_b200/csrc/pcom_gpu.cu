@@ -2010,15 +2010,26 @@ int batch_tiles(pcom_batch *b, int TX, int TY, int points) {
   return PCOM_OK;
 }
 
-// the tile sizes a batch may take (points of a region), the cheapest by the
-// model first (24 box members and basins: 608 points modelled 1.39 ms, 1.38
-// measured; 640: 1.42, 1.42; 320, two tiles on an SM: 1.76, 1.70)
+// the tile sizes a batch may take (points of a region), best first: those
+// that leave the fewest tiles to the multi-tile kernel, which takes several
+// times as long (a step of two 360 x 160 x 3 members, resident at 608 and 640
+// points and not below: 1.29 ms against 3.40), then the cheapest by the model
+// (24 box members and basins: 608 points modelled 1.39 ms, 1.38 measured;
+// 640: 1.42, 1.42; 320, two tiles on an SM: 1.76, 1.70)
 std::vector<int> batch_sizes(const pcom_batch *b) {
-  std::vector<std::pair<double, int>> v;
-  for (int points = 640; points >= 128; points -= 32) v.push_back({batch_plan(b, 24, 18, points).cost, points});
-  std::stable_sort(v.begin(), v.end(), [](const auto &x, const auto &y) { return x.first < y.first; });
+  struct Size {
+    size_t big;
+    double cost;
+    int points;
+  };
+  std::vector<Size> v;
+  for (int points = 640; points >= 128; points -= 32) {
+    const BatchPlan p = batch_plan(b, 24, 18, points);
+    v.push_back({p.big.size(), p.cost, points});
+  }
+  std::stable_sort(v.begin(), v.end(), [](const Size &x, const Size &y) { return x.big != y.big ? x.big < y.big : x.cost < y.cost; });
   std::vector<int> s;
-  for (auto &c : v) s.push_back(c.second);
+  for (auto &c : v) s.push_back(c.points);
   return s;
 }
 
@@ -2288,7 +2299,7 @@ int pcom_gpu_batch_autotune(pcom_batch *b, char *report, int32_t len) {
       return PCOM_OK;
     }
   }
-  // the sizes the model finds cheapest (it is within some percent)
+  // the best sizes by the model (it is within some percent)
   std::vector<int> cand = batch_sizes(b);
   cand.resize(6);
   for (cudaStream_t s : b->member_streams) CK(cudaStreamSynchronize(s));

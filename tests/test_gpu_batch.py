@@ -100,6 +100,32 @@ def test_batch_autotune_keeps_results():
         m.close()
 
 
+@pytest.mark.parametrize("sizes,groups", [([(360, 160)] * 2, 2), ([(200, 148)] * 4, 2), ([(360, 160), (128, 64)], 2)],
+                         ids=["1-degree members", "four basins", "uneven"])
+def test_batch_keeps_large_members_resident(sizes, groups):
+    """Members that fit the resident barotropic kernel at some tile size run
+    in it from the batch's creation on: a step is 13 launches and two per
+    resident group (its tiles, its messages' sequence base); the multi-tile
+    kernel would be one launch for all members left to it.  The tuner keeps
+    them resident as well."""
+    cases = [dict(make_case("basin", noise=0.01, glo_ni=ni, glo_nj=nj, nk=3), dtbt=20, dtbc=1200) for ni, nj in sizes]
+    ms = [Model(c) for c in cases]
+    b = Batch(ms)
+
+    def launches():
+        before = b.launch_count()
+        b.run(1)
+        return b.launch_count() - before
+
+    b.run(3)
+    assert launches() == 13 + 2 * groups
+    report = b.autotune()
+    assert launches() == 13 + 2 * groups, report
+    b.close()
+    for m in ms:
+        m.close()
+
+
 def test_batch_on_caller_stream():
     """Members on the caller's (legacy default) stream: the batch captures on
     its own stream and joins the members' streams by events."""
