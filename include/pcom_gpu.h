@@ -120,7 +120,9 @@ int pcom_gpu_destroy(pcom_handle *h);
 /* --- data movement ------------------------------------------------------- */
 /* Grid data computed by set_hgrid/set_vgrid/set_grid/calc_cf/inistat
  * (main.f90:408-704).  Masks must be the ones set_grid builds
- * (msk = lev >= k); any other mask is rejected with PCOM_ERR_ARG. */
+ * (msk = lev >= k); any other mask is rejected with PCOM_ERR_ARG.  The
+ * barotropic kernel's form is chosen here and its memory taken, so that the
+ * first step allocates nothing. */
 int pcom_gpu_upload_static(pcom_handle *h, const pcom_static *s);
 /* State in/out: at start-up (inistat, main.f90:675-704), restart read
  * (input_rst, mod_mympi.f90:460-478) and restart write (merge_out_rst,

@@ -380,8 +380,8 @@ int trop_max_blocks(int TX, int TY) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const size_t smem = trop_smem_bytes(TX, TY);
-  cudaFuncSetAttribute(k_trop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trop, 256, smem);
+  if (cudaFuncSetAttribute(k_trop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trop, 256, smem) != cudaSuccess) return 0;
   return per * nsm;
 }
 

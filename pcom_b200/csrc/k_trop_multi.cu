@@ -399,26 +399,30 @@ size_t xm_doubles(int glo_ni, int TX) { return (size_t)((glo_ni + TX - 1) / TX) 
 size_t ym_doubles(int nj, int TY) { return (size_t)((nj + TY - 1) / TY) * kYVecs * (TY + 4); }
 }  // namespace
 
-size_t trop_multi_scratch_bytes(int glo_ni, int nj) {
+size_t trop_multi_state_bytes(int glo_ni, int nj) {
   const size_t pn = (size_t)(glo_ni + 4) * nj, n2 = (size_t)(glo_ni + 2) * nj;
+  return (2 * M_STATE * pn + n2) * sizeof(double2);
+}
+
+size_t trop_multi_scratch_bytes(int glo_ni, int nj) {
+  const size_t pn = (size_t)(glo_ni + 4) * nj;
   size_t by_shape = 0;  // metric vectors and tile list
 #define PCOM_MULTI_SHAPE(x, y)                                                                                   \
   by_shape = std::max(by_shape, (xm_doubles(glo_ni, (x)) + ym_doubles(nj, (y))) * sizeof(double) +               \
                                     (size_t)((glo_ni + (x) - 1) / (x)) * ((nj + (y) - 1) / (y)) * sizeof(int));
   PCOM_MULTI_SHAPES(PCOM_MULTI_SHAPE)
 #undef PCOM_MULTI_SHAPE
-  return ((M_COUNT + 2 * M_STATE) * pn + n2) * sizeof(double2) + by_shape;
+  return M_COUNT * pn * sizeof(double2) + by_shape;
 }
 
-void trop_multi_bind(MultiTrop &M, void *scratch, int glo_ni, int nj, int TX, int TY) {
-  const size_t pn = (size_t)(glo_ni + 4) * nj, n2 = (size_t)(glo_ni + 2) * nj;
+void trop_multi_bind(MultiTrop &M, void *state, void *scratch, int glo_ni, int nj, int TX, int TY) {
+  const size_t pn = (size_t)(glo_ni + 4) * nj;
   M.pitch = glo_ni + 4;
-  double2 *v = (double2 *)scratch;  // every part starts on 16 bytes
-  M.cf = v; v += M_COUNT * pn;
-  M.st[0] = v; v += M_STATE * pn;
-  M.st[1] = v; v += M_STATE * pn;
-  M.acc = v; v += n2;
-  M.xm = (double *)v;
+  M.st[0] = (double2 *)state;  // every part starts on 16 bytes
+  M.st[1] = M.st[0] + M_STATE * pn;
+  M.acc = M.st[1] + M_STATE * pn;
+  M.cf = (double2 *)scratch;
+  M.xm = (double *)(M.cf + M_COUNT * pn);
   M.ym = M.xm + xm_doubles(glo_ni, TX);
   M.tiles = (int *)(M.ym + ym_doubles(nj, TY));
 }

@@ -361,8 +361,10 @@ struct pcom_handle {
   bool trop_resident = false;
   // domains too large for the resident kernel: the multi-tile kernels
   bool trop_multi = false;
-  // FP64: packed coefficients and the state between substeps
+  // FP64: packed coefficients, and the state between substeps (over tr_ch,
+  // tr_ub, tr_vb, tr_acc[2..5], which this form does not use)
   unsigned char *ms_scratch = nullptr;
+  double *tr_pool = nullptr;
   MultiTrop ms{};
   std::vector<int> ms_tiles;  // its tiles, those with sea first
   // mixed handles on the multi-tile path: FP32 coefficients and velocities
@@ -582,12 +584,12 @@ int pick_trop_config(pcom_handle *h) {
   }
       PCOM_MULTI_SHAPES(PCOM_TRY_SHAPE)
 #undef PCOM_TRY_SHAPE
-      if (trop_multi_max_blocks(bx, by) > 0) {
-        if (!h->ms_scratch) {
-          int rc = h->alloc(&h->ms_scratch, trop_multi_scratch_bytes(G, nj));
-          if (rc) return rc;
-        }
-        trop_multi_bind(h->ms, h->ms_scratch, G, nj, bx, by);
+      // (no memory left for the packed coefficients: the generic kernel below,
+      // which needs none)
+      if (trop_multi_max_blocks(bx, by) > 0 && !h->ms_scratch && h->alloc(&h->ms_scratch, trop_multi_scratch_bytes(G, nj)))
+        cudaGetLastError();
+      if (trop_multi_max_blocks(bx, by) > 0 && h->ms_scratch) {
+        trop_multi_bind(h->ms, h->tr_pool, h->ms_scratch, G, nj, bx, by);
         h->ms.nwet = bw;
         CK(cudaMemcpyAsync(h->ms.tiles, h->ms_tiles.data(), h->ms_tiles.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
         h->trop_multi = true;
@@ -616,7 +618,7 @@ int pick_trop_config(pcom_handle *h) {
         const int r0 = n % ((G + tx - 1) / tx) * tx, j0 = n / ((G + tx - 1) / tx) * ty + 1;
         t.push_back({0, r0, j0, std::min(tx, G - r0), std::min(ty, nj - j0 + 1)});
       }
-      int rc = h->alloc(&h->d_tiles1, t.size());
+      int rc = h->d_tiles1 ? PCOM_OK : h->alloc(&h->d_tiles1, t.size());  // (as many tiles in every pick)
       if (rc) return rc;
       CK(cudaMemcpy(h->d_tiles1, t.data(), t.size() * sizeof(TileRef), cudaMemcpyHostToDevice));
       h->ntiles1 = (int)t.size();
@@ -646,6 +648,15 @@ int pick_trop_config(pcom_handle *h) {
   }
   if (h->trop_blocks <= 0) return fail(PCOM_ERR_CUDA, "no launchable configuration for the barotropic kernel");
   return PCOM_OK;
+}
+
+// the choice, its memory and tile list ahead of the first step: in the step
+// they cost a new 1440 x 640 model 2 to 19 ms between two of its launches.
+// Where no form fits, the step picks again and reports it
+void plan_trop(pcom_handle *h) {
+  h->trop_blocks = 0;
+  if (pick_trop_config(h) != PCOM_OK) h->trop_blocks = 0;
+  cudaGetLastError();  // what the probing left (an allocation or a tile shape that does not fit)
 }
 
 // ---- the pieces of the step (FP64 handle: D; mixed handle: DM)
@@ -1152,8 +1163,17 @@ int pcom_gpu_create(const pcom_dims *dims, pcom_handle **out) {
   for (int q = 0; q < 4; ++q) { A(&D.bphi[q], n2); A(&D.bgra[q], n2); }
   A(&D.sch_r, n2); A(&D.sch_w, n2);
   A(&D.acch, n2); A(&D.acssh, n2);
-  for (int q = 0; q < 2; ++q) { A(&D.tr_ch[q], n2); A(&D.tr_ub[q], n2); A(&D.tr_vb[q], n2); }
-  for (int q = 0; q < 6; ++q) A(&D.tr_acc[q], n2);
+  A(&D.tr_acc[0], n2); A(&D.tr_acc[1], n2);
+  // (ten planes and 16 nj)
+  A(&h->tr_pool, (long long)(trop_multi_state_bytes(d.glo_ni, d.nj) / sizeof(double)));
+  if (!rc) {
+    double *t = h->tr_pool;
+    for (double **f : {&D.tr_ch[0], &D.tr_ch[1], &D.tr_ub[0], &D.tr_ub[1], &D.tr_vb[0], &D.tr_vb[1], &D.tr_acc[2],
+                       &D.tr_acc[3], &D.tr_acc[4], &D.tr_acc[5]}) {
+      *f = t;
+      t += n2;
+    }
+  }
   A(&D.am1, n2);
   if (h->mixed) {
     D.am = D.am1;  // the barotropic kernel reads am at level 1 only
@@ -1299,7 +1319,7 @@ int pcom_gpu_upload_static(pcom_handle *h, const pcom_static *s) {
       if (rc) return rc;
     }
     D.separable = 1;
-    h->trop_blocks = 0;  // re-pick the barotropic kernel configuration
+    h->trop_blocks = 0;  // planned below
     // smag's dy (j) and dx (i, j) (mod_int.f90:416-418) and their reciprocals
     const double *dx2 = s->dx[1], *dx4 = s->dx[3], *rh4 = s->rh[3];
     for (int j = 0; j < nj; ++j) v[j] = (j + 1 < nj) ? a * (dx2[2 * ((long long)ni * j) + 1] + dx2[2 * ((long long)ni * (j + 1)) + 1]) : 1.0;
@@ -1360,6 +1380,7 @@ int pcom_gpu_upload_static(pcom_handle *h, const pcom_static *s) {
   (void)ni; (void)nj;
   sync_common(h);
   h->static_ok = true;
+  plan_trop(h);
   return PCOM_OK;
 }
 
@@ -1746,7 +1767,8 @@ int pcom_gpu_set_trop_kernel(pcom_handle *h, int32_t which) {
   if (!h || which < 0 || which > 3) return fail(PCOM_ERR_ARG, "which must be 0..3");
   CK(cudaStreamSynchronize(h->stream));
   h->trop_force = which;
-  h->trop_blocks = 0;  // re-pick at the next step
+  h->trop_blocks = 0;
+  if (h->static_ok) plan_trop(h);
   return PCOM_OK;
 }
 

@@ -87,7 +87,9 @@ int trop_batch_max_blocks(int TX, int TY);
 cudaError_t launch_trop_batch(const Dev *dPs, const TileRef *dtiles, int ntiles, int TX, int TY, int nblocks,
                               unsigned long long *cnt, int *err, cudaStream_t s);
 // one FP64 domain with more tiles than SMs (k_trop_multi.cu): tile shapes it
-// is compiled for, and its scratch, which the handle allocates
+// is compiled for, and its memory, which the handle allocates: the state and
+// sums of its launches (they lie over planes of the other forms), the packed
+// coefficients and the tile list
 #define PCOM_MULTI_SHAPES(S) S(24, 14) S(20, 16) S(28, 12)
 struct MultiTrop {
   int pitch;                       // columns of the packed grid: glo_ni and two wrapped ones at each end
@@ -96,8 +98,9 @@ struct MultiTrop {
   double *xm, *ym;                 // metric vectors of every tile column and row
   int *tiles, nwet;                // tile numbers (row * columns + column): those with sea (nwet), those without
 };
+size_t trop_multi_state_bytes(int glo_ni, int nj);
 size_t trop_multi_scratch_bytes(int glo_ni, int nj);
-void trop_multi_bind(MultiTrop &M, void *scratch, int glo_ni, int nj, int TX, int TY);
+void trop_multi_bind(MultiTrop &M, void *state, void *scratch, int glo_ni, int nj, int TX, int TY);
 int trop_multi_max_blocks(int TX, int TY);
 cudaError_t launch_trop_multi(const Dev &P, const MultiTrop &M, int TX, int TY, int nblocks, unsigned long long *cnt,
                               cudaStream_t s);
