@@ -48,8 +48,11 @@ int pcom_model_destroy(pcom_model *m);
 pcom_handle *pcom_model_handle(pcom_model *m);
 /* n passes of the time loop body (main.f90:158-238, without output()).  The
  * steps are enqueued one behind the other and awaited before the call
- * returns; a device-side failure (PCOM_ERR_TIMEOUT) is reported by the next
- * wait, after the steps enqueued behind it. */
+ * returns.  A device-side failure (PCOM_ERR_TIMEOUT) is reported by the next
+ * wait (the call's last, or a model day's first), after the steps enqueued
+ * behind it: they have run on a state that is no longer meaningful, and their
+ * terms are in the accumulators.  pcom_model_iter and pcom_model_date then
+ * give the step that failed. */
 int pcom_model_run(pcom_model *m, int64_t nsteps);
 /* One pass split open, for drivers that put their own work between the
  * subroutines of the step (the halo exchanges of a domain split into row

@@ -46,7 +46,7 @@ __device__ bool grid_barrier(const Dev &P, unsigned nblocks) {
         long long it = 0;
         while (gen.load(cuda::memory_order_acquire) == g) {
           if (++it > kSpinLimit || err.load(cuda::memory_order_relaxed) != 0 || global_ns() - t0 > P.wait_ns) {
-            err.store(1, cuda::memory_order_relaxed);
+            give_up(P.err, P.err_step);
             fail = 1;
             break;
           }
@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(fast_threads<GROUP, CTX, CTY>(), 1)
     if (ring) {
       const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : out, inS2 ? out + 2 * P.n2 : out};
       double v[3] = {0.0, 0.0, 0.0};
-      fail = !xch_wait(in, seq + nt, v, err, P.wait_ns);
+      fail = !xch_wait(in, seq + nt, v, err, P.wait_ns, GROUP ? 1 : P.err_step);
       s.c0 = v[0];
       s.u0 = v[1];
       s.v0 = v[2];
@@ -912,7 +912,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (ring) {
       const ulonglong2 *const in[3] = {out, inS2 ? out + P.n2 : out, inS2 ? out + 2 * P.n2 : out};
       double v[3] = {0.0, 0.0, 0.0};
-      fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns);
+      fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns, P.err_step);
       S(X_CH, p) = v[0];
       if (inS2) { S(X_UB, p) = v[1]; S(X_VB, p) = v[2]; }
     }

@@ -35,7 +35,7 @@ __device__ bool batch_barrier(unsigned long long *cnt, unsigned long long want, 
     // release: cumulative over the CTA's writes ordered before it by bar.sync
     cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> c(*cnt);
     c.fetch_add(1ULL, cuda::memory_order_release);
-    s_fail = wait_count(cnt, want, err, limit_ns) ? 0 : 1;
+    s_fail = wait_count(cnt, want, err, limit_ns, 1) ? 0 : 1;
   }
   __syncthreads();
   return s_fail == 0;

@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (ring) {
       const ulonglong2 *const in[2] = {out, inS2 ? out + P.n2 : out};
       double v[2] = {0.0, 0.0};
-      fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns);
+      fail = !xch_wait(in, seq + nt, v, P.err, P.wait_ns, P.err_step);
       c0 = v[0];
       unpack_uv(v[1], u0, v0);
       SD(D_CH, 0) = c0;

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__((ms_threads<TX, TY>()), 1)
     if (tid == 0) {
       cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> c(*cnt);
       c.fetch_add(1ULL, cuda::memory_order_release);
-      s_stop = wait_count(cnt, (unsigned long long)nt * gridDim.x, P.err, P.wait_ns) ? 0 : 1;
+      s_stop = wait_count(cnt, (unsigned long long)nt * gridDim.x, P.err, P.wait_ns, P.err_step) ? 0 : 1;
       if (!s_stop) {
         fence_proxy();
         if (nt == 1) fetch_c(tx, ty, b);
@@ -351,10 +351,7 @@ __global__ void __launch_bounds__((ms_threads<TX, TY>()), 1)
     }
     finish(i, q, am1, am2, auv);
   }
-  if (!ok && tid == 0) {
-    cuda::atomic_ref<int, cuda::thread_scope_device> e(*P.err);
-    e.store(1, cuda::memory_order_relaxed);
-  }
+  if (!ok && tid == 0) give_up(P.err, P.err_step);
 }
 
 namespace {

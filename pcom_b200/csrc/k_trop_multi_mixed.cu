@@ -36,13 +36,13 @@ enum {                                       // FP32 region fields
 
 __device__ __forceinline__ void prefetch_l2(const void *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 
-__device__ bool grid_barrier(unsigned long long *cnt, unsigned long long want, int *err, unsigned long long limit_ns) {
+__device__ bool grid_barrier(unsigned long long *cnt, unsigned long long want, int *err, unsigned long long limit_ns, int step) {
   __syncthreads();
   __shared__ int s_fail;
   if (threadIdx.x == 0) {
     cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> c(*cnt);
     c.fetch_add(1ULL, cuda::memory_order_release);
-    s_fail = wait_count(cnt, want, err, limit_ns) ? 0 : 1;
+    s_fail = wait_count(cnt, want, err, limit_ns, step) ? 0 : 1;
   }
   __syncthreads();
   return s_fail == 0;
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kThreads) k_trop_multi_mixed(const __grid_cons
 #undef STAGE
       __syncthreads();
     }
-    if (!grid_barrier(cnt, (unsigned long long)nt * gridDim.x, err, P.wait_ns)) return;
+    if (!grid_barrier(cnt, (unsigned long long)nt * gridDim.x, err, P.wait_ns, P.err_step)) return;
   }
 
   // averages (mod_int.f90:276-288)

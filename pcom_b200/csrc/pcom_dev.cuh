@@ -77,10 +77,11 @@ struct DevCommon {
   // substeps deep: xch[(2-parity * 3 + field) * n2 + point]; null on domains
   // too large to be resident
   ulonglong2 *xch;
-  int *err;        // [0] timeout flag, [1] watchdog flag
+  int *err;        // [0] the first step a wait gave up in (err_step), [1] watchdog flag
   // longest a device-side wait (the barotropic kernels' messages and grid barriers) may
-  // take before it gives up and sets err[0] (ns of global time)
+  // take before it gives up and sets err[0] to err_step (ns of global time)
   unsigned long long wait_ns = 2000000000ULL;
+  int err_step = 1;
   // lat-lon (separable) metrics: dx?x depends on i only, dx?y and rh? on j
   // only (set_hgrid builds them from 1-D lon/lat, main.f90:408-493); when the
   // uploaded 2-D arrays have that structure these 1-D copies are set
@@ -151,11 +152,18 @@ PD unsigned long long global_ns() {
   return t;
 }
 
+// *err = step, unless it is set already (the steps enqueued behind one that
+// failed fail as well)
+PD void give_up(int *err, int step) {
+  int none = 0;
+  cuda::atomic_ref<int, cuda::thread_scope_device>(*err).compare_exchange_strong(none, step, cuda::memory_order_relaxed);
+}
+
 // One thread's bounded wait for an arrival counter to reach `want`: gives up
 // when another thread has set *err, or after limit_ns of global time (then
-// it sets *err itself; an iteration cap bounds the loop as well).  Returns
-// true when the counter got there.
-PD bool wait_count(unsigned long long *cnt, unsigned long long want, int *err, unsigned long long limit_ns) {
+// it sets *err to step itself; an iteration cap bounds the loop as well).
+// Returns true when the counter got there.
+PD bool wait_count(unsigned long long *cnt, unsigned long long want, int *err, unsigned long long limit_ns, int step) {
   cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> c(*cnt);
   cuda::atomic_ref<int, cuda::thread_scope_device> e(*err);
   if (c.load(cuda::memory_order_acquire) >= want) return true;
@@ -166,7 +174,7 @@ PD bool wait_count(unsigned long long *cnt, unsigned long long want, int *err, u
     if (global_ns() - t0 > limit_ns) break;
     if (it > 1024) __nanosleep(32);
   }
-  e.store(1, cuda::memory_order_relaxed);
+  give_up(err, step);
   return false;
 }
 
@@ -190,13 +198,13 @@ PD void xch_get(const ulonglong2 *a, double &v, unsigned long long &seq) {
 }
 // One thread's bounded wait for the N messages at a[0 .. N-1]: false when
 // another thread has set *err or after limit_ns of global time (then *err is
-// set; an iteration cap bounds the loop as well).  Every poll issues its N
+// set to step; an iteration cap bounds the loop as well).  Every poll issues its N
 // loads back to back: with a branch around each (messages some threads do
 // not need) a poll took N round trips; predicated loads of the missing ones
 // only were slower too (1 degree FP64 475 -> 521 us).
 template <int N>
 PD bool xch_wait(const ulonglong2 *const (&a)[N], unsigned long long seq, double (&v)[N], int *err,
-                 unsigned long long limit_ns) {
+                 unsigned long long limit_ns, int step) {
   cuda::atomic_ref<int, cuda::thread_scope_device> e(*err);
   unsigned long long t0 = 0;
   for (int it = 0; it < (1 << 26); ++it) {
@@ -213,7 +221,7 @@ PD bool xch_wait(const ulonglong2 *const (&a)[N], unsigned long long seq, double
       if (e.load(cuda::memory_order_relaxed) != 0) return false;
     }
   }
-  e.store(1, cuda::memory_order_relaxed);
+  give_up(err, step);
   return false;
 }
 

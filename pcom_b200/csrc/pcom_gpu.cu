@@ -20,6 +20,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/pcom_gpu.h"
@@ -375,6 +376,7 @@ struct pcom_handle {
   int ntiles1 = 0, nwet1 = 0;
   unsigned long long *d_cnt1 = nullptr;
   double *frc_months = nullptr;  // taux, tauy, t, s, pa: [5][12][nj][ni]
+  int failed_step = 0;  // the step the last timeout was in (pcom_failed_step)
   unsigned long long trop_seq = 0;  // sequence base of the next resident barotropic launch (message_space)
   // second stream of the full step: phases that share no array with the
   // main stream's concurrent phases run on it, forked and joined by events
@@ -462,7 +464,8 @@ int sync_check(pcom_handle *h) {
     cudaMemsetAsync(h->D.err, 0, sizeof err, h->stream);
     cudaMemsetAsync(h->D.bar, 0, 2 * sizeof(unsigned), h->stream);
     cudaStreamSynchronize(h->stream);
-    return fail(PCOM_ERR_TIMEOUT, "a device-side wait of a barotropic kernel gave up (bounded spin)");
+    h->failed_step = err[0];
+    return fail(PCOM_ERR_TIMEOUT, "a device-side wait of a barotropic kernel gave up in step %d (bounded spin)", err[0]);
   }
   return PCOM_OK;
 }
@@ -796,6 +799,7 @@ int do_ts(pcom_handle *h, bool with_2d = true) {
 }
 
 int run_phase(pcom_handle *h, int phase, int64_t iter) {
+  h->D.err_step = (int)std::min<int64_t>(std::max<int64_t>(iter, 1), INT32_MAX);
   switch (phase) {
   case 0: return do_den_alpha(h);
   case 1: return do_pgra(h);
@@ -837,6 +841,7 @@ int enqueue_step(pcom_handle *h, int64_t iter) {
   //    and int_trop only) beside int_ssh and int_ts; joined at the end of
   //    the step.
   int rc;
+  h->D.err_step = (int)std::min<int64_t>(iter, INT32_MAX);
   CK(cudaEventRecord(h->ev_fork[0], h->stream));
   CK(cudaStreamWaitEvent(h->side, h->ev_fork[0], 0));
   if ((rc = do_readyc_2d(h, h->side))) return rc;
@@ -1872,6 +1877,8 @@ void pcom_dev_consts(bool r8, DevConsts &c) { make_consts(r8, c); }
 
 // record a failure for pcom_gpu_last_error from another translation unit
 int pcom_set_error(int code, const char *msg) { return fail(code, "%s", msg); }
+// the step in which the last reported timeout happened, once (0: none since)
+long long pcom_failed_step(pcom_handle *h) { return std::exchange(h->failed_step, 0); }
 
 // =============================================================== batches
 // Ensemble members and basins of uneven size stepped together: every kernel

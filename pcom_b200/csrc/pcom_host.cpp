@@ -6,6 +6,7 @@
 // functions (cos/tan/sin) and a fixed-point iteration; it is computed here in
 // FP64 with the reference's evaluation order and literal precision, and its
 // outputs are uploaded as the static data of the device step.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -15,6 +16,7 @@
 #include "../../include/pcom_host.h"
 
 int pcom_set_error(int code, const char *msg);  // pcom_gpu.cu
+long long pcom_failed_step(pcom_handle *h);
 
 namespace {
 
@@ -462,8 +464,11 @@ int pcom_model_run(pcom_model *M, int64_t nsteps) {
   // the steps are enqueued without waiting and awaited once at the end (the
   // daily calls wait too): a wait per step left the GPU idle for its round
   // trip and for the next step's first launches.  A step that fails is
-  // reported by the wait that follows it
+  // reported by the wait that follows it, and the model's clock goes back to it
   int rc = PCOM_OK;
+  const long long iter0 = M->iter, nday0 = M->nday;
+  const Date ct0 = M->ct, pt0 = M->pt;
+  pcom_failed_step(M->h);
   for (int64_t n = 0; n < nsteps && !rc; ++n) {
     int64_t it = 0;
     int32_t day = 0;
@@ -476,9 +481,22 @@ int pcom_model_run(pcom_model *M, int64_t nsteps) {
     char msg[512] = {0};
     pcom_gpu_last_error(msg, sizeof msg);
     pcom_gpu_sync(M->h);
-    return pcom_set_error(rc, msg);
+    pcom_set_error(rc, msg);
+  } else {
+    rc = pcom_gpu_sync(M->h);
   }
-  return pcom_gpu_sync(M->h);
+  if (const long long failed = pcom_failed_step(M->h)) {
+    // as if the run had stopped there: that step begun, none ended since
+    const long long last = std::min(std::max(failed, iter0 + 1), M->iter);
+    M->iter = iter0; M->nday = nday0; M->ct = ct0; M->pt = pt0;
+    for (;;) {
+      M->iter += 1;
+      if (M->iter == 1 || M->ct.d != M->pt.d) M->nday += 1;
+      if (M->iter >= last) break;
+      pcom_model_end_step(M);
+    }
+  }
+  return rc;
 }
 
 int pcom_model_run_batch(pcom_model *const *ms, int32_t n, pcom_batch *b, int64_t nsteps) {

@@ -45,6 +45,43 @@ def test_barrier_wait_runs_out_and_handle_recovers(form, mixed):
     ref.close()
 
 
+@pytest.mark.parametrize("form,mixed", [(1, False), (2, False), (3, False), (1, True), (2, True)])
+def test_run_of_several_steps_stops_its_clock_at_the_failed_one(form, mixed):
+    """A run enqueues its steps and waits at the end and once a model day: a
+    timeout in its third step leaves the model's clock there, with steps
+    enqueued behind it and over the day's end, and the handle usable."""
+    c = make_case("box")
+    flags = L.PCOM_PREC_MIXED if mixed else L.PCOM_PREC_FP64
+
+    def model():
+        m = Model(c, flags=flags)
+        L.check(m.lib.pcom_gpu_set_trop_kernel(m.handle, form), "set_trop_kernel")
+        return m
+
+    ref = model()
+    ref.run(3)
+    m = model()
+    m.run(2)
+    date = m.date
+    L.check(m.lib.pcom_gpu_set_wait_limit(m.handle, 1e-9), "set_wait_limit")
+    for iteration, steps in ((3, 5), (4, 40)):  # 24 steps are a day
+        with pytest.raises(L.PcomError) as ei:
+            m.run(steps)
+        assert "TIMEOUT" in str(ei.value)
+        assert m.iter == iteration and m.date == date  # that step begun, not ended
+    L.check(m.lib.pcom_gpu_set_wait_limit(m.handle, 2.0), "set_wait_limit")
+    m.run(2)
+    m.close()
+
+    f = model()
+    f.run(3)
+    for name in STATE_FIELDS:
+        r = compare(f.field(name), ref.field(name))
+        assert r["unequal"] == 0, f"{name} differs after a timeout in the same process"
+    f.close()
+    ref.close()
+
+
 def test_wait_limit_rejects_bad_values():
     m = Model(make_case("tiny"))
     for bad in (-1.0, float("nan"), 1e7):
