@@ -28,6 +28,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <type_traits>
@@ -970,9 +971,8 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_tc(const __nv_bfloat16 *__re
 // lying in adjacent slots of the g ring (two MMAs where the ring wraps), and
 // the column taps are row blocks of A: the same pixels one pixel further on,
 // i.e. a leading byte offset of one pixel.  All 9 taps accumulate in tensor
-// memory for the whole run (64 channels: D1 = taps dx -1, 0 on 128 lanes, D2
-// tensor memory (64 channels: D1 = taps dx -1, 0 on 128 lanes, D2 = tap dx +1
-// on 64).  D2's other 64 lanes take a constant block of ones as A, so that its
+// memory (64 channels: D1 = taps dx -1, 0 on 128 lanes, D2 = tap dx +1 on
+// 64).  D2's other 64 lanes take a constant block of ones as A, so that its
 // middle column block is the bias gradient.
 //
 // Sums: tensor memory adds truncate (a chain of n adds of 16-pixel products
@@ -1448,6 +1448,15 @@ cudaError_t conv_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const f
   return cudaGetLastError();
 }
 
+// pixels per CTA of the pixel split (k_wgrad_tc): about 4 waves of CTAs, a
+// multiple of 64
+template <int CIN>
+long long wgrad_chunk(long long npix, int nsm) {
+  constexpr int TPT = kM / CIN, ytiles = (9 + TPT - 1) / TPT;
+  const long long target = std::max(1LL, (long long)nsm * 8 / ytiles);
+  return std::max(64LL, ((npix + target - 1) / target + 63) / 64 * 64);
+}
+
 template <int CIN, int NOUT>
 cudaError_t wgrad_rows_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *dw, float *db, long long npix,
                               int H, int W, int periodic_x, int *err, cudaStream_t s) {
@@ -1466,14 +1475,23 @@ cudaError_t wgrad_rows_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, f
   const int tmem_cap = 512 / (int)wg_cols<CIN, NOUT>();
   per = per < 1 ? 1 : (per > tmem_cap ? tmem_cap : per);
   const long long ntiles = (long long)NR * ((W + kM - 1) / kM);
-  const long long grid = ntiles < (long long)nsm * per ? ntiles : (long long)nsm * per;
+  // The sums' error is held to the pixel split's (below), whose sums are one
+  // chain of a chunk's pixels: no longer a chain of truncating adds (a row is
+  // 128 pixels; 16 rows at most, 3 where a CTA has only a few), and no more
+  // CTAs whose sums meet in dw (on toy images).
+  // 30 images of 360 x 160: 165 us for a 64 -> 64 layer (ncu) against 1,136 us
+  // of the pixel split (which reads both activations 5 times) and 118 us of
+  // the bias gradient's own pass.  Relative error against 64 bits, rms over a
+  // layer, beside the pixel split's: 64 -> 64 0.8e-6 (3.7e-6), 16 -> 64 1.4e-6
+  // (2.3e-6); 36 of 200 x 100 0.7e-6 (1.3e-6), 0.7e-6 (0.9e-6; 1.2e-6 with a
+  // flush every 16 rows); 12 of 131 x 67 2.0e-7 (3.1e-7); 8 of 14 x 12 8e-8
+  // (9e-8; 11e-8 with a CTA per row).  The bias gradient, beside FP32 sums
+  // rounded to nearest: 2.7e-7 (8.2e-7), 2.2e-7 (7.7e-7), 1.4e-7 (2.6e-7),
+  // 1.6e-8 (1.9e-8).
+  const long long chunk = wgrad_chunk<CIN>(npix, nsm);
+  const long long grid = std::min({ntiles, (long long)nsm * per, (npix + chunk - 1) / chunk});
   if (grid < 1) return cudaSuccess;
-  // a flush every 16 rows (chains of 128 adds, 2e-6 short) on long runs, every 3
-  // where a CTA has only a few.  30 images of 360 x 160: 165 us for a 64 -> 64
-  // layer (ncu) against 1,136 us of the per-tap form below (which reads both
-  // activations 5 times) and 118 us of the bias gradient's own pass; relative
-  // error against 64 bits 2e-6 (8e-6); 12 images of 131 x 67: 3.6e-7 (5.0e-7)
-  const int flush = ntiles >= 32 * grid ? 16 : 3;
+  const int flush = ntiles >= 32 * grid ? (int)std::min(16LL, std::max(3LL, chunk / kM)) : 3;
   k_wgrad_rows<CIN, NOUT><<<(unsigned)grid, kWgThreads, sm, s>>>(in, dw, db, (int)nimg, H, W, periodic_x, flush, err, tin,
                                                                  tg);
   return cudaGetLastError();
@@ -1493,15 +1511,10 @@ cudaError_t wgrad_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float 
   if (e != cudaSuccess) return e;
   constexpr int TPT = kM / CIN;
   const int ytiles = (9 + TPT - 1) / TPT;
-  // split K over about 4 waves of CTAs; pixels per CTA a multiple of 64
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  long long target = (long long)nsm * 8 / ytiles;
-  if (target < 1) target = 1;
-  long long ppc = (npix + target - 1) / target;
-  ppc = (ppc + 63) / 64 * 64;
-  if (ppc < 64) ppc = 64;
+  const long long ppc = wgrad_chunk<CIN>(npix, nsm);
   const unsigned gx = (unsigned)((npix + ppc - 1) / ppc);
   k_wgrad_tc<CIN, NOUT><<<dim3(gx, ytiles), kThreads, sm, s>>>(in, g, dw, npix, H, W, periodic_x, ppc, err);
   return cudaGetLastError();

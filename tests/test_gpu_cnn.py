@@ -169,6 +169,35 @@ def test_wgrad_edge_shapes(cin, nout, px, h, w, nimg):
     assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
+# where the row form's sums could be longer than the pixel split's: rows of
+# toy images one CTA each, and runs just long enough for the longest chains
+@pytest.mark.parametrize("h,w,nimg", [(12, 14, 8), (100, 200, 36), (140, 290, 16)])
+@pytest.mark.parametrize("cin,nout", [(16, 64), (64, 16)])
+def test_wgrad_rows_as_accurate_as_pixel_split(cin, nout, h, w, nimg):
+    """Whole images take the row form, a count of pixels that is not whole
+    images the pixel split: the same images with one more pixel of gradient
+    zero.  The row form's rms distance from 64 bits is no larger; 10 % are
+    allowed for the order of the FP32 atomics, which moves either by 3 %."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(h + w + cin)
+    npix = h * w * nimg
+    x = torch.randn((npix + 1, cin), generator=gen, device="cuda").bfloat16()
+    g = torch.randn((npix + 1, nout), generator=gen, device="cuda").bfloat16()
+    g[npix] = 0
+    xi = x[:npix].double().view(nimg, h, w, cin)
+    xi = torch.nn.functional.pad(torch.cat([xi[:, :, -1:], xi, xi[:, :, :1]], 2), (0, 0, 0, 0, 1, 1))
+    ref = torch.stack([g[:npix].double().T @ xi[:, t // 3:t // 3 + h, t % 3:t % 3 + w].reshape(npix, cin)
+                       for t in range(9)])
+    err = []
+    for n in (npix, npix + 1):
+        dw = torch.zeros(9 * nout * cin, dtype=torch.float32, device="cuda")
+        cnn_check(L.load().pcom_cnn_wgrad_layer(cin, nout, x.data_ptr(), g.data_ptr(), dw.data_ptr(), n, h, w, 1,
+                                                C.c_void_p(torch.cuda.current_stream().cuda_stream)), "wgrad")
+        err.append(float((dw.double().view_as(ref) - ref).norm() / ref.norm()))
+    assert err[0] <= 1.1 * err[1], f"rows {err[0]:.2e}, pixel split {err[1]:.2e}"
+
+
 # the 1-degree closure's images: one 160 x 360 level image per model level,
 # periodic in x (the production row walk of the persistent kernel)
 HF, WF, NF = 160, 360, 2
@@ -299,6 +328,34 @@ def test_bias_gradient_and_loss(h, w, nimg, off):
         b = slice(o + 9 * n * k, o + 9 * n * k + n)
         assert np.linalg.norm(g[b] - gref[b]) <= 2e-2 * np.linalg.norm(gref[b]), f"bias of the {k} -> {n} layer"
         o += 9 * n * k + n
+    lib.pcom_cnn_destroy(hn)
+
+
+@pytest.mark.parametrize("h,w,nimg", [(12, 14, 8), (67, 131, 12), (100, 200, 36)])
+def test_bias_gradient_sums(h, w, nimg):
+    """The last layer's bias gradient is the sum of a gradient image that the
+    network's output gives exactly: g = bf16(2 / count (y - t) mask).  With y
+    above t everywhere no sum cancels, and 128 truncating adds of a chain and
+    148 CTAs' atomics lose at most (128 x 2 + 148) x 2^-24 of it."""
+    import torch
+
+    lib = L.load()
+    par, x, t, m = _problem(h, nimg, h, w)
+    hn = _net(lib, nimg, h, w)
+    cnn_check(lib.pcom_cnn_set_params(hn, par.ctypes.data, par.size), "set_params")
+    xd, _ = bf16(x)
+    y = torch.empty(t.shape, device="cuda")
+    cnn_check(lib.pcom_cnn_forward(hn, xd.data_ptr(), y.data_ptr(), nimg), "forward")
+    td = y - 0.5 - torch.from_numpy(np.abs(t)).cuda()
+    md = torch.from_numpy(m).cuda()
+    grad = np.zeros(par.size, np.float32)
+    loss = C.c_double()
+    cnn_check(lib.pcom_cnn_gradient(hn, xd.data_ptr(), td.data_ptr(), md.data_ptr(), nimg, grad.ctypes.data,
+                                    C.byref(loss)), "gradient")
+    scale = np.float32(2.0 / float(md.double().sum()))
+    ref = ((y - td) * md * float(scale)).bfloat16().double().sum(0).cpu().numpy()
+    got = grad[-16:-12]
+    assert np.abs(got - ref).max() <= (256 + 148) * 2.0 ** -24 * np.abs(ref).max()
     lib.pcom_cnn_destroy(hn)
 
 
