@@ -125,6 +125,45 @@ def test_convective_adjustment(oracle_lib):
     m.close()
 
 
+@pytest.mark.parametrize("k", [4, 9, 14])
+def test_convective_adjustment_between_parts(oracle_lib, k):
+    """On small grids four threads share a column's levels; the box's 20 meet
+    below levels 5, 10 and 15.  Columns unstable there and nowhere else are
+    mixed as the oracle mixes them, bit for bit."""
+    c, pick = _unstable_case(k=k)
+    assert pick.sum() > 100 and (c["itn"][pick] == 20).all()
+    o = oracle_lib.Oracle(c)
+    m = Model(c)
+    m.run(1)
+    o.step(1)
+    tc = o.field("tc")[:, 1:-1, 1:-1]
+    assert (tc[k] == tc[k + 1])[pick].mean() > 0.9, "convect did not mix the planted columns"
+    _check(m, o, STATE_FIELDS + ["acr"], m.static()["lev_t"], c["nk"], f"box unstable between levels {k + 1}, {k + 2}")
+    m.close()
+
+
+def _levels_case(nk):
+    """A small basin whose columns have bottoms of their own."""
+    ni, nj = 45, 13
+    c = make_case("basin", glo_ni=ni, glo_nj=nj, nk=nk)
+    itn = np.where(c["itn"] > 0, np.random.default_rng(nk).integers(1, nk + 1, c["itn"].shape), 0).astype(np.int32)
+    itn[3:6, 20:] = 0
+    itn[7, :30] = np.minimum(itn[7, :30], 1)
+    return dict(c, itn=itn)
+
+
+@pytest.mark.parametrize("nk", [2, 3, 7])
+def test_few_levels(oracle_lib, nk):
+    """A column's levels shared by four threads of which some get none."""
+    c = _levels_case(nk)
+    o = oracle_lib.Oracle(c)
+    m = Model(c)
+    m.run(4)
+    o.step(4)
+    _check(m, o, STATE_FIELDS + ["acr"], m.static()["lev_t"], nk, f"{nk} levels")
+    m.close()
+
+
 def test_multi_tile_domain_picked_automatically(oracle_lib):
     """720 x 320 x 30 (0.5 degree) has more barotropic tiles than the GPU
     holds one per CTA: the automatic choice is the multi-tile kernel (forcing
