@@ -1403,6 +1403,12 @@ static inline int wrows(const DevT<R> &P) { return P.j_hi - P.j_lo + 1; }
 static inline size_t sm3(int nk, int planes) { return (size_t)planes * nk * TB_X * sizeof(double); }
 // k_clin: four level planes (column-sum terms, new u and v) and the two sums
 static inline size_t clin_smem(int nk) { return sm3(nk, 4) + 2 * TB_X * sizeof(double); }
+// 48 KB and more of shared memory (four planes of more than 48 levels) have to
+// be allowed per kernel
+template <class K>
+static cudaError_t allow_smem(K *kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 
 // The column kernels' threads per column: 4 while the grid's columns are about
 // what the SMs hold at once (2^17: 148 SMs x 384 threads x 2.3), where the time
@@ -1433,7 +1439,11 @@ static void launch_ts_col(const Dev &P, const Dev *Ps, int nx, int ny, int nz, c
 template <typename R>
 void launch_alpha_tobot(const DevT<R> &P, cudaStream_t s) { k_alpha_tobot<R, false><<<g3(P.ni, wrows(P), 1), kBlock3, sm3(P.nk, 1), s>>>(P, nullptr); }
 template <typename R>
-void launch_pgra2d(const DevT<R> &P, cudaStream_t s) { k_pgra2d<R, false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, sm3(P.nk, 4), s>>>(P, nullptr); }
+void launch_pgra2d(const DevT<R> &P, cudaStream_t s) {
+  static const cudaError_t attr = allow_smem(k_pgra2d<R, false>, sm3(PCOM_MAXK, 4));
+  (void)attr;
+  k_pgra2d<R, false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, sm3(P.nk, 4), s>>>(P, nullptr);
+}
 template <typename R>
 void launch_uv2d(const DevT<R> &P, int mode, cudaStream_t s) {
   k_uv2d<R, false><<<dim3((P.glo_ni + 31) / 32, (P.nj + 3) / 4), dim3(32, 4), 0, s>>>(P, nullptr, mode);
@@ -1454,8 +1464,7 @@ void launch_readyc3d(const DevT<R> &P, cudaStream_t s) {
 template <typename R>
 void launch_clin(const DevT<R> &P, cudaStream_t s) {
   const size_t smem = clin_smem(P.nk);
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_clin<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clin_smem(PCOM_MAXK));
+  static const cudaError_t attr = allow_smem(k_clin<R, false>, clin_smem(PCOM_MAXK));
   (void)attr;
   k_clin<R, false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, smem, s>>>(P, nullptr);
 }
@@ -1474,6 +1483,8 @@ void launch_ts(const DevT<R> &P, cudaStream_t s) {
     launch_ts_col<false>(P, nullptr, P.glo_ni, wrows(P), 1, s);
     k_ts_acc<false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, 0, s>>>(P, nullptr);
   } else {
+    static const cudaError_t attr = allow_smem(k_ts<R, false>, sm3(PCOM_MAXK, 4));
+    (void)attr;
     k_ts<R, false><<<g3(P.glo_ni, wrows(P), 1), kBlock3, sm3(P.nk, 4), s>>>(P, nullptr);
   }
 }
@@ -1501,7 +1512,12 @@ void launch_batch(int kernel, const Dev *dPs, const BatchShape &b, int arg, cuda
   const int n = b.n;
   switch (kernel) {
   case BK_ALPHA_TOBOT: k_alpha_tobot<double, true><<<g3(b.ni, b.nj, n), kBlock3, sm3(b.nk, 1), s>>>(none, dPs); break;
-  case BK_PGRA2D: k_pgra2d<double, true><<<g3(b.glo_ni, b.nj, n), kBlock3, sm3(b.nk, 4), s>>>(none, dPs); break;
+  case BK_PGRA2D: {
+    static const cudaError_t attr = allow_smem(k_pgra2d<double, true>, sm3(PCOM_MAXK, 4));
+    (void)attr;
+    k_pgra2d<double, true><<<g3(b.glo_ni, b.nj, n), kBlock3, sm3(b.nk, 4), s>>>(none, dPs);
+    break;
+  }
   case BK_UV2D: k_uv2d<double, true><<<dim3((b.glo_ni + 31) / 32, (b.nj + 3) / 4, n), dim3(32, 4), 0, s>>>(none, dPs, arg); break;
   case BK_UPWELLING: {
     constexpr int UX = upw_cols<double>();
@@ -1513,8 +1529,7 @@ void launch_batch(int kernel, const Dev *dPs, const BatchShape &b, int arg, cuda
     launch_readyc_col<true>(none, dPs, b.glo_ni, b.nj, b.nk, n, s);
     break;
   case BK_CLIN: {
-    static const cudaError_t attr = cudaFuncSetAttribute(k_clin<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)clin_smem(PCOM_MAXK));
+    static const cudaError_t attr = allow_smem(k_clin<double, true>, clin_smem(PCOM_MAXK));
     (void)attr;
     k_clin<double, true><<<g3(b.glo_ni, b.nj, n), kBlock3, clin_smem(b.nk), s>>>(none, dPs);
     break;

@@ -723,6 +723,7 @@ int do_readyc_3d(pcom_handle *h, int64_t iter) {
   return PCOM_OK;
 }
 int do_trop(pcom_handle *h) {
+  CK(cudaGetLastError());  // of the launches before: setting a kernel's attributes below forgets them
   if (h->trop_blocks <= 0) {
     int rc = pick_trop_config(h);
     if (rc) return rc;
@@ -2121,6 +2122,7 @@ int batch_enqueue(pcom_batch *b, Dev *dP) {
   launch_batch(BK_UV2D, dP, s, 0, st);
   launch_batch(BK_UPWELLING, dP, s, 0, st);
   launch_batch(BK_READYC3D, dP, s, 0, st);
+  CK(cudaGetLastError());  // as in do_trop
   cudaError_t e = batch_trop(b, dP);
   if (e != cudaSuccess) return fail(PCOM_ERR_CUDA, "batched barotropic launch: %s", cudaGetErrorString(e));
   launch_batch(BK_UV2D, dP, s, 2, st);

@@ -7,7 +7,8 @@ for the FP64 path (1e-12 relative per field) is asserted as well.
 import numpy as np
 import pytest
 
-from pcom_b200.model import PHASES, Model
+from pcom_b200 import _lib as L
+from pcom_b200.model import PHASES, Batch, Model
 from pcom_b200.synth import make_case
 from parity_util import PHASE_FIELDS, STATE_FIELDS, acr_mask, compare
 
@@ -162,6 +163,31 @@ def test_few_levels(oracle_lib, nk):
     o.step(4)
     _check(m, o, STATE_FIELDS + ["acr"], m.static()["lev_t"], nk, f"{nk} levels")
     m.close()
+
+
+@pytest.mark.parametrize("nk", [49, 63])
+def test_many_levels(oracle_lib, nk):
+    """More levels than 48 KB of shared memory hold, up to the most there are:
+    one domain, a batch of two, and the mixed form within its bound of T."""
+    c = _levels_case(nk)
+    o = oracle_lib.Oracle(c)
+    o.step(4)
+    ms = [Model(c) for _ in range(3)]
+    ms[0].run(4)
+    b = Batch(ms[1:])
+    b.run(4)
+    lev_t = ms[0].static()["lev_t"]
+    for q, m in enumerate(ms):
+        _check(m, o, STATE_FIELDS + ["acr"], lev_t, nk, f"{nk} levels, model {q}")
+    b.close()
+    mm = Model(c, flags=L.PCOM_PREC_MIXED)
+    mm.run(4)
+    mm.check_finite()
+    wet = lev_t[None] >= np.arange(1, nk + 1)[:, None, None]
+    t, t64 = mm.field("tc")[wet], ms[0].field("tc")[wet]
+    assert np.sqrt(np.mean((t - t64) ** 2) / np.mean(t64 ** 2)) <= 2e-6
+    for m in ms + [mm]:
+        m.close()
 
 
 def test_multi_tile_domain_picked_automatically(oracle_lib):
