@@ -27,7 +27,7 @@
 
 namespace {
 
-constexpr int kThreads = 512;
+constexpr int kThreads = 512, TX = kMixedMultiX, TY = kMixedMultiY;  // (a 36 x 14 region: 504 of the threads)
 enum { D_CH, D_PRED, D_CN, D_CE, D_COUNT };  // FP64 region fields
 enum {                                       // FP32 region fields
   F_UB, F_VB, F_S1, F_X2, F_SCHE, F_A1U, F_A1V, F_GY, F_A2U, F_A2V, F_GX, F_UBC, F_VBC,
@@ -77,13 +77,12 @@ __global__ void k_mm_prep(const __grid_constant__ Dev P, MultiMixed M) {
 
 // SKIP: the tiles from number nwet on are without sea (a form of its own: it
 // costs the other 1 %)
-template <bool SKIP, int CTX = 0, int CTY = 0>
+template <bool SKIP>
 __global__ void __launch_bounds__(kThreads) k_trop_multi_mixed(const __grid_constant__ Dev P, const MultiMixed M,
                                                                const TileRef *__restrict__ tiles, int ntiles, int nwet,
-                                                               int TX, int TY, unsigned long long *cnt, int *err) {
-  if (CTX > 0) { TX = CTX; TY = CTY; }
+                                                               unsigned long long *cnt, int *err) {
   extern __shared__ double smd[];
-  const int W = TX + 4, RS = W * (TY + 4);
+  constexpr int W = TX + 4, RS = W * (TY + 4);
   float *smf = reinterpret_cast<float *>(smd + D_COUNT * RS);
   const int tid = threadIdx.x, nth = blockDim.x;
   const int nstep = P.nstep;
@@ -337,19 +336,9 @@ __global__ void __launch_bounds__(kThreads) k_trop_multi_mixed(const __grid_cons
 }
 
 namespace {
-// the fixed-shape form for the 32 x 10 tiles the single-domain multi-tile
-// path uses
-const void *mm_kernel(int TX, int TY, bool skip) {
-  if (TX == 32 && TY == 10)
-    return skip ? (const void *)k_trop_multi_mixed<true, 32, 10> : (const void *)k_trop_multi_mixed<false, 32, 10>;
-  return skip ? (const void *)k_trop_multi_mixed<true> : (const void *)k_trop_multi_mixed<false>;
-}
+const void *mm_kernel(bool skip) { return skip ? (const void *)k_trop_multi_mixed<true> : (const void *)k_trop_multi_mixed<false>; }
+constexpr size_t kSmem = (size_t)(TX + 4) * (TY + 4) * (D_COUNT * sizeof(double) + F_COUNT * sizeof(float));
 }  // namespace
-
-size_t trop_multi_mixed_smem(int TX, int TY) {
-  const size_t rs = (size_t)(TX + 4) * (TY + 4);
-  return D_COUNT * rs * sizeof(double) + F_COUNT * rs * sizeof(float);
-}
 
 size_t trop_multi_mixed_scratch_bytes(long long n2) {
   return (size_t)n2 * ((MC_COUNT + 4 + 2) * sizeof(float) + 1);
@@ -368,30 +357,31 @@ void trop_multi_mixed_bind(MultiMixed &M, void *scratch, long long n2) {
   M.fl = (unsigned char *)f;
 }
 
-int trop_multi_mixed_max_blocks(int TX, int TY) {
-  int dev = 0, nsm = 0, per = 0;
+// (of whichever form: the tiles to skip are counted with this number)
+int trop_multi_mixed_max_blocks() {
+  int dev = 0, nsm = 0, least = 1 << 20;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = trop_multi_mixed_smem(TX, TY);
-  const void *fn = mm_kernel(TX, TY, true);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kThreads, smem) != cudaSuccess) return 0;
-  return per * nsm;
+  for (bool skip : {false, true}) {
+    int per = 0;
+    if (cudaFuncSetAttribute(mm_kernel(skip), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, mm_kernel(skip), kThreads, kSmem) != cudaSuccess) return 0;
+    least = per < least ? per : least;
+  }
+  return least * nsm;
 }
 
 cudaError_t launch_trop_multi_mixed(const Dev &P, const MultiMixed &M, const TileRef *dtiles, int ntiles, int nwet,
-                                    int TX, int TY, int nblocks, unsigned long long *cnt, int *err, cudaStream_t s) {
+                                    int nblocks, unsigned long long *cnt, int *err, cudaStream_t s) {
   k_mm_prep<<<592, 256, 0, s>>>(P, M);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const size_t smem = trop_multi_mixed_smem(TX, TY);
-  const void *fn = mm_kernel(TX, TY, nwet < ntiles);
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const void *fn = mm_kernel(nwet < ntiles);
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return e;
   // the barrier counter starts from zero in every launch
   e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  void *args[] = {(void *)&P, (void *)&M, (void *)&dtiles, (void *)&ntiles, (void *)&nwet, (void *)&TX, (void *)&TY, (void *)&cnt,
-                  (void *)&err};
-  return cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(kThreads), args, smem, s);
+  void *args[] = {(void *)&P, (void *)&M, (void *)&dtiles, (void *)&ntiles, (void *)&nwet, (void *)&cnt, (void *)&err};
+  return cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(kThreads), args, kSmem, s);
 }

@@ -602,8 +602,8 @@ int pick_trop_config(pcom_handle *h) {
         return PCOM_OK;
       }
     } else {
-      const int tx = 32, ty = 10;
-      const int mmb = trop_multi_mixed_max_blocks(tx, ty);
+      const int tx = kMixedMultiX, ty = kMixedMultiY;
+      const int mmb = trop_multi_mixed_max_blocks();
       if (mmb <= 0) return fail(PCOM_ERR_CUDA, "the mixed multi-tile barotropic kernel cannot be launched");
       std::vector<TileRef> t;
       std::vector<int> list;
@@ -623,7 +623,8 @@ int pick_trop_config(pcom_handle *h) {
       }
       int rc = h->d_tiles1 ? PCOM_OK : h->alloc(&h->d_tiles1, t.size());  // (as many tiles in every pick)
       if (rc) return rc;
-      CK(cudaMemcpy(h->d_tiles1, t.data(), t.size() * sizeof(TileRef), cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(h->d_tiles1, t.data(), t.size() * sizeof(TileRef), cudaMemcpyHostToDevice, h->stream));
+      CK(cudaStreamSynchronize(h->stream));
       h->ntiles1 = (int)t.size();
       if (!h->mm_scratch) {
         rc = h->alloc(&h->mm_scratch, trop_multi_mixed_scratch_bytes(h->n2));
@@ -726,7 +727,10 @@ int do_trop(pcom_handle *h) {
   CK(cudaGetLastError());  // of the launches before: setting a kernel's attributes below forgets them
   if (h->trop_blocks <= 0) {
     int rc = pick_trop_config(h);
-    if (rc) return rc;
+    if (rc) {
+      h->trop_blocks = 0;
+      return rc;
+    }
   }
   Prof p(h, "int_trop");
   cudaError_t e;
@@ -737,8 +741,8 @@ int do_trop(pcom_handle *h) {
       e = launch_trop_fast(h->D, h->trop_tx, h->trop_ty, h->trop_seq, h->stream);
     h->trop_seq += (unsigned long long)h->D.nstep;
   } else if (h->trop_multi && h->mixed) {
-    e = launch_trop_multi_mixed(h->D, h->mm, h->d_tiles1, h->ntiles1, h->nwet1, h->trop_tx, h->trop_ty, h->trop_blocks,
-                                h->d_cnt1, h->D.err, h->stream);
+    e = launch_trop_multi_mixed(h->D, h->mm, h->d_tiles1, h->ntiles1, h->nwet1, h->trop_blocks, h->d_cnt1, h->D.err,
+                                h->stream);
   } else if (h->trop_multi) {
     h->launches++;  // its coefficient packing
     e = launch_trop_multi(h->D, h->ms, h->trop_tx, h->trop_ty, h->trop_blocks, h->d_cnt1, h->stream);

@@ -77,9 +77,10 @@ struct MultiMixed {
 };
 size_t trop_multi_mixed_scratch_bytes(long long n2);
 void trop_multi_mixed_bind(MultiMixed &M, void *scratch, long long n2);
-int trop_multi_mixed_max_blocks(int TX, int TY);
+constexpr int kMixedMultiX = 32, kMixedMultiY = 10;  // its tiles
+int trop_multi_mixed_max_blocks();
 cudaError_t launch_trop_multi_mixed(const Dev &P, const MultiMixed &M, const TileRef *dtiles, int ntiles, int nwet,
-                                    int TX, int TY, int nblocks, unsigned long long *cnt, int *err, cudaStream_t s);
+                                    int nblocks, unsigned long long *cnt, int *err, cudaStream_t s);
 
 // a batch's members too large for the resident form: several tiles per CTA
 size_t trop_batch_smem(int TX, int TY);
