@@ -25,7 +25,7 @@
 //    28 % of such tiles: 2.12 -> 1.77 ms, of 611 x 253: 1.69 -> 1.37 ms; a
 //    domain with none pays nothing.
 // Floor of a 1440 x 640 substep: 270 MB from HBM or L2 (40 us at 6.5 TB/s) and
-// ~38 us of stages.  Measured: see the launcher.
+// ~38 us of stages; measured 61 (7.28 ms for the 120).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
