@@ -8,7 +8,8 @@ import numpy as np
 import pytest
 
 from pcom_b200 import _lib as L
-from pcom_b200.model import PHASES, Batch, Model
+from pcom_b200.model import Batch
+from pcom_b200.model import PHASES, Model
 from pcom_b200.synth import make_case
 from parity_util import PHASE_FIELDS, STATE_FIELDS, acr_mask, compare
 
